@@ -208,7 +208,6 @@ int32_t sa_index_build(const sa_refs* refs, const sa_seeding_params* p, int32_t 
     uint32_t b = bits < 0 ? pick_bits(refs->contigs, idx->sp) : (uint32_t)bits;
     require(b >= 1 && b <= 32, "bits must be in 1..32");
     build_index_gpu(refs->contigs, idx->sp, b, filter_fraction, *idx, 0);
-    finish_index(idx.get());
     *out = idx.release();
     return SA_OK;
     SA_CATCH

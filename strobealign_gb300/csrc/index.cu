@@ -58,25 +58,43 @@ __device__ __forceinline__ uint32_t find_contig(const uint64_t* cstart, uint32_t
     return lo;
 }
 
-__global__ void k_syncmer_flags(const uint64_t* words, const uint64_t* word_off, const uint32_t* clen,
-                                const uint64_t* cstart, uint32_t ncontig, uint64_t total, SeedParams p,
-                                uint8_t* flags) {
-    for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < total;
-         g += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t c = find_contig(cstart, ncontig, g);
-        uint64_t pos = g - cstart[c];
-        uint8_t f = 0;
-        if (pos + p.k <= clen[c]) {
-            const uint64_t* w = words + word_off[c];
-            uint64_t mn = UINT64_MAX, ht = 0;
-            for (uint32_t q = 0; q <= p.k - p.s; q++) {
-                uint64_t h = xxh64_u64(canonical(w, pos + q, p.s, nullptr));
-                mn = h < mn ? h : mn;
-                if (q == p.t - 1) ht = h;
+// Open-syncmer flag of every reference position: the (t-1)-th of the k-mer's k-s+1 s-mer
+// hashes equals their minimum.  A warp takes 32 consecutive s-mers at a time, one hash
+// per lane, and shuffles give each of the first 32 - (k - s) lanes the hashes of its
+// k-mer, so a position costs 32 / (32 - (k - s)) hashes instead of k - s + 1.  Its
+// FLAG_RUN windows are consecutive: the contig is searched for once, and lanes past its
+// end step on from there.  Bound by the hash's 64-bit multiplies and the shuffles: 100 Mbp
+// (k 20, s 16) take 0.77 ms; a thread per position with its five hashes and its own
+// contig search took 1.96 ms.
+constexpr uint32_t FLAG_RUN = 16;
+
+__global__ void __launch_bounds__(256) k_syncmer_flags(const uint64_t* words, const uint64_t* word_off,
+                                                       const uint32_t* clen, const uint64_t* cstart, uint32_t ncontig,
+                                                       uint64_t total, SeedParams p, uint8_t* flags) {
+    const uint32_t lane = threadIdx.x & 31, span = p.k - p.s, step = 32 - span;
+    const uint64_t run = (uint64_t)step * FLAG_RUN, nruns = (total + run - 1) / run;
+    const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x / 32);
+    for (uint64_t w = blockIdx.x * (uint64_t)(blockDim.x / 32) + threadIdx.x / 32; w < nruns; w += nwarps) {
+        uint32_t c = find_contig(cstart, ncontig, w * run);
+        uint64_t c0 = cstart[c], c1 = cstart[c + 1];
+        for (uint32_t x = 0; x < FLAG_RUN; x++) {
+            const uint64_t g = w * run + (uint64_t)x * step + lane;
+            while (g >= c1 && c + 1 < ncontig) {
+                c++;
+                c0 = c1;
+                c1 = cstart[c + 1];
             }
-            f = ht == mn;
+            const uint64_t pos = g - c0, left = c1 > g ? c1 - g : 0;
+            const uint64_t h = left >= p.s && left ? xxh64_u64(canonical(words + word_off[c], pos, p.s, nullptr)) : 0;
+            uint64_t mn = h, ht = p.t == 1 ? h : 0;
+            for (uint32_t d = 1; d <= span; d++) {
+                const uint64_t y = __shfl_down_sync(0xffffffffu, h, d);
+                mn = y < mn ? y : mn;
+                if (d == p.t - 1) ht = y;
+            }
+            // left >= k: the k-mer's s-mers are those of lanes lane .. lane + span
+            if (lane < step && left) flags[g] = left >= p.k && ht == mn;
         }
-        flags[g] = f;
     }
 }
 
@@ -131,40 +149,75 @@ struct RsDecomposer {
     }
 };
 
-// Bucket directory exactly as src/indexer.rs:82-124 fills it: bucket_starts[0] = 0,
-// and for x >= 1 the first position p >= 1 that starts a new hash with top bits
-// >= x (N if none).  Entry 0 only ever starts bucket 0, so when the smallest hash
-// has top bits t > 0, buckets 1..t begin at the end of its run.
-__global__ void k_buckets(const RefRandstrobe* rs, uint64_t n, uint32_t bits, uint64_t* buckets) {
+// One pass over the sorted table for everything derived from it:
+//
+// * the bucket directory exactly as src/indexer.rs:82-124 fills it: bucket_starts[0] = 0,
+//   and for x >= 1 the first position p >= 1 that starts a new hash with top bits >= x (N
+//   if none).  Entry 0 only ever starts bucket 0, so when the smallest hash has top
+//   bits t > 0, buckets 1..t begin at the end of its run;
+// * the histogram of the run lengths of equal hashes (src/indexer.rs:82-137), capped at
+//   101 (a run's walk stops there), and the number of distinct hashes in hist[102];
+// * the largest position and reference index (extent[0], extent[1]).
+//
+// Bound by the table's bytes.  Nearly all runs have one entry: they are counted in
+// registers, the others in shared counters, so that the global counters take a block's
+// sum instead of two 64-bit additions per run on the same two addresses.  20 M entries
+// (320 MB): 0.15 ms, 2.1 TB/s; directory, histogram and extent took 13.8 ms as three
+// kernels, 13.6 of them in those additions.
+__global__ void __launch_bounds__(256) k_table_scan(const RefRandstrobe* rs, uint64_t n, uint32_t bits,
+                                                    uint64_t* buckets, unsigned long long* hist,
+                                                    unsigned int* extent) {
+    __shared__ unsigned int s_hist[103];
+    __shared__ unsigned int s_ext[2];
+    for (uint32_t t = threadIdx.x; t < 103; t += blockDim.x) s_hist[t] = 0;
+    if (threadIdx.x < 2) s_ext[threadIdx.x] = 0;
+    __syncthreads();
     const uint64_t nb = (1ULL << bits) + 1;
     const uint64_t h0 = n ? rs_hash(rs[0]) : 0;
+    unsigned int mp = 0, mr = 0, starts = 0, ones = 0;
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i <= n; i += (uint64_t)gridDim.x * blockDim.x) {
+        uint64_t h = 0, hp = 0;
+        if (i < n) {
+            const RefRandstrobe e = load_rs(rs, i);
+            h = rs_hash(e);
+            mp = max(mp, e.position);
+            mr = max(mr, e.ref_index);
+        }
+        if (i > 0) hp = load_hash(rs, i - 1);
+        if (i > 0 && i < n && h == hp) continue;  // not the start of a new hash
         int64_t lo, hi;
         if (i == 0) {
             lo = -1;
             hi = n == 0 ? (int64_t)nb - 1 : 0;
         } else {
-            uint64_t hp = rs_hash(rs[i - 1]);
-            if (i < n && rs_hash(rs[i]) == hp) continue;  // not the start of a new hash
             lo = hp == h0 ? 0 : (int64_t)(hp >> (64 - bits));
-            hi = i == n ? (int64_t)nb - 1 : (int64_t)(rs_hash(rs[i]) >> (64 - bits));
+            hi = i == n ? (int64_t)nb - 1 : (int64_t)(h >> (64 - bits));
         }
         for (int64_t x = lo + 1; x <= hi; x++) buckets[x] = i;
+        if (i < n) {
+            uint32_t c = 1;
+            while (c < 101 && i + c < n && load_hash(rs, i + c) == h) c++;
+            starts++;
+            if (c == 1) ones++;
+            else atomicAdd(&s_hist[c], 1u);
+        }
     }
-}
-
-// run lengths of equal hashes -> histogram of counts (capped at 101) + number of
-// distinct hashes (src/indexer.rs:82-137)
-__global__ void k_run_hist(const RefRandstrobe* rs, uint64_t n, unsigned long long* hist, unsigned long long* unique) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        uint64_t h = rs_hash(rs[i]);
-        if (i > 0 && rs_hash(rs[i - 1]) == h) continue;
-        atomicAdd(unique, 1ULL);
-        uint64_t e = i + 1;
-        while (e < n && rs_hash(rs[e]) == h) e++;
-        uint64_t c = e - i;
-        atomicAdd(&hist[c > 101 ? 101 : c], 1ULL);
+    for (int d = 16; d > 0; d >>= 1) {
+        mp = max(mp, __shfl_xor_sync(0xffffffffu, mp, d));
+        mr = max(mr, __shfl_xor_sync(0xffffffffu, mr, d));
+        starts += __shfl_xor_sync(0xffffffffu, starts, d);
+        ones += __shfl_xor_sync(0xffffffffu, ones, d);
     }
+    if ((threadIdx.x & 31) == 0) {
+        atomicMax(&s_ext[0], mp);
+        atomicMax(&s_ext[1], mr);
+        atomicAdd(&s_hist[102], starts);
+        atomicAdd(&s_hist[1], ones);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) atomicMax(extent + threadIdx.x, s_ext[threadIdx.x]);
+    for (uint32_t t = threadIdx.x; t < 103; t += blockDim.x)
+        if (s_hist[t]) atomicAdd(&hist[t], (unsigned long long)s_hist[t]);
 }
 
 __global__ void k_lookup(DevIndex ix, const uint64_t* hashes, uint64_t n, int kind, int64_t* out_pos,
@@ -192,6 +245,9 @@ inline unsigned grid_for(uint64_t n, unsigned block) {
     if (g > sm_count() * 64) g = sm_count() * 64;
     return (unsigned)(g == 0 ? 1 : g);
 }
+
+// eight blocks of 256 threads fill an SM; a block's sums go to the global counters once
+inline unsigned scan_grid(uint64_t n) { return std::min(grid_for(n, 256), (unsigned)sm_count() * 8); }
 
 }  // namespace
 
@@ -228,8 +284,8 @@ void build_index_gpu(const std::vector<Contig>& contigs, const SeedParams& sp, u
     DevBuf<uint8_t> d_flags;
     d_flags.reserve(total);
     if (total)
-        k_syncmer_flags<<<grid_for(total, 256), 256, 0, st>>>(d_words.p, d_woff.p, d_clen.p, d_cstart.p, nc, total, sp,
-                                                             d_flags.p);
+        k_syncmer_flags<<<grid_for((total + 13) / 14, 256), 256, 0, st>>>(d_words.p, d_woff.p, d_clen.p, d_cstart.p, nc,
+                                                                           total, sp, d_flags.p);
     // (2) compaction in position order
     DevBuf<uint64_t> d_gpos, d_count;
     d_gpos.reserve(total + 1);
@@ -258,26 +314,44 @@ void build_index_gpu(const std::vector<Contig>& contigs, const SeedParams& sp, u
     SA_CUDA(cudaStreamSynchronize(st));
     SA_CUDA(cudaGetLastError());
     d_sy.release();
-    // (4) sort on (hash_offset, position, ref_index)
+    // (4) sort on (hash_offset, position, ref_index).  The radix sort is stable and the
+    // randstrobes come by (ref_index, position), so the reference index needs no pass, a
+    // single contig's positions none either, and several contigs' positions only those
+    // bits that the longest contig has: 11 passes of 8 bits for contigs below 2^24 nt
+    // and 8 for one contig, of the 16 that the whole 128-bit key takes (240 us each for
+    // 20 M entries: 2.66 ms of passes for 24 contigs, 3.68 ms before).
     idx.rs.reserve(nsy);
     if (nsy) {
-        size_t tmp = 0;
-        cub::DeviceRadixSort::SortKeys(nullptr, tmp, d_unsorted.p, idx.rs.p, (int64_t)nsy, RsDecomposer{}, 0, 128, st);
+        uint32_t max_len = 0;
+        for (uint32_t c = 0; c < nc; c++) max_len = std::max(max_len, clen[c]);
+        const int pos_bits = nc > 1 ? 32 - __builtin_clz(max_len | 1u) : 0;
+        cub::DoubleBuffer<RefRandstrobe> db(d_unsorted.p, idx.rs.p);
+        auto sort_bits = [&](void* tmp, size_t& bytes, int b0, int b1) {
+            SA_CUDA(cub::DeviceRadixSort::SortKeys(tmp, bytes, db, (int64_t)nsy, RsDecomposer{}, b0, b1, st));
+        };
+        size_t tp = 0, th = 0;
+        if (pos_bits) sort_bits(nullptr, tp, 32, 32 + pos_bits);
+        sort_bits(nullptr, th, 64, 128);
         DevBuf<uint8_t> d_tmp;
-        d_tmp.reserve(tmp);
-        cub::DeviceRadixSort::SortKeys(d_tmp.p, tmp, d_unsorted.p, idx.rs.p, (int64_t)nsy, RsDecomposer{}, 0, 128, st);
+        d_tmp.reserve(std::max(tp, th));
+        if (pos_bits) sort_bits(d_tmp.p, tp, 32, 32 + pos_bits);
+        sort_bits(d_tmp.p, th, 64, 128);
         SA_CUDA(cudaStreamSynchronize(st));
+        if (db.Current() != idx.rs.p) {
+            std::swap(d_unsorted.p, idx.rs.p);
+            std::swap(d_unsorted.n, idx.rs.n);
+        }
     }
     d_unsorted.release();
     // (5) bucket directory and filter cutoff
     uint64_t nb = (1ULL << bits) + 1;
     idx.buckets.reserve(nb);
-    k_buckets<<<grid_for(nsy + 1, 256), 256, 0, st>>>(idx.rs.p, nsy, bits, idx.buckets.p);
-    DevBuf<unsigned long long> d_hist;
-    d_hist.reserve(103);
-    SA_CUDA(cudaMemsetAsync(d_hist.p, 0, 103 * 8, st));
-    if (nsy) k_run_hist<<<grid_for(nsy, 256), 256, 0, st>>>(idx.rs.p, nsy, d_hist.p, d_hist.p + 102);
-    unsigned long long hist[103];
+    DevBuf<unsigned long long> d_hist;  // the histogram, then the two extents
+    d_hist.reserve(104);
+    SA_CUDA(cudaMemsetAsync(d_hist.p, 0, 104 * 8, st));
+    k_table_scan<<<scan_grid(nsy + 1), 256, 0, st>>>(idx.rs.p, nsy, bits, idx.buckets.p, d_hist.p,
+                                                      reinterpret_cast<unsigned int*>(d_hist.p + 103));
+    unsigned long long hist[104];
     SA_CUDA(cudaMemcpyAsync(hist, d_hist.p, sizeof(hist), cudaMemcpyDeviceToHost, st));
     SA_CUDA(cudaStreamSynchronize(st));
     SA_CUDA(cudaGetLastError());
@@ -308,6 +382,8 @@ void build_index_gpu(const std::vector<Contig>& contigs, const SeedParams& sp, u
     idx.bits = bits;
     idx.n = nsy;
     idx.sp = sp;
+    idx.max_pos = (uint32_t)hist[103];
+    idx.n_refs_seen = nsy ? (uint32_t)(hist[103] >> 32) + 1 : 1;
 }
 
 void index_extent_gpu(const sa_index& idx, uint32_t& max_pos, uint32_t& max_ref, cudaStream_t st) {
