@@ -87,6 +87,39 @@ struct DevBuf {
     }
 };
 
+// A second stream for work between two points of a stream; made on first use, at the
+// highest priority (as the streams of the NAM pipelines are).
+struct SideStream {
+    cudaStream_t s = nullptr;
+    cudaEvent_t forked = nullptr, joined = nullptr;
+    SideStream() = default;
+    SideStream(const SideStream&) = delete;
+    SideStream& operator=(const SideStream&) = delete;
+    ~SideStream() {
+        if (forked) cudaEventDestroy(forked);
+        if (joined) cudaEventDestroy(joined);
+        if (s) cudaStreamDestroy(s);
+    }
+    // the side stream, its work ordered after what st holds now
+    cudaStream_t fork(cudaStream_t st) {
+        if (!s) {
+            int least = 0, greatest = 0;
+            SA_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+            SA_CUDA(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, greatest));
+        }
+        if (!forked) SA_CUDA(cudaEventCreateWithFlags(&forked, cudaEventDisableTiming));
+        if (!joined) SA_CUDA(cudaEventCreateWithFlags(&joined, cudaEventDisableTiming));
+        SA_CUDA(cudaEventRecord(forked, st));
+        SA_CUDA(cudaStreamWaitEvent(s, forked, 0));
+        return s;
+    }
+    // st's later work ordered after the side stream's
+    void join(cudaStream_t st) {
+        SA_CUDA(cudaEventRecord(joined, s));
+        SA_CUDA(cudaStreamWaitEvent(st, joined, 0));
+    }
+};
+
 // Pinned host buffer, grow-only.
 template <class T>
 struct PinnedBuf {

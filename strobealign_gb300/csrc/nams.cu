@@ -7,6 +7,8 @@
 //                   local rescue, orientation choice (src/hit.rs, src/chainer.rs:205-216)
 //   k_anchors       warp per read: anchor count, then fill (src/chainer.rs:304-384)
 //   segmented sort  (ref_id, ref_start, query_start) packed in a u64 key
+//   k_chain_long_prep, k_chain_big, k_chain_long   orientations of over 96 anchors, their
+//                   position clusters scored apart, beside k_chain4
 //   k_chain4        warp per eight read orientations: anchor sort and dedup, collinear
 //                   chaining DP with the reference's early-break rules evaluated as a
 //                   prefix max over the candidates (four lanes per orientation), chain
@@ -759,100 +761,138 @@ __device__ void warp_radix_sort_desc(uint32_t* idx, uint32_t* tmp, uint32_t m, c
 
 // extract_chains (src/chainer.rs:386-449) for one read orientation (segment sg, anchors
 // b .. b + N of the deduplicated list) by the whole warp; best_score is the segment's
-// best chain score.  hist: this warp's 256 shared counters.
+// best chain score.  hist: this warp's 256 shared counters; scratch: one word per anchor.
+//
+// The reference walks the candidates' chains in order of score and drops a chain that
+// meets an anchor which an earlier walk marked.  The predecessors make a forest, every
+// walk ends at its tree's root, and a walk marks all its anchors but the first.  So a
+// tree's root is marked by the first candidate in order that is not the root itself;
+// that candidate meets no mark, and every later one is marked or meets one at the root at
+// the latest.  A tree therefore keeps that one chain, and the root alone as a chain of its
+// own if it is a candidate and comes before it.  So there is no order to walk in: the
+// roots, each tree's first candidate (a maximum per root), and only the kept chains are
+// sorted and walked, 32 at a time.  Tandem arrays leave hundreds of chains per orientation:
+// walked one after another, 5,200 anchors with 512 chains took 2.2 M cycles (1.1 ms, the
+// kernel's length).
 __device__ void chain_extract(const uint64_t* dedup, const float* dp, const uint32_t* pred, uint32_t* aux,
-                              uint64_t total_anchors, uint64_t b, uint32_t N, uint32_t sg, float best_score,
-                              const AnchorPack& ap, const ChainCtx& cc, NamRec* nam_out, uint32_t* nam_seg_count,
-                              uint64_t* anc_out, uint64_t* anc_start, uint32_t* hist) {
+                              uint64_t total_anchors, unsigned long long* scratch, uint64_t b, uint32_t N, uint32_t sg,
+                              float best_score, const AnchorPack& ap, const ChainCtx& cc, NamRec* nam_out,
+                              uint32_t* nam_seg_count, uint64_t* anc_out, uint64_t* anc_start, uint32_t* hist) {
     const uint32_t lane = lane_id();
     const uint64_t qmask = (1ULL << ap.qbits) - 1, pmask = (1ULL << ap.pbits) - 1;
     const float valid_score = __fmul_rn(best_score, cc.cp.valid_score_threshold);
-    uint32_t* cand = aux + b;
-    uint32_t* sorted_c = aux + total_anchors + b;
-    uint32_t* used = aux + 2 * total_anchors + b;
-    uint32_t M = 0;
+    constexpr uint32_t NO = 0xffffffffu;
+    uint32_t* kept = aux + b;
+    uint32_t* sorted = aux + total_anchors + b;
+    uint32_t* root = aux + 2 * total_anchors + b;
+    unsigned long long* first = scratch + b;
+    // larger = earlier in the reference's order: by score, ties by anchor order
+    auto order_key = [](uint32_t i, float score) { return ((uint64_t)~desc_key(score) << 32) | (NO - i); };
+    // predecessors come before their successors: roots 32 anchors at a time, a
+    // predecessor within the 32 by pointer jumping
     for (uint32_t c = 0; c < N; c += 32) {
-        uint32_t i = c + lane;
-        bool take = i < N && dp[b + i] >= valid_score;
-        uint32_t bal = __ballot_sync(FULL, take);
-        if (take) cand[M + __popc(bal & lanemask_lt())] = i;
-        if (i < N) used[i] = 0;
-        M += __popc(bal);
+        const uint32_t i = c + lane;
+        const uint32_t p = i < N ? pred[b + i] : NO;
+        uint32_t r = p == NO ? i : p;  // an anchor on i's way to the root
+#pragma unroll
+        for (int d = 0; d < 5; d++) {
+            const uint32_t up = __shfl_sync(FULL, r, r >= c ? r - c : lane);
+            if (r >= c) r = up;
+        }
+        if (r < c) r = root[r];
+        if (i < N) {
+            root[i] = r;
+            first[i] = 0;
+        }
+        __syncwarp();
+    }
+    for (uint32_t i = lane; i < N; i += 32) {
+        const float s = dp[b + i];
+        const uint32_t r = root[i];
+        if (s >= valid_score && r != i) atomicMax(&first[r], (unsigned long long)order_key(i, s));
     }
     __syncwarp();
-    // candidates by score, descending, ties in anchor order (a stable sort)
-    if (M <= 32) {
-        const uint32_t ci = lane < M ? cand[lane] : 0;
-        const float s = lane < M ? dp[b + ci] : 0.0f;
+    uint32_t K = 0;
+    for (uint32_t c = 0; c < N; c += 32) {
+        const uint32_t i = c + lane;
+        bool take = false;
+        if (i < N) {
+            const float s = dp[b + i];
+            const uint32_t r = root[i];
+            if (s >= valid_score) {
+                const uint64_t f = __ldcg(&first[r]), key = order_key(i, s);
+                take = i == r ? key > f : key == f;
+            }
+        }
+        const uint32_t bal = __ballot_sync(FULL, take);
+        if (take) kept[K + __popc(bal & lanemask_lt())] = i;
+        K += __popc(bal);
+    }
+    __syncwarp();
+    // by score, descending, ties in anchor order (a stable sort)
+    if (K <= 32) {
+        const uint32_t ci = lane < K ? kept[lane] : 0;
+        const float s = lane < K ? dp[b + ci] : 0.0f;
         uint32_t rank = 0;
-        for (uint32_t u = 0; u < M; u++) {
+        for (uint32_t u = 0; u < K; u++) {
             const float su = __shfl_sync(FULL, s, u);
             rank += (su > s) || (su == s && u < lane);
         }
-        if (lane < M) sorted_c[rank] = ci;
+        if (lane < K) sorted[rank] = ci;
     } else {
-        warp_radix_sort_desc(cand, sorted_c, M, dp + b, hist);
+        warp_radix_sort_desc(kept, sorted, K, dp + b, hist);
     }
     __syncwarp();
-    // the walk's used flags: a bit each in the warp's shared counters (free after the
-    // sort) when they fit, else the global array
-    const bool bits = N <= 32 * 256;
-    if (bits)
-        for (uint32_t w = lane; w < (N + 31) / 32; w += 32) hist[w] = 0;
-    __syncwarp();
-    auto is_used = [&](uint32_t j) -> bool { return bits ? (hist[j >> 5] >> (j & 31)) & 1 : used[j] != 0; };
-    auto set_used = [&](uint32_t j) {
-        if (bits) hist[j >> 5] |= 1u << (j & 31);
-        else used[j] = 1;
-    };
-    if (lane == 0) {
-        uint32_t nn = 0;
-        NamRec* outp = nam_out + b;
-        // a kept chain holds its end anchor (never marked used) and used
-        // predecessors, so kept chains list each anchor at most twice; a dropped
-        // chain's anchors are overwritten: 3 slots per anchor suffice
-        uint64_t* ao = anc_out ? anc_out + 3 * b : nullptr;
-        uint32_t acur = 0;
-        for (uint32_t c = 0; c < M; c++) {
-            uint32_t i = sorted_c[c];
-            if (is_used(i)) continue;
-            uint32_t j = i;
-            bool overlaps = false;
-            uint32_t nanch = 1;
+    // kept chains share no anchor but a root that is also a chain of its own: 2 slots
+    // per anchor suffice (3 are there)
+    uint64_t* ao = anc_out ? anc_out + 3 * b : nullptr;
+    uint32_t acur = 0;
+    for (uint32_t c = 0; c < K; c += 32) {
+        const uint32_t x = c + lane;
+        uint32_t n = 0, i = 0;
+        if (x < K) {
+            i = sorted[x];
             const uint64_t ki = dedup[b + i];
-            if (ao) ao[acur] = ki;
-            uint32_t matching = cc.k;
-            uint32_t cov = (uint32_t)((ki >> ap.qbits) & pmask);
-            while (pred[b + j] != 0xffffffffu) {
+            uint32_t matching = cc.k, cov = (uint32_t)((ki >> ap.qbits) & pmask);
+            uint64_t kj = ki;
+            n = 1;
+            // a root that is followed by its tree's chain stands alone: it has no predecessor
+            for (uint32_t j = pred[b + i]; j != NO;) {
+                kj = dedup[b + j];
                 j = pred[b + j];
-                if (is_used(j)) { overlaps = true; break; }
-                if (ao) ao[acur + nanch] = dedup[b + j];
-                nanch++;
-                set_used(j);
-                uint32_t rsj = (uint32_t)((dedup[b + j] >> ap.qbits) & pmask);
-                uint32_t d = cov > rsj ? cov - rsj : 0;
+                n++;
+                const uint32_t rs = (uint32_t)((kj >> ap.qbits) & pmask), d = cov > rs ? cov - rs : 0;
                 matching += d < cc.k ? d : cc.k;
-                cov = rsj;
+                cov = rs;
             }
-            if (overlaps) continue;
-            const uint64_t kf2 = dedup[b + j];
             NamRec nr;
-            nr.nam_id = nn;
-            nr.query_start = (uint32_t)(kf2 & qmask);
+            nr.nam_id = x;
+            nr.query_start = (uint32_t)(kj & qmask);
             nr.query_end = (uint32_t)(ki & qmask) + cc.k;
-            nr.ref_start = (uint32_t)((kf2 >> ap.qbits) & pmask);
+            nr.ref_start = cov;
             nr.ref_end = (uint32_t)((ki >> ap.qbits) & pmask) + cc.k;
             nr.matching_bases = matching;
             nr.ref_id = (uint32_t)(ki >> (ap.pbits + ap.qbits));
-            nr.score = __fadd_rn(dp[b + i], __fmul_rn(__uint2float_rn(nanch), cc.cp.matches_weight));
+            nr.score = __fadd_rn(dp[b + i], __fmul_rn(__uint2float_rn(n), cc.cp.matches_weight));
             nr.is_revcomp = sg & 1;
-            nr.n_anchors = nanch;
-            if (anc_start) anc_start[b + nn] = 3 * b + acur;
-            acur += nanch;
-            outp[nn++] = nr;
+            nr.n_anchors = n;
+            nam_out[b + x] = nr;
         }
-        nam_seg_count[sg] = nn;
+        if (ao) {
+            uint32_t tot;
+            const uint32_t at = acur + warp_excl_scan(n, tot);
+            if (x < K) {
+                anc_start[b + x] = 3 * b + at;
+                uint32_t j = i;
+                for (uint32_t t = 0; t < n; t++) {
+                    ao[at + t] = dedup[b + j];
+                    j = pred[b + j];
+                }
+            }
+            acur += tot;
+        }
     }
+    if (lane == 0) nam_seg_count[sg] = K;
     __syncwarp();
 }
 
@@ -1069,18 +1109,17 @@ __device__ __forceinline__ uint32_t warp_sort_dedup(uint64_t* keys, uint32_t cnt
 }
 
 // Chaining (src/chainer.rs:128-176 and 386-449) for NG = 8 read orientations per warp.
-// The anchor sort, the deduplication and the extraction run over the whole warp, one
-// orientation after the other.  The DP is serial over a read orientation's anchors;
+// The anchor sort and the deduplication run over the whole warp, one orientation after
+// the other.  The DP is serial over a read orientation's anchors;
 // the candidates j of anchor i (back to max_lookback) are scored in parallel and an
 // exclusive prefix max over them reproduces the reference's downward scan with its
 // ">=" updates and its stops (a different reference or a gap >= max_ref_gap ends the
 // scan; an update on the same diagonal ends it after that candidate).  The DP runs for
 // the NG orientations at once, one group of CG = 4 lanes each, four candidates at a
 // time (most anchors stop at the first candidate: the one before on the same
-// diagonal).  Orientations with more than CHAIN_GROUP_MAX anchors get a warp each and
-// run the DP with all 32 lanes, 32 candidates at a time.  The orientations come from
-// k_seg_list (those with anchors); nam_seg_count of the others is zeroed before the
-// launch.
+// diagonal).  The orientations come from k_seg_list (those with up to CHAIN_GROUP_MAX
+// anchors; longer ones: k_chain_long); nam_seg_count of those without anchors is zeroed
+// before the launch.
 //
 // RING: max_lookback < 64, so the predecessors of anchor i (and their scores) come
 // from a 64-entry ring in shared memory per orientation, written as anchors are
@@ -1122,29 +1161,19 @@ __device__ __forceinline__ void chain_candidates(uint32_t j, bool in, const uint
 }
 
 // The lookback DP of collinear_chaining (src/chainer.rs:85-180) over anchors [c0, c1)
-// of one read orientation (its anchors at dedup[b ..]) by the whole warp: 32
-// predecessors per step, the early-break rules as a prefix max over the lanes.
+// of one read orientation (its anchors at dedup[b ..]) by the whole warp, for a
+// max_lookback of 64 or more (warp_chain_regs otherwise): 32 predecessors per step, the early-break rules as a prefix max over the lanes.
 // Predecessors never go below c0 (earlier anchors lie max_ref_gap or more behind, or
 // on another reference, and end the reference's scan without contributing).  With
 // recheck, (best_score, best_index, best_key) is the running best over all anchors
 // before c0 and is updated as the reference updates it (strict >); without, the
 // best-index re-check (:150-165) is left out.
-template <bool RING>
 __device__ void warp_chain_range(const uint64_t* dedup, float* dp, uint32_t* pred, uint64_t b, uint32_t c0, uint32_t c1,
                                  uint32_t floor, uint32_t max_ref_gap, const ChainCtx& cc, const AnchorPack& ap,
-                                 uint64_t* ring_key, float* ring_dp, bool recheck, float& best_score,
-                                 uint32_t& best_index, uint64_t& best_key) {
+                                 bool recheck, float& best_score, uint32_t& best_index, uint64_t& best_key) {
     const uint32_t lane = lane_id();
     const uint64_t qmask = (1ULL << ap.qbits) - 1, pmask = (1ULL << ap.pbits) - 1;
     const float kf = __uint2float_rn(cc.k);
-    if (RING && c0 > floor) {
-        // resuming inside a cluster: the ring takes the anchors before c0 from memory
-        for (uint32_t j = (c0 - floor > 64 ? c0 - 64 : floor) + lane; j < c0; j += 32) {
-            ring_key[j & 63] = dedup[b + j];
-            ring_dp[j & 63] = dp[b + j];
-        }
-        __syncwarp();
-    }
     uint64_t next_key = c0 < c1 ? dedup[b + c0] : 0;
     for (uint32_t i = c0; i < c1; i++) {
         const uint64_t ki = next_key;
@@ -1162,8 +1191,8 @@ __device__ void warp_chain_range(const uint64_t* dedup, float* dp, uint32_t* pre
             const uint32_t j = i - 1 - t;
             bool hard, valid, diag;
             float val;
-            chain_candidates<RING>(j, in, dedup, dp, b, ring_key, ring_dp, ri, rsi, qi, max_ref_gap, cc, ap, hard,
-                                   valid, diag, val);
+            chain_candidates<false>(j, in, dedup, dp, b, nullptr, nullptr, ri, rsi, qi, max_ref_gap, cc, ap, hard,
+                                    valid, diag, val);
             // the common case: the first candidate updates and lies on the same diagonal,
             // which ends the scan (the prefix max below would find the same)
             if (__ballot_sync(FULL, lane == 0 && valid && diag && val >= cur)) {
@@ -1216,10 +1245,6 @@ __device__ void warp_chain_range(const uint64_t* dedup, float* dp, uint32_t* pre
         if (lane == 0) {
             dp[b + i] = cur;
             pred[b + i] = cur_pred;
-            if (RING) {
-                ring_key[i & 63] = ki;
-                ring_dp[i & 63] = cur;
-            }
         }
         if (recheck && cur > best_score) {
             best_score = cur;
@@ -1229,6 +1254,172 @@ __device__ void warp_chain_range(const uint64_t* dedup, float* dp, uint32_t* pre
         if (!recheck && cur > best_score) best_score = cur;  // the range's maximum
         __syncwarp();
     }
+}
+
+// One predecessor pair's share of chain_candidates without the predecessor's score:
+// chain_score, or -inf where the pair is no candidate; both anchors on one reference.
+__device__ __forceinline__ float pair_score(uint32_t rsi, uint32_t qi, uint32_t rsj, uint32_t qj, bool in,
+                                            uint32_t max_ref_gap, const ChainCtx& cc, bool& diag) {
+    const uint32_t dq = qi - qj, dr = rsi - rsj;
+    const uint32_t mx = dq > dr ? dq : dr, mn = dq < dr ? dq : dr;
+    const bool ok = in && qi >= qj && dr < max_ref_gap && !ratio_above(mx, mn, cc);
+    diag = ok && dq == dr;
+    return ok ? chain_score(dq, dr, cc) : -INFINITY;
+}
+
+// Slots as bits (a: slots 0-31, c: slots 32-63) in scan order of anchor i: the predecessor
+// at distance t (anchor i - 1 - t, slot (i - 1 - t) & 63) at bit 63 - t.
+__device__ __forceinline__ uint64_t scan_order(uint32_t i, bool a, bool c) {
+    const uint64_t m = __ballot_sync(FULL, a) | ((uint64_t)__ballot_sync(FULL, c) << 32);
+    const uint32_t rot = 63 - ((i - 1) & 63);
+    return rot ? (m << rot) | (m >> (64 - rot)) : m;
+}
+
+// The outcome of anchor i's predecessor scan (src/chainer.rs:98-147) from the candidates'
+// chain scores, lane l holding those of slots l (vA) and l + 32 (vB), -inf for no
+// candidate; diag marks those on the anchor's diagonal, in scan order.  A candidate whose
+// gap ends the reference's scan is simply none (positions are sorted, so none after it
+// could count).  Without one on the same diagonal the result is the maximum, ties to the
+// farthest; with one, it ends the scan if it reaches the maximum (checked first) or the
+// maximum over the nearer ones (a prefix maximum).  Scores below k never update and all
+// others are positive, so their bits order as integers (redux).
+__device__ __forceinline__ void scan_outcome(uint32_t i, float vA, float vB, uint64_t diag, float kf, float& cur,
+                                             uint32_t& cur_pred) {
+    const uint32_t lane = lane_id();
+    const float M = __uint_as_float(__reduce_max_sync(FULL, __float_as_uint(fmaxf(fmaxf(vA, vB), 0.0f))));
+    cur = kf;
+    cur_pred = 0xffffffffu;
+    if (!(M >= kf)) return;
+    if (diag) {
+        uint32_t t = (uint32_t)__clzll((long long)diag);
+        uint32_t slot = (i - 1 - t) & 63;
+        float v = __shfl_sync(FULL, slot & 32 ? vB : vA, slot & 31);
+        bool stopped = v >= M;
+        if (!stopped) {
+            // does a same-diagonal candidate reach the maximum over the nearer ones?
+            // each lane has one candidate at distance r and one at r + 32
+            const uint32_t r = (i - 1 - lane) & 31;
+            const bool near_b = (i - 1 - r) & 32;
+            const float near = near_b ? vB : vA, far = near_b ? vA : vB;
+            float pn = near, pf = far;
+#pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const float yn = __shfl_sync(FULL, pn, (lane + d) & 31), yf = __shfl_sync(FULL, pf, (lane + d) & 31);
+                if (r >= d) {
+                    pn = fmaxf(pn, yn);
+                    pf = fmaxf(pf, yf);
+                }
+            }
+            const float all_near = __shfl_sync(FULL, pn, (i - 32) & 31);  // the lane with r = 31
+            float en = __shfl_sync(FULL, pn, (lane + 1) & 31), ef = __shfl_sync(FULL, pf, (lane + 1) & 31);
+            if (r == 0) en = ef = -INFINITY;
+            ef = fmaxf(ef, all_near);
+            const uint32_t un = __ballot_sync(FULL, ((diag >> (63 - r)) & 1) && near >= fmaxf(kf, en));
+            const uint32_t uf = __ballot_sync(FULL, ((diag >> (31 - r)) & 1) && far >= fmaxf(kf, ef));
+            if (un | uf) {
+                // the nearest one's lane to bit 31
+                const uint32_t m = un ? un : uf;
+                t = __clz(__funnelshift_l(m, m, 31 - ((i - 1) & 31))) + (un ? 0 : 32);
+                slot = (i - 1 - t) & 63;
+                v = __shfl_sync(FULL, slot & 32 ? vB : vA, slot & 31);
+                stopped = true;
+            }
+        }
+        if (stopped) {
+            cur = v;
+            cur_pred = i - 1 - t;
+            return;
+        }
+    }
+    cur = M;
+    const uint64_t eq = scan_order(i, vA == M, vB == M);
+    cur_pred = i - 1 - (uint32_t)(64 - __ffsll((long long)eq));
+}
+
+// The best-index re-check (:150-165) of an anchor (its key, position and query start)
+// against the running best: whether it applies, and the score it gives.
+__device__ __forceinline__ bool recheck_score(uint64_t key, uint32_t rs, uint32_t q, uint64_t best_key,
+                                              float best_score, uint32_t max_ref_gap, const ChainCtx& cc,
+                                              const AnchorPack& ap, float& ns) {
+    const uint64_t pmask = (1ULL << ap.pbits) - 1;
+    const uint32_t rsb = (uint32_t)((best_key >> ap.qbits) & pmask),
+                   qb = (uint32_t)best_key & (uint32_t)((1ULL << ap.qbits) - 1);
+    const uint32_t dq = q - qb, dr = rs - rsb;
+    if (dr >= max_ref_gap || dr == 0 || q <= qb) return false;
+    if ((best_key >> (ap.pbits + ap.qbits)) != (key >> (ap.pbits + ap.qbits))) return false;
+    if (ratio_above(dq > dr ? dq : dr, dq < dr ? dq : dr, cc)) return false;
+    ns = __fadd_rn(best_score, chain_score(dq, dr, cc));
+    return true;
+}
+
+// warp_chain_range with the re-check, for max_lookback < 64, the predecessors in
+// registers: slot j & 63 of the last 64 anchors, two per lane; used where a cluster is
+// scored again from an anchor on.
+__device__ void warp_chain_regs(const uint64_t* dedup, float* dp, uint32_t* pred, uint64_t b, uint32_t c0, uint32_t c1,
+                                uint32_t floor, uint32_t max_ref_gap, const ChainCtx& cc, const AnchorPack& ap,
+                                float& best_score, uint32_t& best_index, uint64_t& best_key) {
+    const uint32_t lane = lane_id();
+    const uint64_t pmask = (1ULL << ap.pbits) - 1;
+    const uint32_t qmask = (uint32_t)((1ULL << ap.qbits) - 1);
+    const float kf = __uint2float_rn(cc.k);
+    const uint32_t lookback = cc.cp.max_lookback;
+    auto ref_of = [&](uint64_t k) { return (uint32_t)((k >> ap.qbits) & pmask); };
+    uint32_t rsA = 0, qA = 0, rsB = 0, qB = 0;
+    float dA = 0.0f, dB = 0.0f;
+    if (c0 > floor) {
+        // resuming inside a cluster: the anchors before c0 from memory
+        const uint32_t jA = c0 - 1 - ((c0 - 1 - lane) & 63), jB = c0 - 1 - ((c0 - 33 - lane) & 63);
+        if ((int32_t)(jA - floor) >= 0 && jA < c0) {
+            const uint64_t k = dedup[b + jA];
+            rsA = ref_of(k);
+            qA = (uint32_t)k & qmask;
+            dA = dp[b + jA];
+        }
+        if ((int32_t)(jB - floor) >= 0 && jB < c0) {
+            const uint64_t k = dedup[b + jB];
+            rsB = ref_of(k);
+            qB = (uint32_t)k & qmask;
+            dB = dp[b + jB];
+        }
+    }
+    for (uint32_t i = c0; i < c1; i++) {
+        const uint64_t ki = dedup[b + i];
+        const uint32_t rsi = ref_of(ki), qi = (uint32_t)ki & qmask;
+        uint32_t span = i > lookback ? lookback : i;
+        if (span > i - floor) span = i - floor;
+        bool gA, gB;
+        const float sA = pair_score(rsi, qi, rsA, qA, ((i - 1 - lane) & 63) < span, max_ref_gap, cc, gA);
+        const float sB = pair_score(rsi, qi, rsB, qB, ((i - 33 - lane) & 63) < span, max_ref_gap, cc, gB);
+        float cur, ns;
+        uint32_t cur_pred;
+        scan_outcome(i, __fadd_rn(dA, sA), __fadd_rn(dB, sB), scan_order(i, gA, gB), kf, cur, cur_pred);
+        if (best_index != 0xffffffffu &&
+            recheck_score(ki, rsi, qi, best_key, best_score, max_ref_gap, cc, ap, ns) && ns > cur) {
+            cur = ns;
+            cur_pred = best_index;
+        }
+        if (lane == 0) {
+            dp[b + i] = cur;
+            pred[b + i] = cur_pred;
+        }
+        if (lane == (i & 31)) {
+            if (i & 32) {
+                rsB = rsi;
+                qB = qi;
+                dB = cur;
+            } else {
+                rsA = rsi;
+                qA = qi;
+                dA = cur;
+            }
+        }
+        if (cur > best_score) {
+            best_score = cur;
+            best_index = i;
+            best_key = ki;
+        }
+    }
+    __syncwarp();
 }
 
 // The first anchor of [lo, hi) (one cluster) where the best-index re-check
@@ -1381,16 +1572,18 @@ __device__ __forceinline__ uint32_t orientation_dedup(const uint64_t* sorted, ui
 // without contributing), so a cluster's DP depends on the others only through the
 // best-index re-check (src/chainer.rs:150-165), which can fire only once the cluster
 // holds the running best, a strict maximum over all earlier anchors.  So the clusters
-// are scored at once without the re-check, here, and k_chain4 then takes, in order, each
-// cluster whose maximum beats the running best of the clusters before it, finds the
-// first anchor where the re-check fires and scores again from there (carrying the
-// running best on); the others are final.
+// are scored at once, the small ones without the re-check, here, the large ones with
+// their own running best (k_chain_big), and k_chain4 then takes them in order.  A small
+// cluster whose maximum beats the running best of those before it is scored again from
+// the first anchor where the re-check fires; a large one only if it first fired while an
+// earlier cluster still held the running best (a cluster of thousands of anchors would
+// otherwise run its serial DP twice).
 //
 // k_chain_long_prep: a warp per long orientation u: the dedup, the cluster starts
 // (aux[b ..]), and the clusters of up to lane_max anchors scored a thread each (maxima
 // at aux[T + b ..] as floats); the larger ones are queued as (u, cluster) items for
 // k_chain_big, a warp each.  long_n[u] / long_c[u]: anchors after dedup, clusters.
-// k_chain4 then checks each record cluster for the first anchor where the re-check
+// k_chain4 checks each small record cluster for the first anchor where the re-check
 // fires (recheck_first_fire) and scores again from there only.
 __global__ void __launch_bounds__(128) k_chain_long_prep(const uint64_t* __restrict__ off, const uint64_t* seg_off,
                                                          const uint64_t* sorted, uint64_t* dedup, float* dp,
@@ -1454,21 +1647,189 @@ __global__ void __launch_bounds__(128) k_chain_long_prep(const uint64_t* __restr
     }
 }
 
-// The queued large clusters, a warp each, without the re-check (their maxima into
-// aux[T + b + cluster]).
-template <bool RING>
+// What k_chain_big leaves of a large cluster at aux[2T + b + its first anchor ..] besides
+// the maximum at aux[T + b + cluster].
+struct BigCluster {
+    uint32_t best_index;  // the first anchor that reaches the maximum
+    uint32_t fire;        // the first anchor whose score the cluster's own re-check changed (~0u: none)
+    float fire_best;      // the maximum before that anchor
+};
+
+// The queued large clusters for max_lookback < 64, a block each (their maxima into
+// aux[T + b + cluster]), with the re-check against the cluster's own running best.  That
+// is the reference's score of every anchor if the best of the clusters before is already
+// beaten when the re-check first changes a score (BigCluster::fire), and in any case up to
+// that anchor; k_chain_long scores the rest again where it is not.
+//
+// A cluster is one serial chain of anchors and the kernel lasts as long as its longest
+// cluster (a tandem repeat's: thousands of anchors), so what counts is the first warp's
+// instructions from one anchor's score to the next.  The other warps prepare, 32 anchors
+// ahead in shared memory, everything that does not depend on scores: the pair scores
+// (gap, ratio test, chain_score) against the 64 anchors before, and which of them lie on
+// the same diagonal.  The first warp holds those anchors' scores two per lane.
+//
+// The longest clusters of 53k-read parts on a 310 Mbp human-shaped genome (up to 3,100
+// anchors): 0.34 ms a launch on average, 0.56 at most; with the whole DP in one warp 1.06
+// and 1.69 ms, and 1.1 and 1.9 ms with the predecessors in shared memory.
+constexpr uint32_t BIG_CHUNK = 32;
+
 __global__ void __launch_bounds__(128) k_chain_big(const uint64_t* __restrict__ off, const uint64_t* seg_off,
-                                                   const uint64_t* dedup, float* dp, uint32_t* pred, uint32_t* aux,
-                                                   uint64_t total_anchors, AnchorPack ap, ChainCtx cc,
+                                                   const uint64_t* __restrict__ dedup, float* dp, uint32_t* pred,
+                                                   uint32_t* aux, uint64_t total_anchors, AnchorPack ap, ChainCtx cc,
                                                    const uint32_t* long_list, const uint32_t* long_n,
                                                    const uint32_t* long_c, const uint32_t* big_items,
                                                    const uint32_t* n_big) {
-    __shared__ uint64_t ring_key_s[RING ? 4 * 64 : 1];
-    __shared__ float ring_dp_s[RING ? 4 * 64 : 1];
-    const uint32_t lane = lane_id(), wib = threadIdx.x / 32;
+    __shared__ float s_pair[2][BIG_CHUNK][64];
+    __shared__ uint64_t s_diag[2][BIG_CHUNK];  // the same-diagonal candidates in scan order
+    __shared__ uint2 s_near[2][BIG_CHUNK];     // the nearest one: its distance, its pair score
+    __shared__ uint2 s_pos[2][BIG_CHUNK];      // the anchor's reference position and query start
+    __shared__ uint64_t s_key[128];  // anchor j's key in slot j & 127
+    const uint32_t lane = lane_id(), w = threadIdx.x / 32;
+    const uint64_t pmask = (1ULL << ap.pbits) - 1;
+    const uint32_t qmask = (uint32_t)((1ULL << ap.qbits) - 1);
+    const float kf = __uint2float_rn(cc.k);
+    const uint32_t lookback = cc.cp.max_lookback;
+    const uint32_t nb = *n_big;
+    for (uint32_t x = blockIdx.x; x < nb; x += gridDim.x) {
+        const uint32_t u = big_items[2 * x], c = big_items[2 * x + 1];
+        const uint32_t sg = long_list[u], N = long_n[u], C = long_c[u];
+        const uint64_t seg_b = seg_off[sg];
+        const uint32_t* cstart = aux + seg_b;
+        const uint32_t lo = cstart[c], n = (c + 1 < C ? cstart[c + 1] : N) - lo;
+        const uint64_t b = seg_b + lo;  // anchors 0 .. n of the cluster
+        const uint32_t read_len = (uint32_t)(off[(sg >> 1) + 1] - off[sg >> 1]);
+        const uint32_t max_ref_gap = cc.cp.max_ref_gap ? cc.cp.max_ref_gap : read_len;
+        // pair scores of chunk q's anchors, by warps w0 .. 3
+        auto prepare = [&](uint32_t q, uint32_t w0) {
+            for (uint32_t a = w - w0; a < BIG_CHUNK; a += 4 - w0) {
+                const uint32_t i = q * BIG_CHUNK + a;
+                if (i >= n) break;
+                const uint64_t ki = s_key[i & 127];
+                const uint32_t rsi = (uint32_t)((ki >> ap.qbits) & pmask), qi = (uint32_t)ki & qmask;
+                const uint32_t span = i < lookback ? i : lookback;
+                bool g[2];
+#pragma unroll
+                for (uint32_t h = 0; h < 2; h++) {
+                    const uint32_t t = (i - 1 - lane - 32 * h) & 63;
+                    const uint64_t kj = s_key[(i - 1 - t) & 127];
+                    s_pair[q & 1][a][lane + 32 * h] =
+                        pair_score(rsi, qi, (uint32_t)((kj >> ap.qbits) & pmask), (uint32_t)kj & qmask, t < span,
+                                   max_ref_gap, cc, g[h]);
+                }
+                const uint64_t d = scan_order(i, g[0], g[1]);
+                __syncwarp();
+                if (lane == 0) {
+                    const uint32_t t = d ? (uint32_t)__clzll((long long)d) : 63;
+                    s_diag[q & 1][a] = d;
+                    s_near[q & 1][a] =
+                        make_uint2(t, __float_as_uint(d ? s_pair[q & 1][a][(i - 1 - t) & 63] : -INFINITY));
+                    s_pos[q & 1][a] = make_uint2(rsi, qi);
+                }
+            }
+        };
+        __syncthreads();  // the cluster before is done with the shared buffers
+        for (uint32_t j = threadIdx.x; j < 2 * BIG_CHUNK; j += blockDim.x)
+            if (j < n) s_key[j] = dedup[b + j];
+        __syncthreads();
+        prepare(0, 0);
+        __syncthreads();
+        float best_score = 0.0f, fire_best = 0.0f;
+        uint32_t best_index = 0xffffffffu, best_pos = 0, fire = 0xffffffffu;
+        uint64_t best_key = 0;
+        float dA = 0.0f, dB = 0.0f;
+        const uint32_t chunks = (n + BIG_CHUNK - 1) / BIG_CHUNK;
+        for (uint32_t q = 0; q < chunks; q++) {
+            if (w > 0) {
+                // the keys of chunk q + 2 take the slots of chunk q - 2
+                const uint32_t j = (q + 2) * BIG_CHUNK + lane;
+                uint64_t kn = 0;
+                if (w == 1 && j < n) kn = dedup[b + j];
+                if (q + 1 < chunks) prepare(q + 1, 1);
+                if (w == 1 && j < n) s_key[j & 127] = kn;
+            } else {
+                // Most anchors take the nearest candidate on their diagonal.  Its score dj
+                // is fetched an anchor ahead (it is the last one's only for distance 0), so
+                // that path needs one addition, one comparison and one vote from the last
+                // anchor's score to this one's.
+                const uint32_t i0 = q * BIG_CHUNK, m = n - i0 < BIG_CHUNK ? n - i0 : BIG_CHUNK;
+                const bool high = q & 1;
+                float sA = s_pair[q & 1][0][lane], sB = s_pair[q & 1][0][lane + 32];
+                uint2 near = s_near[q & 1][0];
+                uint2 pos = s_pos[q & 1][0];
+                uint32_t slot = (i0 - 1 - near.x) & 63;
+                float dj = __shfl_sync(FULL, slot & 32 ? dB : dA, slot & 31);
+                uint32_t my_pred = 0xffffffffu;
+                for (uint32_t a = 0; a < m; a++) {
+                    const uint32_t i = i0 + a;
+                    const float v0 = __fadd_rn(dj, __uint_as_float(near.y));  // -inf without one
+                    const float vA = __fadd_rn(dA, sA), vB = __fadd_rn(dB, sB);
+                    const uint32_t t0 = near.x;
+                    const uint2 here = pos;
+                    const uint32_t a1 = a + 1 < m ? a + 1 : a;
+                    sA = s_pair[q & 1][a1][lane];
+                    sB = s_pair[q & 1][a1][lane + 32];
+                    near = s_near[q & 1][a1];
+                    pos = s_pos[q & 1][a1];
+                    slot = (i - near.x) & 63;
+                    dj = __shfl_sync(FULL, slot & 32 ? dB : dA, slot & 31);
+                    // the re-check's score needs only the best before
+                    float cur = v0, ns = 0.0f;
+                    uint32_t cur_pred = i - 1 - t0;
+                    const bool again = here.x - best_pos < max_ref_gap && best_index != 0xffffffffu &&
+                                       recheck_score(s_key[i & 127], here.x, here.y, best_key, best_score, max_ref_gap,
+                                                     cc, ap, ns);
+                    if (__any_sync(FULL, vA > v0 || vB > v0) || !(v0 >= kf))
+                        scan_outcome(i, vA, vB, s_diag[q & 1][a], kf, cur, cur_pred);
+                    if (again && ns > cur) {
+                        cur = ns;
+                        cur_pred = best_index;
+                        if (fire == 0xffffffffu) {
+                            fire = i;
+                            fire_best = best_score;
+                        }
+                    }
+                    if (lane == a) {
+                        if (high) dB = cur;
+                        else dA = cur;
+                        my_pred = cur_pred == 0xffffffffu ? cur_pred : lo + cur_pred;
+                    }
+                    if (near.x == 0) dj = cur;
+                    if (cur > best_score) {
+                        best_score = cur;
+                        best_index = i;
+                        best_pos = here.x;
+                        best_key = s_key[i & 127];
+                    }
+                }
+                if (lane < m) {
+                    dp[b + i0 + lane] = high ? dB : dA;
+                    pred[b + i0 + lane] = my_pred;
+                }
+            }
+            __syncthreads();
+        }
+        if (threadIdx.x == 0) {
+            // a large cluster has at least three anchors (lane_max >= 2)
+            uint32_t* info = aux + 2 * total_anchors + b;
+            info[0] = lo + best_index;
+            info[1] = fire == 0xffffffffu ? fire : lo + fire;
+            info[2] = __float_as_uint(fire_best);
+            reinterpret_cast<float*>(aux + total_anchors + seg_b)[c] = best_score;
+        }
+    }
+}
+
+// The queued large clusters for longer lookbacks, a warp each, without the re-check.
+__global__ void __launch_bounds__(128) k_chain_big_far(const uint64_t* __restrict__ off, const uint64_t* seg_off,
+                                                       const uint64_t* dedup, float* dp, uint32_t* pred, uint32_t* aux,
+                                                       uint64_t total_anchors, AnchorPack ap, ChainCtx cc,
+                                                       const uint32_t* long_list, const uint32_t* long_n,
+                                                       const uint32_t* long_c, const uint32_t* big_items,
+                                                       const uint32_t* n_big) {
+    const uint32_t lane = lane_id();
     const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
     const uint32_t nb = *n_big;
-    for (uint32_t x = blockIdx.x * (blockDim.x / 32) + wib; x < nb; x += nwarps) {
+    for (uint32_t x = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; x < nb; x += nwarps) {
         const uint32_t u = big_items[2 * x], c = big_items[2 * x + 1];
         const uint32_t sg = long_list[u], N = long_n[u], C = long_c[u];
         const uint64_t b = seg_off[sg];
@@ -1479,11 +1840,91 @@ __global__ void __launch_bounds__(128) k_chain_big(const uint64_t* __restrict__ 
         float mx = 0.0f;
         uint32_t bi = 0xffffffffu;
         uint64_t bk = 0;
-        warp_chain_range<RING>(dedup, dp, pred, b, lo, hi, lo, max_ref_gap, cc, ap,
-                               ring_key_s + (RING ? wib * 64 : 0), ring_dp_s + (RING ? wib * 64 : 0), false, mx, bi,
-                               bk);
+        warp_chain_range(dedup, dp, pred, b, lo, hi, lo, max_ref_gap, cc, ap, false, mx, bi, bk);
         if (lane == 0) reinterpret_cast<float*>(aux + total_anchors + b)[c] = mx;
         __syncwarp();
+    }
+}
+
+// A long orientation per warp, its clusters scored by k_chain_long_prep (without the
+// re-check) and k_chain_big: in order, the clusters whose maximum beats the running best,
+// then the chains.  A kernel apart from k_chain4: the rings there take the shared memory
+// that the L1 needs here (the walks are chains of dependent loads; 300-500 cycles an
+// anchor from L2).
+template <bool RING>
+__global__ void __launch_bounds__(128) k_chain_long(const uint64_t* __restrict__ off, const uint64_t* seg_off,
+                                                    uint64_t* dedup, float* dp, uint32_t* pred, uint32_t* aux,
+                                                    uint64_t total_anchors, unsigned long long* scratch, AnchorPack ap,
+                                                    ChainCtx cc, NamRec* nam_out, uint32_t* nam_seg_count, uint64_t* anc_out,
+                                                    uint64_t* anc_start, const uint32_t* long_list, uint32_t n_long,
+                                                    const uint32_t* long_n, const uint32_t* long_c,
+                                                    uint32_t lane_max) {
+    __shared__ uint32_t hist[4 * 256];
+    constexpr uint32_t NONE = 0xffffffffu;
+    const uint32_t lane = lane_id(), wib = threadIdx.x / 32;
+    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
+    for (uint32_t u = blockIdx.x * (blockDim.x / 32) + wib; u < n_long; u += nwarps) {
+        const uint32_t sg = long_list[u], N = long_n[u];
+        const uint64_t b = seg_off[sg];
+        const uint32_t read_len = (uint32_t)(off[(sg >> 1) + 1] - off[sg >> 1]);
+        const uint32_t max_ref_gap = cc.cp.max_ref_gap ? cc.cp.max_ref_gap : read_len;
+        const uint32_t* cstart = aux + b;
+        const float* cmax = reinterpret_cast<const float*>(aux + total_anchors + b);
+        const uint32_t* info = aux + 2 * total_anchors + b;
+        const uint32_t C = long_c[u];
+        float best_score = 0.0f;
+        uint32_t best_index = NONE;
+        uint64_t best_key = 0;
+        for (uint32_t c0 = 0; c0 < C; c0 += 32) {
+            const uint32_t c = c0 + lane;
+            const float m = c < C ? cmax[c] : -INFINITY;
+            const uint32_t my_lo = c < C ? cstart[c] : 0, my_hi = c + 1 < C ? cstart[c + 1] : N;
+            const bool my_big = RING && c < C && my_hi - my_lo > lane_max;
+            const uint32_t my_fire = my_big ? info[my_lo + 1] : NONE;
+            uint32_t from = 0;
+            for (;;) {
+                // a cluster that its own re-check changed counts up to the score
+                // that a chain's end needs: below it, its anchors are in no chain
+                const bool rec = c < C && lane >= from &&
+                                 (best_index == NONE || m > best_score ||
+                                  (my_fire != NONE && !(m < __fmul_rn(best_score, cc.cp.valid_score_threshold))));
+                const uint32_t bal = __ballot_sync(FULL, rec);
+                if (!bal) break;
+                const uint32_t l = __ffs(bal) - 1;
+                from = l + 1;
+                const uint32_t lo = __shfl_sync(FULL, my_lo, l), hi = __shfl_sync(FULL, my_hi, l);
+                uint32_t i0;
+                if (__shfl_sync(FULL, my_big, l)) {
+                    i0 = __shfl_sync(FULL, my_fire, l);
+                    if (i0 == NONE || best_index == NONE || __uint_as_float(info[lo + 2]) > best_score) {
+                        // every score of the cluster stands
+                        const float cm = __shfl_sync(FULL, m, l);
+                        if (cm > best_score) {
+                            best_score = cm;
+                            best_index = info[lo];
+                            best_key = dedup[b + best_index];
+                        }
+                        continue;
+                    }
+                } else {
+                    // the values scored without the re-check stand up to the first
+                    // anchor where it would fire; only the rest is scored again
+                    i0 = recheck_first_fire(dedup, dp, b, lo, hi, max_ref_gap, cc, ap, best_score, best_index,
+                                            best_key);
+                }
+                if (i0 < hi) {
+                    if (RING)
+                        warp_chain_regs(dedup, dp, pred, b, i0, hi, lo, max_ref_gap, cc, ap, best_score, best_index,
+                                        best_key);
+                    else
+                        warp_chain_range(dedup, dp, pred, b, i0, hi, lo, max_ref_gap, cc, ap, true, best_score,
+                                         best_index, best_key);
+                }
+            }
+        }
+        __syncwarp();
+        chain_extract(dedup, dp, pred, aux, total_anchors, scratch, b, N, sg, best_score, ap, cc, nam_out,
+                      nam_seg_count, anc_out, anc_start, hist + wib * 256);
     }
 }
 
@@ -1492,10 +1933,7 @@ __global__ void __launch_bounds__(32 * CHAIN_WARPS, 8) k_chain4(const uint64_t* 
                                                 const uint64_t* sorted, uint64_t* dedup, float* dp, uint32_t* pred,
                                                 uint32_t* aux, uint64_t total_anchors, AnchorPack ap, ChainCtx cc,
                                                 NamRec* nam_out, uint32_t* nam_seg_count, uint64_t* anc_out,
-                                                uint64_t* anc_start, const uint32_t* seg_list, uint32_t n_list,
-                                                const uint32_t* long_list, uint32_t n_long, const uint32_t* long_n,
-                                                const uint32_t* long_c) {
-    __shared__ uint32_t hist[CHAIN_WARPS * 256];
+                                                uint64_t* anc_start, const uint32_t* seg_list, uint32_t n_list) {
     __shared__ uint64_t ring_key_s[RING ? CHAIN_WARPS * NG * 64 : 1];
     __shared__ float ring_dp_s[RING ? CHAIN_WARPS * NG * 64 : 1];
     const uint32_t lane = lane_id(), g = lane / CG, gl = lane % CG, gsh = CG * g;
@@ -1504,27 +1942,23 @@ __global__ void __launch_bounds__(32 * CHAIN_WARPS, 8) k_chain4(const uint64_t* 
     const uint64_t qmask = (1ULL << ap.qbits) - 1, pmask = (1ULL << ap.pbits) - 1;
     const float kf = __uint2float_rn(cc.k);
     constexpr uint32_t NONE = 0xffffffffu;
-    // units: the long orientations first (one per warp, so they start first), then the
-    // short ones NG at a time.  Lane q holds the q-th orientation's segment, anchor count
-    // after dedup, first anchor and best score.
-    const uint32_t n_units = n_long + (n_list + NG - 1) / NG;
+    // units of NG orientations.  Lane q holds the q-th orientation's segment, anchor count
+    // after dedup and first anchor.
+    const uint32_t n_units = (n_list + NG - 1) / NG;
     for (uint32_t u = blockIdx.x * (blockDim.x / 32) + wib; u < n_units; u += nwarps) {
         uint32_t my_sg = NONE;
-        if (u < n_long) {
-            if (lane == 0) my_sg = long_list[u];
-        } else {
-            const uint32_t l = NG * (u - n_long) + lane;
+        {
+            const uint32_t l = NG * u + lane;
             if (lane < NG && l < n_list) my_sg = seg_list[l];
         }
-        // dedup (src/chainer.rs:228-229), one orientation after the other; the long
-        // orientations were deduplicated by k_chain_long_prep
+        // dedup (src/chainer.rs:228-229), one orientation after the other
         uint32_t my_n = 0;
         uint64_t my_b = 0;
         for (uint32_t q = 0; q < NG; q++) {
             const uint32_t sg = __shfl_sync(FULL, my_sg, q);
             if (sg == NONE) continue;
             const uint64_t b = seg_off[sg], e = seg_off[sg + 1];
-            const uint32_t N = u < n_long ? long_n[u] : orientation_dedup(sorted, dedup, b, e);
+            const uint32_t N = orientation_dedup(sorted, dedup, b, e);
             if (lane == q) {
                 my_n = N;
                 my_b = b;
@@ -1532,8 +1966,7 @@ __global__ void __launch_bounds__(32 * CHAIN_WARPS, 8) k_chain4(const uint64_t* 
         }
         __syncwarp();
         const uint32_t nmax = __reduce_max_sync(FULL, my_n);
-        float my_best = 0.0f;
-        if (u >= n_long && nmax <= CHAIN_GROUP_MAX) {
+        {
             // grouped DP: group g scores the g-th orientation
             const uint32_t sg = __shfl_sync(FULL, my_sg, g);
             const uint32_t N = __shfl_sync(FULL, my_n, g);
@@ -1626,68 +2059,10 @@ __global__ void __launch_bounds__(32 * CHAIN_WARPS, 8) k_chain4(const uint64_t* 
                 }
                 __syncwarp();
             }
-            const float bs = __shfl_sync(FULL, best_score, (lane % NG) * CG);
-            if (lane < NG) my_best = bs;
             // the eight extractions side by side, a group each
             __syncwarp();
             group_chain_extract(dedup, dp, pred, aux, total_anchors, b, N, nmax, sg, best_score, ap, cc, nam_out,
                                 nam_seg_count, anc_out, anc_start);
-            continue;
-        } else {
-            // a long orientation (k_chain_long_prep and k_chain_big scored its clusters
-            // without the re-check): the clusters whose maximum beats the running best,
-            // in order, again with the re-check
-            uint64_t* ring_key = ring_key_s + (RING ? wib * NG * 64 : 0);
-            float* ring_dp = ring_dp_s + (RING ? wib * NG * 64 : 0);
-            for (uint32_t q = 0; q < NG; q++) {
-                const uint32_t sg = __shfl_sync(FULL, my_sg, q), N = __shfl_sync(FULL, my_n, q);
-                const uint64_t b = __shfl_sync(FULL, my_b, q);
-                if (sg == NONE || N == 0) continue;
-                const uint32_t read_len = (uint32_t)(off[(sg >> 1) + 1] - off[sg >> 1]);
-                const uint32_t max_ref_gap = cc.cp.max_ref_gap ? cc.cp.max_ref_gap : read_len;
-                const uint32_t* cstart = aux + b;
-                const float* cmax = reinterpret_cast<const float*>(aux + total_anchors + b);
-                const uint32_t C = long_c[u];
-                // in order: clusters whose maximum beats the running best, scored again
-                float best_score = 0.0f;
-                uint32_t best_index = 0xffffffffu;
-                uint64_t best_key = 0;
-                for (uint32_t c0 = 0; c0 < C; c0 += 32) {
-                    const uint32_t c = c0 + lane;
-                    const float m = c < C && c > 0 ? cmax[c] : -INFINITY;
-                    uint32_t from = 0;
-                    for (;;) {
-                        const bool rec = c < C && lane >= from && (best_index == 0xffffffffu || m > best_score);
-                        const uint32_t bal = __ballot_sync(FULL, rec);
-                        if (!bal) break;
-                        const uint32_t l = __ffs(bal) - 1, cc0 = c0 + l;
-                        const uint32_t lo = cstart[cc0], hi = cc0 + 1 < C ? cstart[cc0 + 1] : N;
-                        // the values scored without the re-check stand up to the first
-                        // anchor where it would fire; only the rest is scored again
-                        const uint32_t i0 = recheck_first_fire(dedup, dp, b, lo, hi, max_ref_gap, cc, ap, best_score,
-                                                               best_index, best_key);
-                        if (i0 < hi)
-                            warp_chain_range<RING>(dedup, dp, pred, b, i0, hi, lo, max_ref_gap, cc, ap, ring_key,
-                                                   ring_dp, true, best_score, best_index, best_key);
-                        from = l + 1;
-                    }
-                }
-                if (lane == q) my_best = best_score;
-                __syncwarp();
-            }
-        }
-        __syncwarp();
-        for (uint32_t q = 0; q < NG; q++) {
-            const uint32_t sg = __shfl_sync(FULL, my_sg, q), N = __shfl_sync(FULL, my_n, q);
-            const uint64_t b = __shfl_sync(FULL, my_b, q);
-            const float best = __shfl_sync(FULL, my_best, q);
-            if (sg == NONE) continue;
-            if (N == 0) {
-                if (lane == 0) nam_seg_count[sg] = 0;
-                continue;
-            }
-            chain_extract(dedup, dp, pred, aux, total_anchors, b, N, sg, best, ap, cc, nam_out,
-                          nam_seg_count, anc_out, anc_start, hist + wib * 256);
         }
     }
 }
@@ -2054,48 +2429,49 @@ uint32_t run_nam_pipeline(const DevIndex& ix, const DevRefs& refs, const NamConf
     }
     kt->begin(KS_CHAIN, st);
     SA_CUDA(cudaMemsetAsync(ws.nam_seg_count.p, 0, 2 * (size_t)n * sizeof(uint32_t), st));
-    const uint64_t chain_units = (uint64_t)n_list[2] + ((uint64_t)n_list[0] + NG - 1) / NG;
+    const uint64_t chain_units = ((uint64_t)n_list[0] + NG - 1) / NG;
     const unsigned chain_grid = (unsigned)std::max<uint64_t>(
         1, std::min<uint64_t>((chain_units + CHAIN_WARPS - 1) / CHAIN_WARPS, sm_count() * 64));
     if (cfg.nam_anchors) {
         ws.anc_sparse.reserve(3 * total_anchors + 1);
         ws.anc_start.reserve(total_anchors + 1);
     }
-    // long orientations: dedup, clusters and their first scoring, before k_chain4
+    uint64_t* const anc_out = cfg.nam_anchors ? ws.anc_sparse.p : nullptr;
+    uint64_t* const anc_start = cfg.nam_anchors ? ws.anc_start.p : nullptr;
+    // The long orientations' kernels last as long as the longest cluster's serial chain,
+    // with most of the device idle: they run beside the short ones' k_chain4.
     uint32_t* const long_n = ws.seg_key_alt.p;
     uint32_t* const long_c = ws.seg_key_alt.p + 2 * (size_t)n;
+    // a large cluster has three words of BigCluster at its first anchors
+    const uint32_t lane_max = std::max<uint32_t>(2, cfg.chain_lane_max);
+    const bool ring = cfg.cp.max_lookback < 64;
     if (n_list[2]) {
-        const uint32_t lane_max = std::max<uint32_t>(1, cfg.chain_lane_max);
         const uint64_t cap = total_anchors / (lane_max + 1) + 1;
         ws.chain_big.reserve(2 * cap + 2);
-        SA_CUDA(cudaMemsetAsync(ws.chain_big.p, 0, 4, st));
+        const cudaStream_t sl = ws.side.fork(st);
+        SA_CUDA(cudaMemsetAsync(ws.chain_big.p, 0, 4, sl));
         const unsigned pgrid = (unsigned)std::min<uint64_t>(((uint64_t)n_list[2] + 3) / 4, sm_count() * 16);
-        k_chain_long_prep<<<pgrid, 128, 0, st>>>(ws.off.p, ws.seg_off.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p,
+        k_chain_long_prep<<<pgrid, 128, 0, sl>>>(ws.off.p, ws.seg_off.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p,
                                                  ws.pred.p, ws.aux.p, total_anchors, ap, cc, long_sorted, n_list[2],
                                                  long_n, long_c, ws.chain_big.p + 2, ws.chain_big.p, lane_max);
         const unsigned bgrid = (unsigned)(sm_count() * 8);
-        if (cfg.cp.max_lookback < 64)
-            k_chain_big<true><<<bgrid, 128, 0, st>>>(ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p,
-                                                     ws.aux.p, total_anchors, ap, cc, long_sorted, long_n, long_c,
-                                                     ws.chain_big.p + 2, ws.chain_big.p);
-        else
-            k_chain_big<false><<<bgrid, 128, 0, st>>>(ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p,
-                                                      ws.aux.p, total_anchors, ap, cc, long_sorted, long_n, long_c,
-                                                      ws.chain_big.p + 2, ws.chain_big.p);
-        launches += 2;
+        (ring ? k_chain_big : k_chain_big_far)<<<bgrid, 128, 0, sl>>>(
+            ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p, total_anchors, ap, cc, long_sorted,
+            long_n, long_c, ws.chain_big.p + 2, ws.chain_big.p);
+        (ring ? k_chain_long<true> : k_chain_long<false>)<<<pgrid, 128, 0, sl>>>(
+            ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p, total_anchors,
+            reinterpret_cast<unsigned long long*>(ws.anchors_sorted.p), ap, cc, ws.nam_scratch.p, ws.nam_seg_count.p,
+            anc_out, anc_start, long_sorted, n_list[2], long_n, long_c, lane_max);
+        launches += 3;
     }
-    if (cfg.cp.max_lookback < 64)
-        k_chain4<true><<<chain_grid, 32 * CHAIN_WARPS, 0, st>>>(
+    if (n_list[0]) {
+        (ring ? k_chain4<true> : k_chain4<false>)<<<chain_grid, 32 * CHAIN_WARPS, 0, st>>>(
             ws.off.p, n, ws.seg_off.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p,
-            total_anchors, ap, cc, ws.nam_scratch.p, ws.nam_seg_count.p, cfg.nam_anchors ? ws.anc_sparse.p : nullptr,
-            cfg.nam_anchors ? ws.anc_start.p : nullptr, short_list, n_list[0], long_sorted, n_list[2], long_n, long_c);
-    else
-        k_chain4<false><<<chain_grid, 32 * CHAIN_WARPS, 0, st>>>(
-            ws.off.p, n, ws.seg_off.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p,
-            total_anchors, ap, cc, ws.nam_scratch.p, ws.nam_seg_count.p, cfg.nam_anchors ? ws.anc_sparse.p : nullptr,
-            cfg.nam_anchors ? ws.anc_start.p : nullptr, short_list, n_list[0], long_sorted, n_list[2], long_n, long_c);
+            total_anchors, ap, cc, ws.nam_scratch.p, ws.nam_seg_count.p, anc_out, anc_start, short_list, n_list[0]);
+        launches++;
+    }
+    if (n_list[2]) ws.side.join(st);
     kt->end(st);
-    launches++;
     ws.nam_count.reserve((size_t)n + 1);
     ws.nam_off.reserve((size_t)n + 1);
     kt->begin(KS_NAMS_OTHER, st);

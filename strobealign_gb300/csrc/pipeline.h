@@ -64,6 +64,7 @@ struct NamWorkspace {
     uint64_t last_total_nam_anchors = 0;
     DevBuf<uint8_t> cub_tmp;
     DevBuf<float> log2_lut;
+    SideStream side;  // the long orientations' chaining
     uint64_t last_total_nams = 0;
     uint32_t anchor_qbits = 0, anchor_pbits = 0;
 };
