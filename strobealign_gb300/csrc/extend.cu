@@ -21,6 +21,7 @@
 #include <type_traits>
 
 #include "extend.h"
+#include "ssw16.h"
 
 namespace sa {
 
@@ -1108,9 +1109,11 @@ __device__ __noinline__ EndPos ssw_warp_pass(const uint8_t* q, int qlen, bool q_
 // the shortest-read variant fits 5 blocks per SM without spills (96 registers)
 template <int RMAX>
 __global__ void __launch_bounds__(128, RMAX <= 4 ? 5 : 1) k_ssw(SswTask* tasks, const uint32_t* order, uint32_t n_tasks,
-                                             const PrepRec* prep, const uint8_t* arena, AlignScores sc, int bias,
-                                             uint32_t* counters, uint32_t* queue, uint32_t qmin) {
+                                             const uint32_t* n_tasks_ptr, const PrepRec* prep, const uint8_t* arena,
+                                             AlignScores sc, int bias, uint32_t* counters, uint32_t* queue,
+                                             uint32_t qmin) {
     constexpr int RW = (RMAX + 3) / 4;
+    if (n_tasks_ptr) n_tasks = *n_tasks_ptr;
     extern __shared__ __align__(16) uint32_t ssw_smem[];
     const int lane = threadIdx.x & 31;
     uint32_t* prof = ssw_smem + (threadIdx.x / 32) * (5 * 32 * RW);
@@ -1123,7 +1126,7 @@ __global__ void __launch_bounds__(128, RMAX <= 4 ? 5 : 1) k_ssw(SswTask* tasks, 
         const uint32_t ti = order ? order[li] : li;
         SswTask tk = tasks[ti];
         const PrepRec p = prep[tk.job];
-        if (p.qlen <= qmin) continue;  // k_ssw_wave's task
+        if (p.qlen <= qmin) continue;  // another kernel's task
         const uint8_t* q = arena + p.arena_off;
         const uint8_t* r = q + p.qlen;
         // forward: byte, word on overflow (ext/ssw/ssw.c:840-862)
@@ -1200,15 +1203,9 @@ constexpr int WV_SCALE = 8;  // log2 of the score scale (rows < 256)
 struct WaveScores {
     int gO, gE;  // scaled
 };
-// the default gap penalties (12, 1) as constants: the per-row offsets of the lazy-F
-// raise become immediates and the penalties leave the registers
-struct DefaultWaveScores {
-    static constexpr int gO = 12 << WV_SCALE, gE = 1 << WV_SCALE;
-};
-
-template <int N, bool BYTE, class WS>
+template <int N, bool BYTE>
 __device__ __forceinline__ EndPos wave_loop(const uint8_t* r, int rlen, bool r_rev, int qlen, bool check_term,
-                                            int terminate, int bias, WS ws, const uint4* prof, int gl,
+                                            int terminate, int bias, WaveScores ws, const uint4* prof, int gl,
                                             unsigned m, bool run) {
     constexpr int NW = (N + 7) / 8;
     int H[N], E[N];
@@ -1323,7 +1320,7 @@ __device__ __forceinline__ EndPos wave_loop(const uint8_t* r, int rlen, bool r_r
 // per thread.  All 32 threads enter together.  When the running groups share N, the
 // warp runs them in lockstep (full-warp shuffles and votes); otherwise each group runs
 // on its own with its own mask.
-template <int NMAX, bool BYTE, bool DEF>
+template <int NMAX, bool BYTE>
 __device__ __forceinline__ EndPos wave_pass(bool run, const uint8_t* q, int qlen, bool q_rev, const uint8_t* r, int rlen,
                             bool r_rev, bool check_term, int terminate, const AlignScores& sc, int bias, uint4* prof,
                             int gl, unsigned gm) {
@@ -1363,15 +1360,13 @@ __device__ __forceinline__ EndPos wave_pass(bool run, const uint8_t* q, int qlen
                 prof[(b * nw + w) * 32] = make_uint4(v[0], v[1], v[2], v[3]);
             }
     }
-    using WS = std::conditional_t<DEF, DefaultWaveScores, WaveScores>;
-    WS ws{};
-    if constexpr (!DEF) ws = WaveScores{(int)sc.gap_open << WV_SCALE, (int)sc.gap_extend << WV_SCALE};
+    const WaveScores ws{(int)sc.gap_open << WV_SCALE, (int)sc.gap_extend << WV_SCALE};
     EndPos res = z;
     // byte mode: N is even, so the odd cases are never taken there
 #define SA_WV(K)                                                                                                 \
     case K:                                                                                                      \
         if constexpr (K <= NMAX && (!BYTE || K % 2 == 0))                                                        \
-            res = wave_loop<K, BYTE, WS>(r, rlen, r_rev, qlen, check_term, terminate, bias, ws, prof, gl, m, run); \
+            res = wave_loop<K, BYTE>(r, rlen, r_rev, qlen, check_term, terminate, bias, ws, prof, gl, m, run); \
         break;
     switch (NN) {
         SA_WV(1) SA_WV(2) SA_WV(3) SA_WV(4) SA_WV(5) SA_WV(6) SA_WV(7) SA_WV(8)
@@ -1441,10 +1436,10 @@ __device__ __forceinline__ int wave_diag_bound(bool run, const uint8_t* q, int q
 // the longest-first order of k_ssw: each warp takes four consecutive tasks (one per
 // group of eight threads) and runs the forward byte pass, the forward word pass of the
 // tasks that overflowed, then the reverse passes in each task's mode.
-template <int NMAX, bool DEF>
+template <int NMAX>
 __global__ void __launch_bounds__(128, NMAX <= 20 ? 5 : 4) k_ssw_wave(SswTask* tasks, const uint32_t* order, uint32_t n_tasks,
                                                       const PrepRec* prep, const uint8_t* arena, AlignScores sc,
-                                                      int bias, uint32_t* counters, uint32_t qmax) {
+                                                      int bias, uint32_t* counters, uint32_t qmin, uint32_t qmax) {
     constexpr int NW = (NMAX + 7) / 8;
     extern __shared__ __align__(16) uint4 wv_smem[];
     const int lane = threadIdx.x & 31, gi = lane / WV_T, gl = lane % WV_T;
@@ -1462,7 +1457,8 @@ __global__ void __launch_bounds__(128, NMAX <= 20 ? 5 : 4) k_ssw_wave(SswTask* t
         bool have = li < n_tasks;
         if (have) {
             ti = order ? order[li] : li;
-            have = prep[tasks[ti].job].qlen <= qmax;  // longer reads: k_ssw's task
+            const uint32_t ql = prep[tasks[ti].job].qlen;
+            have = ql > qmin && ql <= qmax;  // the others are another kernel's tasks
         }
         int qlen = 0, wlen = 0;
         const uint8_t* q = arena;
@@ -1481,10 +1477,10 @@ __global__ void __launch_bounds__(128, NMAX <= 20 ? 5 : 4) k_ssw_wave(SswTask* t
         if (__any_sync(FULLM, try_bound))
             certain = wave_diag_bound(try_bound, q, qlen, r, wlen, (int)d0, sc, gl) >= 255 - bias;
         // forward: byte, word on overflow (ext/ssw/ssw.c:840-862)
-        EndPos e = wave_pass<NMAX, true, DEF>(have && !certain, q, qlen, false, r, wlen, false, false, 0, sc, bias, prof, gl,
+        EndPos e = wave_pass<NMAX, true>(have && !certain, q, qlen, false, r, wlen, false, false, 0, sc, bias, prof, gl,
                                          gm);
         const bool word = have && (certain || e.score == 255);
-        const EndPos ew = wave_pass<NMAX, false, DEF>(word, q, qlen, false, r, wlen, false, false, 0, sc, bias, prof, gl,
+        const EndPos ew = wave_pass<NMAX, false>(word, q, qlen, false, r, wlen, false, false, 0, sc, bias, prof, gl,
                                                  gm);
         unsigned long long c_fb = certain ? 0 : (unsigned long long)qlen * e.cols, c_fw = 0, c_rb = 0, c_rw = 0;
         if (word) {
@@ -1493,9 +1489,9 @@ __global__ void __launch_bounds__(128, NMAX <= 20 ? 5 : 4) k_ssw_wave(SswTask* t
         }
         // reverse pass over read[0..=read_end1] and ref[0..=ref_end1] (ext/ssw/ssw.c:870-888)
         const bool rev = have && e.ref >= 0;
-        const EndPos bb = wave_pass<NMAX, true, DEF>(rev && !word, q, e.read + 1, true, r, e.ref + 1, true, true, e.score,
+        const EndPos bb = wave_pass<NMAX, true>(rev && !word, q, e.read + 1, true, r, e.ref + 1, true, true, e.score,
                                                 sc, bias, prof, gl, gm);
-        const EndPos bw = wave_pass<NMAX, false, DEF>(rev && word, q, e.read + 1, true, r, e.ref + 1, true, true, e.score,
+        const EndPos bw = wave_pass<NMAX, false>(rev && word, q, e.read + 1, true, r, e.ref + 1, true, true, e.score,
                                                  sc, bias, prof, gl, gm);
         EndPos b = word ? bw : bb;
         if (!rev) {
@@ -1523,12 +1519,17 @@ __global__ void __launch_bounds__(128, NMAX <= 20 ? 5 : 4) k_ssw_wave(SswTask* t
     }
 }
 
-// window length of each task, for the longest-first order of k_ssw
+// Each task's key for the order the SSW kernels take them in: largest first (in steps of a
+// quarter octave of cells), reads of one length together (the groups of a warp then have
+// the same number of rows).
 __global__ void k_task_keys(const SswTask* tasks, uint32_t n, const PrepRec* prep, uint32_t* key, uint32_t* idx) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const PrepRec p = prep[tasks[i].job];
-        const uint32_t cells = p.wlen * (p.qlen + 1) >> 7;  // < 2^16 for windows <= 2000, queries <= 2048
-        key[i] = 0xffffu - (cells < 0xffffu ? cells : 0xffffu);  // ascending: largest first
+        const uint64_t c64 = (uint64_t)p.wlen * (p.qlen + 1) | 4;
+        const uint32_t cells = c64 < 0xffffffffu ? (uint32_t)c64 : 0xffffffffu;
+        const uint32_t lg = 31 - __clz(cells), step = 4 * (lg - 2) + ((cells >> (lg - 2)) & 3);  // lg >= 2
+        const uint32_t q = p.qlen < 511 ? p.qlen : 511;
+        key[i] = (127 - step) << 9 | (511 - q);  // 16 bits, ascending: largest first
         idx[i] = i;
     }
 }
@@ -3270,20 +3271,25 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
             const int wpb = tpb / 32;
             uint64_t blocks = ((uint64_t)n_tasks + wpb - 1) / wpb;
             if (blocks > sm_count() * 16) blocks = sm_count() * 16;
-#define SA_SSW(RM)                                                                                              \
-    k_ssw<RM><<<(unsigned)blocks, tpb, (size_t)wpb * 5 * 32 * ((RM + 3) / 4) * 4, st>>>(                       \
-        ws.tasks.p, ws.order.p, n_tasks, ws.prep.p, ws.arena.p, sc, bias, ws.counters.p, ws.counters.p + 21, \
-        wave_qmax)
-            // tasks of reads up to wave_qmax (at most 192) nt: eight threads per task; the
-            // longer ones of a batch of mixed lengths a warp per task, in a launch before
+#define SA_SSW(RM, ORDER, N_PTR, QUEUE, BLOCKS, QMIN)                                                            \
+    k_ssw<RM><<<(unsigned)(BLOCKS), tpb, (size_t)wpb * 5 * 32 * ((RM + 3) / 4) * 4, st>>>(                      \
+        ws.tasks.p, ORDER, n_tasks, N_PTR, ws.prep.p, ws.arena.p, sc, bias, ws.counters.p, ws.counters.p + QUEUE, \
+        QMIN)
+            // Reads up to q16 nt go to the packed 16-bit kernel, where their scores fit (default
+            // scores: 511 nt); of the others those up to wave_qmax (at most 192) nt to the
+            // lane wavefront in 32 bits, and the rest a warp per task.  A wave_qmax below its
+            // largest value keeps longer reads off both wavefronts.
             const uint32_t wave_qmax = std::min<uint32_t>(ws.wave_qmax, 8 * WAVE_NMAX);
-            if (max_qlen > wave_qmax) {
-                if (rmax == 4) SA_SSW(4);
-                else if (rmax == 8) SA_SSW(8);
-                else SA_SSW(16);
+            uint32_t q16 = ssw16_max_qlen(sc);
+            if (wave_qmax < 8 * WAVE_NMAX) q16 = std::min(q16, wave_qmax);
+            const uint32_t qmin = std::max(q16, wave_qmax);
+            if (max_qlen > qmin) {
+                if (rmax == 4) SA_SSW(4, ws.order.p, nullptr, 21, blocks, qmin);
+                else if (rmax == 8) SA_SSW(8, ws.order.p, nullptr, 21, blocks, qmin);
+                else SA_SSW(16, ws.order.p, nullptr, 21, blocks, qmin);
                 launches++;
             }
-            {
+            if (q16 < wave_qmax && max_qlen > q16) {
                 const uint64_t per_block = (uint64_t)wpb * (32 / WV_T);  // tasks per block and round
                 uint64_t wblocks = ((uint64_t)n_tasks + per_block - 1) / per_block;
                 if (wblocks > sm_count() * 16) wblocks = sm_count() * 16;
@@ -3291,19 +3297,27 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
                 const bool short_reads = std::min<uint32_t>(max_qlen, wave_qmax) <= 8 * WAVE_NMAX_SHORT;
                 const int nmax = short_reads ? WAVE_NMAX_SHORT : WAVE_NMAX;
                 const size_t smem = (size_t)wpb * 5 * ((nmax + 7) / 8) * 32 * sizeof(uint4);
-                const bool def_gaps = sc.gap_open == 12 && sc.gap_extend == 1;
-#define SA_SSWW(NM, DF)                                                                                      \
-    k_ssw_wave<NM, DF><<<(unsigned)wblocks, tpb, smem, st>>>(ws.tasks.p, ws.order.p, n_tasks, ws.prep.p,   \
-                                                             ws.arena.p, sc, bias, ws.counters.p, wave_qmax)
-                if (short_reads && def_gaps) SA_SSWW(WAVE_NMAX_SHORT, true);
-                else if (short_reads) SA_SSWW(WAVE_NMAX_SHORT, false);
-                else if (def_gaps) SA_SSWW(WAVE_NMAX, true);
-                else SA_SSWW(WAVE_NMAX, false);
+#define SA_SSWW(NM)                                                                                       \
+    k_ssw_wave<NM><<<(unsigned)wblocks, tpb, smem, st>>>(ws.tasks.p, ws.order.p, n_tasks, ws.prep.p,    \
+                                                         ws.arena.p, sc, bias, ws.counters.p, q16, wave_qmax)
+                if (short_reads) SA_SSWW(WAVE_NMAX_SHORT);
+                else SA_SSWW(WAVE_NMAX);
 #undef SA_SSWW
+                launches++;
+            }
+            if (q16) {
+                const Ssw16Args a{ws.tasks.p, ws.order.p, n_tasks, ws.prep.p, ws.arena.p, sc, bias, ws.counters.p, q16,
+                                  ws.list_word.p, ws.counters.p + 31, st};
+                launch_ssw16(a, std::min(max_qlen, q16));
+                // the tasks whose reverse pass went beyond the forward score
+                if (rmax == 4) SA_SSW(4, ws.list_word.p, ws.counters.p + 31, 23, sm_count(), 0);
+                else if (rmax == 8) SA_SSW(8, ws.list_word.p, ws.counters.p + 31, 23, sm_count(), 0);
+                else SA_SSW(16, ws.list_word.p, ws.counters.p + 31, 23, sm_count(), 0);
+                launches += 2;
             }
 #undef SA_SSW
             kt->end(st);
-            launches += 3;
+            launches += 2;
         } else {
         // forward byte pass over all tasks
         kt->begin(KS_SW_BYTE, st);

@@ -1,0 +1,38 @@
+// The packed 16-bit SSW kernel (ssw16.cuh).
+#pragma once
+#include "extend.h"
+
+namespace sa {
+
+constexpr uint32_t SSW16_MAX_QLEN = 511;
+// below this many tasks a block's two warps share a task's byte and word passes
+constexpr uint32_t SSW16_PAIR_TASKS = 4096;
+
+struct Ssw16Args {
+    SswTask* tasks;
+    const uint32_t* order;
+    uint32_t n_tasks;
+    const PrepRec* prep;
+    const uint8_t* arena;
+    AlignScores sc;
+    int bias;
+    uint32_t* counters;
+    uint32_t qmax;     // tasks of longer reads are left to another kernel
+    uint32_t* redo;    // tasks to run again on the warp-per-task kernel, and their count
+    uint32_t* n_redo;
+    cudaStream_t st;
+};
+
+// The longest read whose scores fit (0: these scores do not).  Scores are scaled by 32 in
+// 16 bits: match * L <= 1022 keeps every H with its row key below 2^15.  The other limits
+// keep the raise's row offsets (gap_extend <= 31, and no more than a lane's rows add
+// to the score) and a word pass's first lane of two rows or more (a byte pass overflows at
+// 255 - mismatch, which takes 12 rows or more) within what the kernel assumes; the
+// lazy-F raise is exact for gap_open > gap_extend.
+uint32_t ssw16_max_qlen(const AlignScores& sc);
+
+// The end searches of every task of a read up to a.qmax nt; longest: the longest such read.
+void launch_ssw16(const Ssw16Args& a, uint32_t longest);
+void launch_ssw16_pair(const Ssw16Args& a, uint32_t longest);
+
+}  // namespace sa
