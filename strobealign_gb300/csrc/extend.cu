@@ -4,16 +4,17 @@
 //
 //   k_prepare   thread per job: NAM consistency / orientation repair
 //               (src/nam.rs:49-135), projected window, Hamming eligibility
-//   k_fill      thread per job: Hamming fast path (src/aligner.rs:166-259) or the
-//               SSW task's query and reference bytes
+//   k_fill      thread per job: Hamming fast path (src/aligner.rs:166-259), or an SSW /
+//               piecewise task (its query and reference bytes: k_copy, a warp per task)
 //   k_sw        SSW (ext/ssw/ssw.c:163-596) with the library's striped semantics:
 //               one lane per SSE lane, 16 lanes per task in byte mode and 8 in word
 //               mode, so 2 resp. 4 tasks per warp; the lazy-F pass leaves E alone
 //               and byte mode reruns in word mode once max + bias >= 255
-//   k_ssw_wave  the same passes for reads up to 192 nt: eight threads per task, one
-//               or two SSE lanes per thread, a wavefront over the reference columns
-//   k_band_*    banded_sw (ext/ssw/ssw.c:598-769): band doubling, then the final
-//               pass with directions and the traceback, one thread per task
+//   k_ssw16     the same passes in packed 16-bit scores for reads up to 511 nt
+//               (ssw16.cuh); k_ssw_wave up to 192 nt in 32 bits and k_ssw a warp per
+//               task where the scores do not fit
+//   k_band_*    banded_sw (ext/ssw/ssw.c:598-769): band doubling with directions, then the
+//               traceback; a thread per task for narrow bands, a warp for the others
 //   k_finalize  M -> =/X (src/cigar.rs:149-187), edit distance and the end-bonus
 //               extension of Aligner::align
 #include <cub/cub.cuh>
@@ -276,7 +277,8 @@ __global__ void k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restr
             ab = (uint64_t)L + p.wlen;
             cap = 2ull * L + p.wlen + 4;
             uint64_t len = L > p.wlen ? L : p.wlen;
-            hs = 3 * (2 * len + 8);
+            // the literal pass's three rows; k_band_small's words of three widths, maxima, CIGAR
+            hs = 8 * len + 24;
         }
         p.cigar_cap = (uint32_t)cap;
         res[t] = r;
@@ -379,35 +381,23 @@ __device__ __forceinline__ uint32_t hamming_cigar_bits(const uint32_t* bits, uin
     return mm;
 }
 
-// A warp takes 32 consecutive jobs, a lane each.  Hamming jobs (hamming_align,
-// src/aligner.rs:181-259) run on their lane: the match bits of the read against the
-// reference, 32 bases per pair of packed reference words, then the best segment and its
-// =/X runs from the bits.  The SSW / piecewise jobs' query and reference window bytes are
-// copied into the arena by the whole warp, one job after another.
+// A thread per job: Hamming jobs (hamming_align, src/aligner.rs:181-259) are run (the match
+// bits of the read against the reference, 32 bases per pair of packed reference words, then
+// the best segment and its =/X runs from the bits); SSW and piecewise jobs are listed for
+// k_copy.
 __global__ void __launch_bounds__(256) k_fill(const ExtJob* jobs, uint32_t n, const uint8_t* __restrict__ seq,
-                                              const uint64_t* __restrict__ off, DevRefs R, const uint8_t* raw_refs,
-                                              const uint64_t* raw_off, AlignScores sc, PrepRec* prep,
-                                              const uint64_t* off_arena, const uint64_t* off_cigar,
-                                              const uint64_t* off_h, uint8_t* arena, uint32_t* cigar, ExtResult* res,
-                                              SswTask* tasks, uint32_t* counters, uint32_t* pw_list) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t b0 = (blockIdx.x * blockDim.x + threadIdx.x) / 32 * 32; b0 < n; b0 += nwarps * 32) {
-        const uint32_t t = b0 + lane;
-        PrepRec p{};
-        uint64_t s_off = 0;
-        bool align_raw = false;
-        if (t < n) {
-            p = prep[t];
-            p.arena_off = off_arena[t];
-            p.cigar_off = off_cigar[t];
-            p.h_off = off_h[t];
-            prep[t] = p;
-            s_off = off[p.read];
-            align_raw = p.type == 2 && jobs[t].kind == JOB_ALIGN;
-        }
-        if (t < n && p.type == 1) {
-            const uint8_t* s = seq + s_off;
+                                              const uint64_t* __restrict__ off, DevRefs R, AlignScores sc,
+                                              PrepRec* prep, const uint64_t* off_arena, const uint64_t* off_cigar,
+                                              const uint64_t* off_h, uint32_t* cigar, ExtResult* res, SswTask* tasks,
+                                              uint32_t* counters, uint32_t* pw_list) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        PrepRec p = prep[t];
+        p.arena_off = off_arena[t];
+        p.cigar_off = off_cigar[t];
+        p.h_off = off_h[t];
+        prep[t] = p;
+        if (p.type == 1) {
+            const uint8_t* s = seq + off[p.read];
             const uint32_t L = p.qlen;
             uint32_t bits[MAX_READ_LEN / 32];
             const uint32_t nw = (L + 31) / 32;
@@ -435,42 +425,48 @@ __global__ void __launch_bounds__(256) k_fill(const ExtJob* jobs, uint32_t n, co
             r.cigar_offset = (uint32_t)p.cigar_off;
             r.cigar_len = cw.n;
             res[t] = r;
+        } else if (p.type == 3) {
+            pw_list[atomicAdd(&counters[19], 1u)] = t;
+        } else if (p.type == 2) {
+            const uint32_t ti = atomicAdd(&counters[0], 1u);
+            atomicAdd(reinterpret_cast<unsigned long long*>(counters + 8), (unsigned long long)p.qlen * p.wlen);
+            SswTask tk{};
+            tk.job = t;
+            tk.raw_off = RAW_FALLBACK;
+            tk.ref_begin1 = -1;
+            tk.read_begin1 = -1;
+            tasks[ti] = tk;
         }
-        // the copies, a job at a time by the whole warp
-        uint32_t todo = __ballot_sync(FULLM, t < n && (p.type == 2 || p.type == 3));
-        while (todo) {
-            const int src = __ffs(todo) - 1;
-            todo &= todo - 1;
-            const uint32_t jt = b0 + (uint32_t)src;
-            const uint64_t aoff = __shfl_sync(FULLM, (unsigned long long)p.arena_off, src);
-            const uint64_t so = __shfl_sync(FULLM, (unsigned long long)s_off, src);
-            const uint32_t L = __shfl_sync(FULLM, p.qlen, src), rcf = __shfl_sync(FULLM, p.rc, src);
-            const uint32_t wlen = __shfl_sync(FULLM, p.wlen, src), wstart = __shfl_sync(FULLM, p.wstart, src);
-            const uint32_t ref_id = __shfl_sync(FULLM, p.ref_id, src), type = __shfl_sync(FULLM, p.type, src);
-            const bool raw = __shfl_sync(FULLM, align_raw, src);
-            const uint8_t* s = seq + so;
-            uint8_t* q = arena + aoff;
-            for (uint32_t i = lane; i < L; i += 32) q[i] = read_char(s, L, i, rcf);
-            uint8_t* w = q + L;
-            if (raw) {
-                const uint8_t* rr = raw_refs + raw_off[ref_id];
-                for (uint32_t i = lane; i < wlen; i += 32) w[i] = rr[i];
-            } else {
-                for (uint32_t i = lane; i < wlen; i += 32) w[i] = ref_base(R, ref_id, (uint64_t)wstart + i);
-            }
-            if (lane == (uint32_t)src) {
-                if (type == 3) {
-                    pw_list[atomicAdd(&counters[19], 1u)] = jt;
-                } else {
-                    uint32_t ti = atomicAdd(&counters[0], 1u);
-                    atomicAdd(reinterpret_cast<unsigned long long*>(counters + 8), (unsigned long long)L * wlen);
-                    SswTask tk{};
-                    tk.job = jt;
-                    tk.raw_off = RAW_FALLBACK;
-                    tk.ref_begin1 = -1;
-                    tk.read_begin1 = -1;
-                    tasks[ti] = tk;
-                }
+    }
+}
+
+// The query and reference window bytes of the SSW and piecewise jobs into the arena, a warp
+// per job: four bases per lane and step, the window's from one or two packed words.  (With
+// 32 jobs per warp one after another, a wave of 30 jobs took 110 us here.)
+__global__ void __launch_bounds__(256) k_copy(const ExtJob* jobs, const uint8_t* __restrict__ seq,
+                                              const uint64_t* __restrict__ off, DevRefs R, const uint8_t* raw_refs,
+                                              const uint64_t* raw_off, const PrepRec* prep, uint8_t* arena,
+                                              const SswTask* tasks, const uint32_t* pw_list,
+                                              const uint32_t* counters) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
+    const uint32_t n_ssw = counters[0], n_pw = counters[19];
+    for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) / 32; x < n_ssw + n_pw; x += nwarps) {
+        const uint32_t t = x < n_ssw ? tasks[x].job : pw_list[x - n_ssw];
+        const PrepRec p = prep[t];
+        const uint8_t* s = seq + off[p.read];
+        uint8_t* q = arena + p.arena_off;
+        const uint32_t L = p.qlen;
+        for (uint32_t i = lane; i < L; i += 32) q[i] = read_char(s, L, i, p.rc);
+        uint8_t* w = q + L;
+        if (p.type == 2 && jobs[t].kind == JOB_ALIGN) {
+            const uint8_t* rr = raw_refs + raw_off[p.ref_id];
+            for (uint32_t i = lane; i < p.wlen; i += 32) w[i] = rr[i];
+        } else {
+            for (uint32_t i = 4 * lane; i < p.wlen; i += 128) {
+                const uint32_t c = (uint32_t)ref_codes32(R, p.ref_id, (uint64_t)p.wstart + i);
+                const uint32_t m = p.wlen - i < 4 ? p.wlen - i : 4;
+                for (uint32_t y = 0; y < m; y++) w[i + y] = code_char((c >> (2 * y)) & 3);
             }
         }
     }
@@ -1599,7 +1595,15 @@ __device__ int band_pass_warp(const uint8_t* ref, const uint8_t* read, int rl, i
     const int width = 2 * bw + 3;
     constexpr int NEG = -(1 << 28);
     int prevH = 0, prevE = 0, mx = 0;
+    // the next row's query and column bytes are loaded a row ahead
+    uint8_t qn = ql > 0 ? read[0] : 0, rn = lane < rl ? ref[lane] : 0;
     for (int i = 0; i < ql; i++) {
+        const int qcode = c_ssw_code[qn], rcode = c_ssw_code[rn];
+        {
+            const int c = (i + 1 - bw > 0 ? i + 1 - bw : 0) + lane;
+            qn = i + 1 < ql ? read[i + 1] : 0;
+            rn = c < rl ? ref[c] : 0;
+        }
         const int x = i - bw > 0 ? i - bw : 0, xe = i - 1 - bw > 0 ? i - 1 - bw : 0;
         const int end = rl - 1 < i + bw ? rl - 1 : i + bw;
         const int n = end - x + 1;
@@ -1621,7 +1625,7 @@ __device__ int band_pass_warp(const uint8_t* ref, const uint8_t* read, int rl, i
         const int E = t1 > t2 ? t1 : t2;
         const bool dde3 = t1 > t2;
         int D = 0;
-        if (act) D = dg + mat_score(c_ssw_code[ref[x + lane]], c_ssw_code[read[i]], sc);
+        if (act) D = dg + mat_score(rcode, qcode, sc);
         const int e1 = E > 0 ? E : 0;
         const int B = e1 > D ? e1 : D;
         int T = act ? B - gO : NEG;
@@ -1689,27 +1693,26 @@ __device__ __forceinline__ void count_band_cells(uint32_t* counters, uint64_t co
     }
 }
 
-// banded_sw's traceback (ext/ssw/ssw.c:680-753) by one thread over the direction bits
-// of the last pass: words(row, w0, w1, w2, w3) gives row `row`'s bits for band index k
-// (E opened, F opened, H from the diagonal, E over F).  The library walks a flat
-// (2bw+1) x 3-byte-per-row array, so an index that leaves a row reads the neighbouring
-// row's entries, or 0 where the pass wrote nothing; the walk does the same.  Writes the
-// CIGAR (reversed into order) to c; false when the walk fails or c is too small.
+// banded_sw's traceback (ext/ssw/ssw.c:680-753) by one warp over the direction bits of the
+// last pass: words(row, w0, w1, w2, w3) gives row `row`'s bits for band index k (E opened,
+// F opened, H from the diagonal, E over F).  The library walks a flat (2bw+1) x
+// 3-byte-per-row array, so an index that leaves a row reads the neighbouring row's
+// entries, or 0 where the pass wrote nothing; the walk does the same.  All lanes walk
+// together; where the band slides, the diagonal keeps its band index, and a run of
+// matches is taken 32 rows at a time (a step at a time the walk of 150 rows took 50 to
+// 150 thousand cycles).  Writes the CIGAR (reversed into order) to c; false when the walk
+// fails or c is too small.
 template <class Words>
-__device__ bool band_trace_thread(Words words, int rl, int ql, int bw, uint32_t* c, uint32_t cap, uint32_t& nc) {
+__device__ bool band_trace_warp(Words words, int rl, int ql, int bw, uint32_t* c, uint32_t cap, uint32_t& nc) {
+    const int lane = threadIdx.x & 31;
     const int width_d = 2 * bw + 1;
     const int64_t dsize = (int64_t)width_d * ql * 3;
-    // the row's four direction words, loaded when the walk enters a row
-    int cached = -1;
-    uint32_t w0 = 0, w1 = 0, w2 = 0, w3 = 0;
     auto dir_of = [&](int row, int k, int w) -> int {
         const int x = row - bw > 0 ? row - bw : 0;
         const int end = rl - 1 < row + bw ? rl - 1 : row + bw;
         if (k > end - x) return 0;  // not written by the pass
-        if (row != cached) {
-            words(row, w0, w1, w2, w3);
-            cached = row;
-        }
+        uint32_t w0, w1, w2, w3;
+        words(row, w0, w1, w2, w3);
         const int dde = (w0 >> k) & 1 ? 3 : 2;
         const int ddf = (w1 >> k) & 1 ? 5 : 4;
         if (w == 0) return dde;
@@ -1720,46 +1723,76 @@ __device__ bool band_trace_thread(Words words, int rl, int ql, int bw, uint32_t*
     char op = 'M', prev = 'M';
     nc = 0;
     auto enc = [](int l, char o) -> uint32_t { return ((uint32_t)l << 4) | (o == 'M' ? 0u : o == 'I' ? 1u : 2u); };
+    auto put = [&](uint32_t v) {
+        if (lane == 0) c[nc] = v;
+        nc++;
+    };
     while (i >= 0 && j > 0) {
         const int x = i - bw > 0 ? i - bw : 0;
         const int k = j - x;
-        int d;
-        if (k >= 0 && k < width_d) {
-            d = dir_of(i, k, which);  // the flat index falls in row i
+        int steps = 0;
+        if (which == 2 && x > 0 && k >= 0 && k < width_d) {
+            // rows i, i - 1, ... while they slide (x > 0) and the walk goes on (j > 0)
+            const int row = i - lane;
+            bool m = false;
+            if (row > bw && j - lane > 0) {
+                uint32_t w0, w1, w2, w3;
+                words(row, w0, w1, w2, w3);
+                m = (w2 >> k) & 1;
+            }
+            const uint32_t bal = __ballot_sync(FULLM, m);
+            steps = bal == FULLM ? 32 : __ffs(~bal) - 1;
+            if (steps) {
+                i -= steps;
+                j -= steps;
+                op = 'M';
+            }
+        }
+        if (steps == 0) {
+            int d;
+            if (k >= 0 && k < width_d) {
+                d = dir_of(i, k, which);  // the flat index falls in row i
+            } else {
+                // the flat index (row i, band column k) runs into a neighbouring row
+                const int64_t at = (int64_t)width_d * i * 3 + (int64_t)k * 3 + which;
+                if (at < 0 || at >= dsize) return false;
+                const int rem = (int)(at % (3 * width_d));
+                d = dir_of((int)(at / (3 * width_d)), rem / 3, rem % 3);
+            }
+            switch (d) {
+                case 1: --i; --j; which = 2; op = 'M'; break;
+                case 2: --i; which = 0; op = 'I'; break;
+                case 3: --i; which = 2; op = 'I'; break;
+                case 4: --j; which = 1; op = 'D'; break;
+                case 5: --j; which = 2; op = 'D'; break;
+                default: return false;
+            }
+            steps = 1;
+        }
+        if (op == prev) {
+            e += steps;
         } else {
-            // the flat index (row i, band column k) runs into a neighbouring row
-            const int64_t at = (int64_t)width_d * i * 3 + (int64_t)k * 3 + which;
-            if (at < 0 || at >= dsize) return false;
-            const int rem = (int)(at % (3 * width_d));
-            d = dir_of((int)(at / (3 * width_d)), rem / 3, rem % 3);
-        }
-        switch (d) {
-            case 1: --i; --j; which = 2; op = 'M'; break;
-            case 2: --i; which = 0; op = 'I'; break;
-            case 3: --i; which = 2; op = 'I'; break;
-            case 4: --j; which = 1; op = 'D'; break;
-            case 5: --j; which = 2; op = 'D'; break;
-            default: return false;
-        }
-        if (op == prev) ++e;
-        else {
             if (nc >= cap) return false;
-            c[nc++] = enc(e, prev);
+            put(enc(e, prev));
             prev = op;
-            e = 1;
+            e = steps;
         }
     }
     if (nc + 2 > cap) return false;
-    if (op == 'M') c[nc++] = enc(e + 1, op);
-    else {
-        c[nc++] = enc(e, op);
-        c[nc++] = enc(1, 'M');
+    if (op == 'M') {
+        put(enc(e + 1, op));
+    } else {
+        put(enc(e, op));
+        put(enc(1, 'M'));
     }
-    for (uint32_t a = 0, b = nc - 1; a < b; a++, b--) {
-        const uint32_t tmp = c[a];
-        c[a] = c[b];
-        c[b] = tmp;
-    }
+    __syncwarp();
+    if (lane == 0)
+        for (uint32_t a = 0, b = nc - 1; a < b; a++, b--) {
+            const uint32_t tmp = c[a];
+            c[a] = c[b];
+            c[b] = tmp;
+        }
+    __syncwarp();
     return true;
 }
 
@@ -1777,7 +1810,7 @@ __device__ int band_pass_thread(const uint8_t* ref, const uint8_t* read, int rl,
                                 uint32_t* rows, uint64_t& cells) {
     constexpr int K = 2 * BW + 1;  // band cells per row
     constexpr int W = K + 2;       // the library's width
-    const int gO = sc.gap_open, gE = sc.gap_extend;
+    const int gO = sc.gap_open, gE = sc.gap_extend, match = sc.match, mismatch = -(int)sc.mismatch;
     int hb[W], eb[W], hc[W], rc[K];
 #pragma unroll
     for (int t = 0; t < W; t++) {
@@ -1790,7 +1823,9 @@ __device__ int band_pass_thread(const uint8_t* ref, const uint8_t* read, int rl,
 #pragma unroll
     for (int k = 0; k < K; k++) rc[k] = k <= end0 ? c_ssw_code[ref[k]] : 4;
     int mx = 0, prev_end = end0;
-    for (int i = 0; i < ql; i++) {
+    // any row: the first ones, until the band slides, and the last ones, past the
+    // reference's end
+    auto any_row = [&](int i) {
         const int x = i - BW > 0 ? i - BW : 0;
         const int sh = i - BW > 0 ? 1 : 0;  // x - max(0, i - 1 - BW)
         const int end = rl - 1 < i + BW ? rl - 1 : i + BW;
@@ -1853,7 +1888,54 @@ __device__ int band_pass_thread(const uint8_t* ref, const uint8_t* read, int rl,
             rows[2 * i] = d0;
             rows[2 * i + 1] = d1;
         }
+    };
+    // rows [i1, i2) hold the whole band, one column further than the row before: no
+    // cell needs a test, and H and E are updated in place
+    const int i1 = BW + 1, i2 = rl - BW < ql ? rl - BW : ql;
+    int i = 0;
+    for (; i < ql && i < i1; i++) any_row(i);
+    if (i < i2) {
+        hb[W - 1] = eb[W - 1] = 0;
+        int qn = c_ssw_code[read[i]], rn = c_ssw_code[ref[i + BW]];
+        for (; i < i2; i++) {
+#pragma unroll
+            for (int k = 0; k + 1 < K; k++) rc[k] = rc[k + 1];
+            rc[K - 1] = rn;
+            const int qc = qn < 4 ? qn : -1;  // N matches nothing
+            if (i + 1 < i2) {
+                qn = c_ssw_code[read[i + 1]];
+                rn = c_ssw_code[ref[i + 1 + BW]];
+            }
+            uint32_t d0 = 0, d1 = 0;
+            int h = 0, f = 0;
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                int t1 = hb[k + 2] - gO, t2 = eb[k + 2] - gE;
+                const int E = t1 > t2 ? t1 : t2;
+                eb[k + 1] = E;
+                if (t1 > t2) d0 |= 1u << k;
+                t1 = h - gO;
+                t2 = f - gE;
+                f = t1 > t2 ? t1 : t2;
+                if (t1 > t2) d0 |= 1u << (16 + k);
+                const int f1 = f > 0 ? f : 0;
+                const int D = hb[k + 1] + (rc[k] == qc ? match : mismatch);
+                t1 = E > f1 ? E : f1;
+                h = t1 > D ? t1 : D;
+                hb[k + 1] = h;
+                mx = h > mx ? h : mx;
+                if (t1 <= D) d1 |= 1u << k;
+                if (E > f1) d1 |= 1u << (16 + k);
+            }
+            cells += (uint64_t)K;
+            if (rows) {
+                rows[2 * i] = d0;
+                rows[2 * i + 1] = d1;
+            }
+        }
+        prev_end = i2 - 1 + BW;
     }
+    for (; i < ql; i++) any_row(i);
     return mx;
 }
 
@@ -1861,77 +1943,124 @@ constexpr int BAND_THREAD_MAX_BW = 5;  // bands up to 11 cells a thread per task
 
 // Tasks by starting band width |rl - ql| + 1: bucket b (1 .. BAND_THREAD_MAX_BW) holds
 // its tasks at buckets[b * n_tasks ..] and their count at bucket_n[b]; wider ones go
-// straight to k_band_warp's list.  k_band_small then runs the buckets in turn, so the
-// threads of a warp share their band width (one template instance per warp).
-__global__ void k_band_bucket(const SswTask* tasks, uint32_t n_tasks, uint32_t* buckets, uint32_t* bucket_n,
+// straight to k_band_warp's list, the width in band_width.  k_band_small then runs the
+// buckets in turn, so the threads of a warp share their band width (one template instance
+// per warp).
+__global__ void k_band_bucket(SswTask* tasks, uint32_t n_tasks, uint32_t* buckets, uint32_t* bucket_n,
                               uint32_t* warp_list, uint32_t* counters) {
     for (uint32_t ti = blockIdx.x * blockDim.x + threadIdx.x; ti < n_tasks; ti += gridDim.x * blockDim.x) {
         const SswTask tk = tasks[ti];
         if (tk.ref_begin1 < 0 || tk.read_begin1 < 0) continue;
+        // its CIGAR known from the scores (ungapped), or dropped (k_finalize)
+        if (tk.raw_off != RAW_FALLBACK || tk.flag != 0) continue;
         const int rl = tk.ref_end1 - tk.ref_begin1 + 1, ql = tk.read_end1 - tk.read_begin1 + 1;
         const int bw = (rl > ql ? rl - ql : ql - rl) + 1;
-        if (bw > BAND_THREAD_MAX_BW) warp_list[atomicAdd(&counters[28], 1u)] = ti;
-        else buckets[(size_t)bw * n_tasks + atomicAdd(&bucket_n[bw], 1u)] = ti;
+        if (bw > BAND_THREAD_MAX_BW) {
+            tasks[ti].band_width = bw;
+            warp_list[atomicAdd(&counters[28], 1u)] = ti;
+        } else buckets[(size_t)bw * n_tasks + atomicAdd(&bucket_n[bw], 1u)] = ti;
     }
 }
 
-// banded_sw (ext/ssw/ssw.c:598-769) a thread per task while the band width stays at
-// most BAND_THREAD_MAX_BW (the band of an alignment without indels is 3 cells wide, so
-// a warp per task left most lanes idle).  A task whose doubling goes past that is left
-// for k_band_warp (raw_off stays RAW_FALLBACK), which starts its doubling over.
-__global__ void __launch_bounds__(128) k_band_small(SswTask* tasks, uint32_t n_tasks, const PrepRec* prep,
-                                                    const uint8_t* arena, int32_t* hscratch, AlignScores sc,
-                                                    uint32_t* counters, uint32_t* warp_list, const uint32_t* buckets,
-                                                    const uint32_t* bucket_n) {
-    uint64_t computed = 0, canonical = 0;
-    const uint32_t stride = gridDim.x * blockDim.x;
-    uint32_t bucket = 1, i = blockIdx.x * blockDim.x + threadIdx.x;
+// banded_sw's passes (ext/ssw/ssw.c:598-769) a thread per task for band widths up to
+// BAND_THREAD_MAX_BW (the band of an alignment without indels is 3 cells wide, so a warp
+// per task leaves most lanes idle).  A launch lasts as long as one thread's rows, so the
+// widths that the doubling may go through run side by side, a warp of the block each
+// (32 tasks of one starting width b: b, 2b, 4b), instead of one after another with the
+// warp's other tasks waiting; k_band_trace then takes the one that the doubling ends on.
+// Each width leaves its rows' direction words and its maximum in the task's scratch.
+// A wave of 90 to 190 tasks: 46 us and 10 us for the tracebacks, 424 us with the widths in
+// turn and the traceback on the task's thread (and ungapped tasks among them, which
+// k_ssw16 now settles).
+constexpr int BAND_WIDTHS = 3;
+
+// scratch of width index w: its rows' words; after the three, the maxima and the CIGAR
+__device__ __forceinline__ size_t band_rows_at(int ql, int w) { return 2 * (size_t)ql * w; }
+__device__ __forceinline__ size_t band_max_at(int ql) { return 2 * (size_t)ql * BAND_WIDTHS; }
+
+__global__ void __launch_bounds__(32 * BAND_WIDTHS) k_band_small(const SswTask* tasks, uint32_t n_tasks,
+                                                                 const PrepRec* prep, const uint8_t* arena,
+                                                                 int32_t* hscratch, AlignScores sc, uint32_t* counters,
+                                                                 const uint32_t* buckets, const uint32_t* bucket_n) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x / 32;
+    uint64_t computed = 0;
+    // units of 32 tasks of one starting width
+    uint32_t bucket = 1, unit = blockIdx.x;
     for (;;) {
-        // the next task: bucket by bucket, the threads striding through each
-        while (bucket <= (uint32_t)BAND_THREAD_MAX_BW && i >= bucket_n[bucket]) {
-            i -= bucket_n[bucket];
+        while (bucket <= (uint32_t)BAND_THREAD_MAX_BW && unit >= (bucket_n[bucket] + 31) / 32) {
+            unit -= (bucket_n[bucket] + 31) / 32;
             bucket++;
         }
         if (bucket > (uint32_t)BAND_THREAD_MAX_BW) break;
-        const uint32_t ti = buckets[(size_t)bucket * n_tasks + i];
-        i += stride;
-        SswTask tk = tasks[ti];
+        const uint32_t x = 32 * unit + lane;
+        const int bw = (int)bucket << w;
+        unit += gridDim.x;
+        if (bw > BAND_THREAD_MAX_BW || x >= bucket_n[bucket]) continue;
+        const SswTask tk = tasks[buckets[(size_t)bucket * n_tasks + x]];
         const PrepRec p = prep[tk.job];
         const uint8_t* q = arena + p.arena_off + tk.read_begin1;
         const uint8_t* r = arena + p.arena_off + p.qlen + tk.ref_begin1;
         const int rl = tk.ref_end1 - tk.ref_begin1 + 1, ql = tk.read_end1 - tk.read_begin1 + 1;
-        const int len = rl > ql ? rl : ql;
-        int bw = (rl > ql ? rl - ql : ql - rl) + 1;
-        // rows in the task's scratch as k_band_warp keeps them, the CIGAR after them
-        uint32_t* rows = reinterpret_cast<uint32_t*>(hscratch + p.h_off);
-        int mx = 0;
-        bool small = true;
+        if (w > 0 && bw > (rl > ql ? rl : ql)) continue;  // the doubling ends before
+        int32_t* h = hscratch + p.h_off;
+        uint32_t* rows = reinterpret_cast<uint32_t*>(h + band_rows_at(ql, w));
         uint64_t cells = 0;
-        do {
-            if (bw > BAND_THREAD_MAX_BW) {
-                small = false;
-                break;
-            }
-            cells = 0;
-            switch (bw) {
-                case 1: mx = band_pass_thread<1>(r, q, rl, ql, sc, rows, cells); break;
-                case 2: mx = band_pass_thread<2>(r, q, rl, ql, sc, rows, cells); break;
-                case 3: mx = band_pass_thread<3>(r, q, rl, ql, sc, rows, cells); break;
-                case 4: mx = band_pass_thread<4>(r, q, rl, ql, sc, rows, cells); break;
-                default: mx = band_pass_thread<5>(r, q, rl, ql, sc, rows, cells); break;
-            }
-            computed += cells;
+        int mx;
+        switch (bw) {
+            case 1: mx = band_pass_thread<1>(r, q, rl, ql, sc, rows, cells); break;
+            case 2: mx = band_pass_thread<2>(r, q, rl, ql, sc, rows, cells); break;
+            case 3: mx = band_pass_thread<3>(r, q, rl, ql, sc, rows, cells); break;
+            case 4: mx = band_pass_thread<4>(r, q, rl, ql, sc, rows, cells); break;
+            default: mx = band_pass_thread<5>(r, q, rl, ql, sc, rows, cells); break;
+        }
+        h[band_max_at(ql) + w] = mx;
+        computed += cells;
+    }
+    // the cells of this thread's tasks, one atomic per warp
+    unsigned long long cs = computed;
+    for (int d = 16; d > 0; d >>= 1) cs += __shfl_xor_sync(FULLM, cs, d);
+    count_band_cells(counters, cs, 0);
+}
+
+// The width each of k_band_small's tasks ends on and its traceback, a warp per task.  A task
+// whose doubling goes past BAND_THREAD_MAX_BW is left for k_band_warp, with the next
+// width to try (raw_off stays RAW_FALLBACK).
+__global__ void __launch_bounds__(128) k_band_trace(SswTask* tasks, uint32_t n_tasks, const PrepRec* prep,
+                                                    int32_t* hscratch, uint32_t* counters, uint32_t* warp_list,
+                                                    const uint32_t* buckets, const uint32_t* bucket_n) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
+    uint32_t bucket = 1, x = (blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    for (;;) {
+        while (bucket <= (uint32_t)BAND_THREAD_MAX_BW && x >= bucket_n[bucket]) {
+            x -= bucket_n[bucket];
+            bucket++;
+        }
+        if (bucket > (uint32_t)BAND_THREAD_MAX_BW) break;
+        const uint32_t ti = buckets[(size_t)bucket * n_tasks + x];
+        x += nwarps;
+        SswTask tk = tasks[ti];
+        const PrepRec p = prep[tk.job];
+        const int rl = tk.ref_end1 - tk.ref_begin1 + 1, ql = tk.read_end1 - tk.read_begin1 + 1;
+        const int len = rl > ql ? rl : ql;
+        const int32_t* h = hscratch + p.h_off;
+        // band doubling (ext/ssw/ssw.c:626-660)
+        int bw = (int)bucket, w = 0;
+        while (bw <= BAND_THREAD_MAX_BW && h[band_max_at(ql) + w] < tk.score1 && 2 * bw <= len) {
             bw *= 2;
-        } while (mx < tk.score1 && bw <= len);
-        if (!small) {  // raw_off stays RAW_FALLBACK: k_band_warp takes it
-            warp_list[atomicAdd(&counters[28], 1u)] = ti;
+            w++;
+        }
+        if (bw > BAND_THREAD_MAX_BW) {
+            if (lane == 0) {
+                tasks[ti].band_width = bw;
+                warp_list[atomicAdd(&counters[28], 1u)] = ti;
+            }
             continue;
         }
-        bw /= 2;
-        canonical += cells;
-        uint32_t* c = rows + 4 * (size_t)ql;
+        const uint32_t* rows = reinterpret_cast<const uint32_t*>(h + band_rows_at(ql, w));
+        const size_t at = band_max_at(ql) + BAND_WIDTHS;
         uint32_t nc = 0;
-        const bool ok = band_trace_thread(
+        const bool ok = band_trace_warp(
             [&](int row, uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
                 const uint32_t a = rows[2 * row], b = rows[2 * row + 1];
                 w0 = a & 0xffffu;
@@ -1939,26 +2068,21 @@ __global__ void __launch_bounds__(128) k_band_small(SswTask* tasks, uint32_t n_t
                 w2 = b & 0xffffu;
                 w3 = b >> 16;
             },
-            rl, ql, bw, c, (uint32_t)(rl + ql + 4), nc);
-        tk.band_width = bw;
-        if (!ok) {
-            tk.flag = 1;
-            tk.raw_len = 0;
-        } else {
-            tk.raw_len = nc;
+            rl, ql, bw, reinterpret_cast<uint32_t*>(hscratch + p.h_off + at), (uint32_t)(rl + ql + 4), nc);
+        count_band_cells(counters, 0, band_cells(rl, ql, bw));
+        if (lane == 0) {
+            tk.band_width = bw;
+            if (!ok) tk.flag = 1;
+            tk.raw_len = ok ? nc : 0;
+            tk.raw_off = (uint64_t)p.h_off + at;
+            tasks[ti] = tk;
         }
-        tk.raw_off = (uint64_t)p.h_off + 4 * (uint64_t)ql;
-        tasks[ti] = tk;
     }
-    // the cells of this thread's tasks, one atomic per warp
-    unsigned long long cs = computed, cn = canonical;
-    for (int d = 16; d > 0; d >>= 1) {
-        cs += __shfl_xor_sync(FULLM, cs, d);
-        cn += __shfl_xor_sync(FULLM, cn, d);
-    }
-    count_band_cells(counters, cs, cn);
 }
 
+// banded_sw a warp per task for the bands of 13 to 31 cells: the tasks that start there and
+// those k_band_trace left.  Widths that were tried are not tried again (up to 185 us a
+// launch with them and the traceback a step at a time, 50 us now).
 __global__ void __launch_bounds__(128) k_band_warp(SswTask* tasks, const uint32_t* list, const PrepRec* prep,
                                                    const uint8_t* arena, int32_t* hscratch, AlignScores sc,
                                                    uint32_t* counters, uint32_t* wide_list) {
@@ -1978,7 +2102,7 @@ __global__ void __launch_bounds__(128) k_band_warp(SswTask* tasks, const uint32_
         const uint8_t* r = q + p.qlen;
         const int rl = tk.ref_end1 - tk.ref_begin1 + 1, ql = tk.read_end1 - tk.read_begin1 + 1;
         const int len = rl > ql ? rl : ql;
-        int bw = (rl > ql ? rl - ql : ql - rl) + 1;
+        int bw = tk.band_width;  // the widths below were tried by k_band_small
         // band doubling (ext/ssw/ssw.c:626-660).  Every pass records its direction bits:
         // the doubling ends on the width it ran last, so the last pass's bits are the
         // ones the traceback reads and no pass is repeated to record them.
@@ -1997,32 +2121,31 @@ __global__ void __launch_bounds__(128) k_band_warp(SswTask* tasks, const uint32_
         } while (mx < tk.score1 && bw <= len);
         if (fallback) {
             count_band_cells(counters, computed, 0);
-            if (lane == 0) wide_list[atomicAdd(&counters[29], 1u)] = ti;
+            if (lane == 0) {
+                tasks[ti].band_width = bw;
+                wide_list[atomicAdd(&counters[29], 1u)] = ti;
+            }
             continue;  // raw_off stays RAW_FALLBACK
         }
         bw /= 2;
         count_band_cells(counters, computed, band_cells(rl, ql, bw));
         __syncwarp();
+        // traceback over the four ballot words per row the passes recorded
+        uint32_t* c = rowbits + 4 * (size_t)ql;
+        uint32_t nc = 0;
+        const bool ok = band_trace_warp(
+            [&](int row, uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
+                const uint32_t* rb = rowbits + 4 * (size_t)row;
+                w0 = rb[0];
+                w1 = rb[1];
+                w2 = rb[2];
+                w3 = rb[3];
+            },
+            rl, ql, bw, c, (uint32_t)(rl + ql + 4), nc);
         if (lane == 0) {
-            // traceback over the four ballot words per row the passes recorded
-            uint32_t* c = rowbits + 4 * (size_t)ql;
-            uint32_t nc = 0;
-            const bool ok = band_trace_thread(
-                [&](int row, uint32_t& w0, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
-                    const uint32_t* rb = rowbits + 4 * (size_t)row;
-                    w0 = rb[0];
-                    w1 = rb[1];
-                    w2 = rb[2];
-                    w3 = rb[3];
-                },
-                rl, ql, bw, c, (uint32_t)(rl + ql + 4), nc);
             tk.band_width = bw;
-            if (!ok) {
-                tk.flag = 1;
-                tk.raw_len = 0;
-            } else {
-                tk.raw_len = nc;
-            }
+            if (!ok) tk.flag = 1;
+            tk.raw_len = ok ? nc : 0;
             tk.raw_off = (uint64_t)p.h_off + 4 * (uint64_t)ql;
             tasks[ti] = tk;
         }
@@ -2222,7 +2345,7 @@ __global__ void __launch_bounds__(32) k_band_width_wide(SswTask* tasks, const ui
         const uint8_t* r = q + p.qlen;
         const int rl = tk.ref_end1 - tk.ref_begin1 + 1, ql = tk.read_end1 - tk.read_begin1 + 1;
         const int len = rl > ql ? rl : ql;
-        int bw = (rl > ql ? rl - ql : ql - rl) + 1;
+        int bw = tk.band_width;  // the widths below were tried
         int mx = 0;
         bool fail = false;
         uint64_t computed = 0;
@@ -2324,7 +2447,7 @@ __global__ void k_band_width(SswTask* tasks, const uint32_t* n_tasks_ptr, const 
     }
 }
 
-__global__ void k_band_trace(SswTask* tasks, const uint32_t* n_tasks_ptr, const PrepRec* prep, const uint8_t* arena,
+__global__ void k_band_trace_literal(SswTask* tasks, const uint32_t* n_tasks_ptr, const PrepRec* prep, const uint8_t* arena,
                              int32_t* hscratch, AlignScores sc, const uint64_t* dir_off, uint8_t* dir,
                              const uint64_t* raw_off, uint32_t* raw) {
     const uint32_t n = *n_tasks_ptr;
@@ -3167,12 +3290,12 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
     ws.list_rev_word.reserve(n);
     kt->begin(KS_FILL, st);
     ws.pw_list.reserve(n);
-    k_fill<<<grid1(n), 256, 0, st>>>(
-        ws.jobs.p, n, seq, off, refs, raw_refs, raw_off, sc, ws.prep.p, of[0], of[1],
-                                     of[2], ws.arena.p, ws.cigar.p, ws.results.p, ws.tasks.p, ws.counters.p,
-                                     ws.pw_list.p);
+    k_fill<<<grid1(n), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, sc, ws.prep.p, of[0], of[1], of[2], ws.cigar.p,
+                                     ws.results.p, ws.tasks.p, ws.counters.p, ws.pw_list.p);
+    k_copy<<<grid1((uint64_t)n * 32), 256, 0, st>>>(ws.jobs.p, seq, off, refs, raw_refs, raw_off, ws.prep.p,
+                                                    ws.arena.p, ws.tasks.p, ws.pw_list.p, ws.counters.p);
     kt->end(st);
-    launches++;
+    launches += 2;
     if (max_pw_window) {
         // single-end piecewise jobs: a warp per job, each warp with its own DP scratch
         if (!anchors) throw Error(SA_ERR_INVALID, "internal: piecewise jobs without anchors");
@@ -3307,7 +3430,7 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
             }
             if (q16) {
                 const Ssw16Args a{ws.tasks.p, ws.order.p, n_tasks, ws.prep.p, ws.arena.p, sc, bias, ws.counters.p, q16,
-                                  ws.list_word.p, ws.counters.p + 31, st};
+                                  ws.list_word.p, ws.counters.p + 31, ws.hscratch.p, st};
                 launch_ssw16(a, std::min(max_qlen, q16));
                 // the tasks whose reverse pass went beyond the forward score
                 if (rmax == 4) SA_SSW(4, ws.list_word.p, ws.counters.p + 31, 23, sm_count(), 0);
@@ -3340,8 +3463,6 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
             kt->begin(KS_BAND, st);
             uint64_t blocks = ((uint64_t)n_tasks + 3) / 4;
             if (blocks > sm_count() * 16) blocks = sm_count() * 16;
-            uint64_t tblocks = ((uint64_t)n_tasks + 127) / 128;
-            if (tblocks > sm_count() * 16) tblocks = sm_count() * 16;
             ws.band_list.reserve(n_tasks);
             ws.wide_list.reserve(n_tasks);
             ws.band_buckets.reserve((size_t)(BAND_THREAD_MAX_BW + 1) * n_tasks + 8);
@@ -3349,9 +3470,12 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
             SA_CUDA(cudaMemsetAsync(bucket_n, 0, 8 * sizeof(uint32_t), st));
             k_band_bucket<<<grid1(n_tasks), 256, 0, st>>>(ws.tasks.p, n_tasks, ws.band_buckets.p, bucket_n,
                                                           ws.band_list.p, ws.counters.p);
-            k_band_small<<<(unsigned)tblocks, 128, 0, st>>>(ws.tasks.p, n_tasks, ws.prep.p, ws.arena.p,
-                                                             ws.hscratch.p, sc, ws.counters.p, ws.band_list.p,
-                                                             ws.band_buckets.p, bucket_n);
+            const uint64_t units = ((uint64_t)n_tasks + 31) / 32 + BAND_THREAD_MAX_BW;
+            k_band_small<<<(unsigned)std::min<uint64_t>(units, sm_count() * 16), 32 * BAND_WIDTHS, 0, st>>>(
+                ws.tasks.p, n_tasks, ws.prep.p, ws.arena.p, ws.hscratch.p, sc, ws.counters.p, ws.band_buckets.p,
+                bucket_n);
+            k_band_trace<<<(unsigned)blocks, 128, 0, st>>>(ws.tasks.p, n_tasks, ws.prep.p, ws.hscratch.p, ws.counters.p,
+                                                           ws.band_list.p, ws.band_buckets.p, bucket_n);
             k_band_warp<<<(unsigned)blocks, 128, 0, st>>>(ws.tasks.p, ws.band_list.p, ws.prep.p, ws.arena.p,
                                                           ws.hscratch.p, sc, ws.counters.p, ws.wide_list.p);
             kt->end(st);
@@ -3405,7 +3529,7 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
                                                                  ws.prep.p, ws.arena.p, sc, maxc, ws.dir_off.p,
                                                                  ws.dir.p, ws.raw_off.p, ws.raw.p, ws.counters.p);
         else
-            k_band_trace<<<grid1(n_tasks, 128), 128, 0, st>>>(ws.tasks.p, ws.counters.p, ws.prep.p, ws.arena.p,
+            k_band_trace_literal<<<grid1(n_tasks, 128), 128, 0, st>>>(ws.tasks.p, ws.counters.p, ws.prep.p, ws.arena.p,
                                                               ws.hscratch.p, sc, ws.dir_off.p, ws.dir.p, ws.raw_off.p,
                                                               ws.raw.p);
         kt->end(st);

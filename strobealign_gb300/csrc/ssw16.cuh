@@ -365,7 +365,8 @@ __device__ __forceinline__ int diag_bound(bool run, const uint8_t* q, int qlen, 
 template <int NB, bool PAIR, class GP>
 __global__ void __launch_bounds__(32 * SSW16_WARPS, NB > 20 ? 4 : 6)
     k_ssw16(SswTask* tasks, const uint32_t* order, uint32_t n_tasks, const PrepRec* prep, const uint8_t* arena,
-            AlignScores sc, GP gp, int bias, uint32_t* counters, uint32_t qmax, uint32_t* redo, uint32_t* n_redo) {
+            AlignScores sc, GP gp, int bias, uint32_t* counters, uint32_t qmax, uint32_t* redo, uint32_t* n_redo,
+            int32_t* hscratch) {
     constexpr int T = T16, NW = (NB + 7) / 8, G = 32 / T;
     extern __shared__ __align__(16) uint4 s16_smem[];
     __shared__ uint32_t s_base;
@@ -454,7 +455,25 @@ __global__ void __launch_bounds__(32 * SSW16_WARPS, NB > 20 ? 4 : 6)
             b.beyond = false;
         }
         // the warp of the task's mode has its reverse pass
-        if (have && gl == 0 && (!PAIR || wib == (int)word)) {
+        const bool mine = have && (!PAIR || wib == (int)word);
+        // Both ends known, equally long spans whose diagonal alone scores score1: banded_sw
+        // would find that diagonal (its first band holds it; a cell of it above the
+        // diagonal's own prefix sum would make a path better than score1, and its
+        // traceback takes the diagonal on ties).  The passes miss only paths with an
+        // insertion next to a deletion, which within that band cost no less than the
+        // mismatches they replace if mismatch <= gap_open + gap_extend.
+        const int ql = b.read + 1, qs = e.read - b.read, rs = b.ref;
+        const bool even = mine && rev && e.score <= b.score && !b.beyond && e.ref - rs + 1 == ql &&
+                          (int)sc.mismatch <= (int)sc.gap_open + (int)sc.gap_extend;
+        int same = 0;
+        for (int i = gl; even && i < ql; i += T) {
+            const int c = code[q[qs + i]];
+            same += c < 4 && c == code[r[rs + i]];
+        }
+#pragma unroll
+        for (int o = 1; o < T; o <<= 1) same += __shfl_xor_sync(FULLM, same, o, T);
+        const bool ungapped = even && same * (int)sc.match - (ql - same) * (int)sc.mismatch == e.score;
+        if (mine && gl == 0) {
             SswTask& tk = tasks[ti];
             tk.score1 = e.score;
             tk.ref_end1 = e.ref;
@@ -463,6 +482,14 @@ __global__ void __launch_bounds__(32 * SSW16_WARPS, NB > 20 ? 4 : 6)
             tk.ref_begin1 = b.ref;
             tk.read_begin1 = e.read - b.read;
             tk.flag = e.score > b.score ? 2 : 0;
+            if (ungapped) {
+                // as k_band_small leaves a task: its CIGAR after the rows' words
+                const uint64_t at = prep[tk.job].h_off + 4 * (uint64_t)ql;
+                hscratch[at] = ql << 4;
+                tk.band_width = 1;
+                tk.raw_len = 1;
+                tk.raw_off = at;
+            }
             if (b.beyond) redo[atomicAdd(n_redo, 1u)] = ti;
             const unsigned long long c_r = (unsigned long long)(e.read + 1) * b.cols;
             if (c_fb) atomicAdd(cells + 1, c_fb);
@@ -488,7 +515,8 @@ void launch_one(const Ssw16Args& a, GP gp) {
     const uint64_t per_block = (uint64_t)(PAIR ? 1 : SSW16_WARPS) * G;
     const uint64_t blocks = std::min<uint64_t>((a.n_tasks + per_block - 1) / per_block, sm_count() * 32);
     k_ssw16<NB, PAIR, GP><<<(unsigned)std::max<uint64_t>(1, blocks), 32 * SSW16_WARPS, smem, a.st>>>(
-        a.tasks, a.order, a.n_tasks, a.prep, a.arena, a.sc, gp, a.bias, a.counters, a.qmax, a.redo, a.n_redo);
+        a.tasks, a.order, a.n_tasks, a.prep, a.arena, a.sc, gp, a.bias, a.counters, a.qmax, a.redo, a.n_redo,
+        a.hscratch);
 }
 
 template <bool PAIR>

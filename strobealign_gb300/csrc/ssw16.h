@@ -20,6 +20,7 @@ struct Ssw16Args {
     uint32_t qmax;     // tasks of longer reads are left to another kernel
     uint32_t* redo;    // tasks to run again on the warp-per-task kernel, and their count
     uint32_t* n_redo;
+    int32_t* hscratch;  // per-job scratch (PrepRec::h_off), for ungapped tasks' CIGARs
     cudaStream_t st;
 };
 
