@@ -59,6 +59,12 @@ inline uint64_t sm_count() {
     return cached;
 }
 
+// Device memory from a bounded cache of freed blocks (devmem.cpp); null when there is none.
+// dev_free waits for the device, as cudaFree does; dev_trim gives the cache back.
+void* dev_alloc(size_t bytes);
+void dev_free(void* p);
+void dev_trim();
+
 // Device buffer with RAII release.
 template <class T>
 struct DevBuf {
@@ -69,7 +75,7 @@ struct DevBuf {
     DevBuf& operator=(const DevBuf&) = delete;
     ~DevBuf() { release(); }
     void release() {
-        if (p) cudaFree(p);
+        dev_free(p);
         p = nullptr;
         n = 0;
     }
@@ -78,11 +84,8 @@ struct DevBuf {
         if (count <= n && p) return;
         release();
         size_t c = std::max<size_t>(count, 1);
-        cudaError_t e = cudaMalloc(&p, c * sizeof(T));
-        if (e != cudaSuccess) {
-            p = nullptr;
-            throw Error(SA_ERR_OOM, "cudaMalloc of " + std::to_string(c * sizeof(T)) + " bytes failed");
-        }
+        p = static_cast<T*>(dev_alloc(c * sizeof(T)));
+        if (!p) throw Error(SA_ERR_OOM, "cudaMalloc of " + std::to_string(c * sizeof(T)) + " bytes failed");
         n = c;
     }
 };

@@ -112,6 +112,7 @@ Session::Session(const sa_index* idx, const sa_refs* refs, const sa_chaining_par
     // memory-based admission: the arena and the lanes' workspaces come out of the free
     // device memory, less a reserve kept for everything else on the device
     size_t mem_free = 0, mem_total = 0;
+    dev_trim();
     SA_CUDA(cudaMemGetInfo(&mem_free, &mem_total));
     reserve_ = cfg_.device_reserve_bytes ? cfg_.device_reserve_bytes
                                          : std::max<uint64_t>(2ull << 30, (uint64_t)mem_total / 20);
@@ -410,6 +411,7 @@ void Session::admitter(AdmitLane& lane) {
             const uint64_t need = growth(bases);
             if (!need) return true;
             size_t f = 0, t = 0;
+            dev_trim();
             if (cudaMemGetInfo(&f, &t) != cudaSuccess) return false;
             return (uint64_t)f >= reserve_ + pending_growth_ + need;
         };
