@@ -41,7 +41,7 @@ Mapper::Mapper(const sa_index* idx, const sa_refs* refs, const sa_chaining_param
     SA_CUDA(cudaStreamCreateWithFlags(&st_, cudaStreamNonBlocking));
     int prio_least = 0, prio_greatest = 0;
     SA_CUDA(cudaDeviceGetStreamPriorityRange(&prio_least, &prio_greatest));
-    SA_CUDA(cudaStreamCreateWithPriority(&stn_, cudaStreamNonBlocking, prio_greatest));
+    for (NamLane& l : lanes_) SA_CUDA(cudaStreamCreateWithPriority(&l.st, cudaStreamNonBlocking, prio_greatest));
     const auto& cs = refs->contigs;
     const uint32_t nc = (uint32_t)cs.size();
     std::vector<uint64_t> woff(nc);
@@ -80,42 +80,57 @@ Mapper::~Mapper() {
     // the fetch granularity is the context's: give back the value found at construction
     if (l2_fetch_ && l2_fetch_default_) cudaDeviceSetLimit(cudaLimitMaxL2FetchGranularity, l2_fetch_default_);
     if (st_) cudaStreamDestroy(st_);
-    if (stn_) cudaStreamDestroy(stn_);
+    for (NamLane& l : lanes_)
+        if (l.st) cudaStreamDestroy(l.st);
 }
 
-void Mapper::upload_reads(const ReadSpan& reads) {
-    uint64_t total = 0;
-    for (size_t i = 0; i < reads.size(); i++) {
-        if (reads[i].len > MAX_READ_LEN)
-            throw Error(SA_ERR_INVALID, "read longer than " + std::to_string(MAX_READ_LEN) + " nt");
-        total += reads[i].len;
-    }
-    const uint32_t n = (uint32_t)reads.size();
-    h_seq_.reserve(total + 16);
-    h_off_.reserve((size_t)n + 1);
-    uint64_t o = 0;
-    for (uint32_t i = 0; i < n; i++) {
-        h_off_.p[i] = o;
-        o += reads[i].len;
-    }
-    h_off_.p[n] = o;
-    // the bases into pinned staging, in parallel
-    parallel_ranges(n, policy_threads_, [&](uint64_t a, uint64_t b) {
-        for (uint64_t i = a; i < b; i++) std::memcpy(h_seq_.p + h_off_.p[i], reads[i].seq, reads[i].len);
+// Views and offsets of the batch's reads, in one parallel pass (a read's offset follows
+// from the caller's offsets); the bases stay where they are.  Refuses reads that the
+// kernels do not take before anything is uploaded.
+template <class View>
+void Mapper::prepare_reads(uint64_t n_rec, unsigned per_rec, uint64_t total, View view) {
+    const uint64_t n = n_rec * per_rec;
+    reads_.resize(n);
+    h_off_.reserve(n + 1);
+    std::atomic<uint64_t> longest{1};
+    parallel_ranges(n_rec, policy_threads_, [&](uint64_t a, uint64_t b) {
+        uint64_t mx = 1;
+        for (uint64_t i = a; i < b; i++) mx = std::max(mx, view(i));
+        uint64_t cur = longest.load();
+        while (mx > cur && !longest.compare_exchange_weak(cur, mx)) {
+        }
     });
+    if (longest > MAX_READ_LEN)
+        throw Error(SA_ERR_INVALID, "read longer than " + std::to_string(MAX_READ_LEN) + " nt");
+    max_qlen_ = (uint32_t)longest;
+    h_off_.p[n] = total;
+    h_seq_.reserve(total + 16);
     nws_.seq.reserve(total + 16);
-    nws_.off.reserve((size_t)n + 1);
-    SA_CUDA(cudaMemcpyAsync(nws_.seq.p, h_seq_.p, total, cudaMemcpyHostToDevice, st_));
-    SA_CUDA(cudaMemcpyAsync(nws_.off.p, h_off_.p, ((size_t)n + 1) * 8, cudaMemcpyHostToDevice, st_));
+    nws_.off.reserve(n + 1);
+    SA_CUDA(cudaMemcpyAsync(nws_.off.p, h_off_.p, (n + 1) * 8, cudaMemcpyHostToDevice, st_));
+    bv_.reads = ReadSpan{reads_.data(), reads_.size()};
     total_bases_ = total;
-    n_reads_ = n;
-    h2d_bytes_ += total + ((size_t)n + 1) * 8;
+    n_reads_ = (uint32_t)n;
+    h2d_bytes_ = (n + 1) * 8;
+    have_batch_ = true;
 }
 
-// The NAM pipeline for one part, on stn_: the part's bases are copied out of the
-// uploaded batch with local offsets, and its NAMs, statistics (and for single-end
-// piecewise extension the NAMs' chain anchors) come back into the part's pinned buffers.
-void Mapper::part_nams(Part& p, uint32_t& launches) {
+// The prepared batch's bases onto the device.
+void Mapper::upload_all() {
+    // into pinned staging, in parallel
+    parallel_ranges(n_reads_, policy_threads_, [&](uint64_t a, uint64_t b) {
+        for (uint64_t i = a; i < b; i++) std::memcpy(h_seq_.p + h_off_.p[i], reads_[i].seq, reads_[i].len);
+    });
+    SA_CUDA(cudaMemcpyAsync(nws_.seq.p, h_seq_.p, total_bases_, cudaMemcpyHostToDevice, st_));
+    h2d_bytes_ += total_bases_;
+    SA_CUDA(cudaStreamSynchronize(st_));
+}
+
+// The NAM pipeline for one part, on its lane: the part's bases are uploaded if the batch's
+// are not on the device yet, and copied with local offsets; its NAMs, statistics (and for
+// single-end piecewise extension the NAMs' chain anchors) come back into the part's pinned
+// buffers.
+void Mapper::part_nams(Part& p, NamLane& lane, uint32_t& launches) {
     const auto t0 = std::chrono::steady_clock::now();
     const uint32_t n = p.read_hi - p.read_lo;
     const uint64_t base = h_off_.p[p.read_lo], total = h_off_.p[p.read_hi] - base;
@@ -126,41 +141,55 @@ void Mapper::part_nams(Part& p, uint32_t& launches) {
     cfg.rescue_distance = mp_.rescue_distance;
     cfg.nam_anchors = single_end_piecewise_ && (!bv_.paired || bv_.rec_read);
     cfg.chain_lane_max = chain_lane_max_;
-    pws_.seq.reserve(total + 16);
-    pws_.off.reserve((size_t)n + 1);
-    h_poff_.reserve((size_t)n + 1);
-    for (uint32_t i = 0; i <= n; i++) h_poff_.p[i] = h_off_.p[p.read_lo + i] - base;
-    if (total) SA_CUDA(cudaMemcpyAsync(pws_.seq.p, nws_.seq.p + base, total, cudaMemcpyDeviceToDevice, stn_));
-    SA_CUDA(cudaMemcpyAsync(pws_.off.p, h_poff_.p, ((size_t)n + 1) * 8, cudaMemcpyHostToDevice, stn_));
+    NamWorkspace& ws = lane.ws;
+    const cudaStream_t st = lane.st;
+    ws.seq.reserve(total + 16);
+    ws.off.reserve((size_t)n + 1);
+    lane.off.reserve((size_t)n + 1);
+    for (uint32_t i = 0; i <= n; i++) lane.off.p[i] = h_off_.p[p.read_lo + i] - base;
+    if (pending_ && total) {
+        parallel_ranges(n, std::min(policy_threads_, 4u), [&](uint64_t a, uint64_t b) {
+            for (uint64_t i = p.read_lo + a; i < p.read_lo + b; i++)
+                std::memcpy(h_seq_.p + h_off_.p[i], reads_[i].seq, reads_[i].len);
+        });
+        SA_CUDA(cudaMemcpyAsync(nws_.seq.p + base, h_seq_.p + base, total, cudaMemcpyHostToDevice, st));
+        h2d_bytes_ += total;
+    }
+    if (total) SA_CUDA(cudaMemcpyAsync(ws.seq.p, nws_.seq.p + base, total, cudaMemcpyDeviceToDevice, st));
+    SA_CUDA(cudaMemcpyAsync(ws.off.p, lane.off.p, ((size_t)n + 1) * 8, cudaMemcpyHostToDevice, st));
     launches += run_nam_pipeline(idx_->view(), refs_view_, cfg, n, total, max_contig_len_,
-                                 (uint32_t)refs_->contigs.size(), pws_, stn_, &kt_nam_);
-    const uint64_t tn = pws_.last_total_nams;
+                                 (uint32_t)refs_->contigs.size(), ws, st, &kt_nam_);
+    const uint64_t tn = ws.last_total_nams;
     p.n_nams = tn;
     uint64_t d2h = 0;
     if (cfg.nam_anchors) {
-        const uint64_t ta = pws_.last_total_nam_anchors;
+        const uint64_t ta = ws.last_total_nam_anchors;
         p.anc_off.reserve(tn + 1);
         p.anc.reserve(ta);
-        SA_CUDA(cudaMemcpyAsync(p.anc_off.p, pws_.nam_anc_off.p, (tn + 1) * 8, cudaMemcpyDeviceToHost, stn_));
-        if (ta) SA_CUDA(cudaMemcpyAsync(p.anc.p, pws_.nam_anc.p, ta * 8, cudaMemcpyDeviceToHost, stn_));
+        SA_CUDA(cudaMemcpyAsync(p.anc_off.p, ws.nam_anc_off.p, (tn + 1) * 8, cudaMemcpyDeviceToHost, st));
+        if (ta) SA_CUDA(cudaMemcpyAsync(p.anc.p, ws.nam_anc.p, ta * 8, cudaMemcpyDeviceToHost, st));
         d2h += (tn + 1) * 8 + ta * 8;
     }
     p.nam_off.reserve((size_t)n + 1);
     p.nams.reserve(tn);
     p.details.reserve(n);
-    SA_CUDA(cudaMemcpyAsync(p.nam_off.p, pws_.nam_off.p, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, stn_));
-    if (tn) SA_CUDA(cudaMemcpyAsync(p.nams.p, pws_.nams.p, tn * sizeof(NamRec), cudaMemcpyDeviceToHost, stn_));
-    SA_CUDA(cudaMemcpyAsync(p.details.p, pws_.details.p, (size_t)n * sizeof(NamDetailsRec), cudaMemcpyDeviceToHost,
-                            stn_));
-    SA_CUDA(cudaStreamSynchronize(stn_));
+    SA_CUDA(cudaMemcpyAsync(p.nam_off.p, ws.nam_off.p, ((size_t)n + 1) * 8, cudaMemcpyDeviceToHost, st));
+    if (tn) SA_CUDA(cudaMemcpyAsync(p.nams.p, ws.nams.p, tn * sizeof(NamRec), cudaMemcpyDeviceToHost, st));
+    SA_CUDA(cudaMemcpyAsync(p.details.p, ws.details.p, (size_t)n * sizeof(NamDetailsRec), cudaMemcpyDeviceToHost, st));
+    SA_CUDA(cudaStreamSynchronize(st));
     d2h += ((size_t)n + 1) * 8 + tn * sizeof(NamRec) + (size_t)n * sizeof(NamDetailsRec);
     p.bv.nams = p.nams.p;
     p.bv.nam_off = p.nam_off.p;
     p.bv.details = p.details.p;
     p.bv.nam_anc_off = cfg.nam_anchors ? p.anc_off.p : nullptr;
     p.bv.nam_anc = cfg.nam_anchors ? p.anc.p : nullptr;
-    p.bv.anc_qbits = pws_.anchor_qbits;
-    p.bv.anc_pbits = pws_.anchor_pbits;
+    p.bv.anc_qbits = ws.anchor_qbits;
+    p.bv.anc_pbits = ws.anchor_pbits;
+    p.n_randstrobes = p.n_anchors = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        p.n_randstrobes += p.details.p[i].n_randstrobes;
+        p.n_anchors += p.details.p[i].n_anchors;
+    }
     p.seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     d2h_bytes_ += d2h;  // atomic: the wave thread adds its transfers meanwhile
     h2d_bytes_ += ((size_t)n + 1) * 8;
@@ -216,77 +245,88 @@ ReadView read_view(const sa_read_batch* b, uint64_t i) {
 }
 }  // namespace
 
-void Mapper::upload(const sa_read_batch* r1, const sa_read_batch* r2) {
-    auto t0 = std::chrono::steady_clock::now();
+void Mapper::prepare(const sa_read_batch* r1, const sa_read_batch* r2) {
     const bool paired = r2 != nullptr;
     if (paired && r2->n != r1->n) throw Error(SA_ERR_INVALID, "r1 and r2 batches differ in size");
-    const uint64_t nrec = r1->n;
+    have_batch_ = false;
     bv_ = BatchView();
     bv_.paired = paired;
     rec_read_.clear();
-    reads_.resize(paired ? 2 * nrec : nrec);
-    auto view = read_view;
-    parallel_ranges(nrec, policy_threads_, [&](uint64_t a, uint64_t b) {
-        for (uint64_t i = a; i < b; i++) {
-            if (paired) {
-                reads_[2 * i] = view(r1, i);
-                reads_[2 * i + 1] = view(r2, i);
-            } else {
-                reads_[i] = view(r1, i);
-            }
+    const uint64_t n = r1->n, o1 = r1->seq_offsets[0], o2 = paired ? r2->seq_offsets[0] : 0;
+    const uint64_t total = r1->seq_offsets[n] - o1 + (paired ? r2->seq_offsets[n] - o2 : 0);
+    prepare_reads(n, paired ? 2 : 1, total, [&](uint64_t i) {
+        const uint64_t l1 = r1->seq_offsets[i + 1] - r1->seq_offsets[i];
+        if (!paired) {
+            reads_[i] = read_view(r1, i);
+            h_off_.p[i] = r1->seq_offsets[i] - o1;
+            return l1;
         }
+        reads_[2 * i] = read_view(r1, i);
+        reads_[2 * i + 1] = read_view(r2, i);
+        h_off_.p[2 * i] = r1->seq_offsets[i] - o1 + r2->seq_offsets[i] - o2;
+        h_off_.p[2 * i + 1] = r1->seq_offsets[i + 1] - o1 + r2->seq_offsets[i] - o2;
+        return std::max(l1, (uint64_t)(r2->seq_offsets[i + 1] - r2->seq_offsets[i]));
     });
-    max_qlen_ = 1;
-    bv_.reads = ReadSpan{reads_.data(), reads_.size()};
-    for (auto& r : reads_) max_qlen_ = std::max(max_qlen_, r.len);
-    h2d_bytes_ = 0;
-    upload_reads(bv_.reads);
-    SA_CUDA(cudaStreamSynchronize(st_));
-    have_batch_ = true;
+}
+
+void Mapper::prepare_interleaved(const sa_read_batch* reads) {
+    const uint64_t n = reads->n;
+    if (n >= UINT32_MAX) throw Error(SA_ERR_INVALID, "batch too large");
+    have_batch_ = false;
+    bv_ = BatchView();
+    pair_records_by_name(*reads, true, rec_read_);
+    bv_.rec_read = rec_read_.data();
+    const uint64_t o = reads->seq_offsets[0];
+    prepare_reads(n, 1, reads->seq_offsets[n] - o, [&](uint64_t i) {
+        reads_[i] = read_view(reads, i);
+        h_off_.p[i] = reads->seq_offsets[i] - o;
+        return (uint64_t)(reads->seq_offsets[i + 1] - reads->seq_offsets[i]);
+    });
+}
+
+void Mapper::upload(const sa_read_batch* r1, const sa_read_batch* r2) {
+    auto t0 = std::chrono::steady_clock::now();
+    prepare(r1, r2);
+    upload_all();
     stats_.seconds_upload = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
 }
 
 void Mapper::upload_interleaved(const sa_read_batch* reads) {
     auto t0 = std::chrono::steady_clock::now();
-    const uint64_t n = reads->n;
-    if (n >= UINT32_MAX) throw Error(SA_ERR_INVALID, "batch too large");
-    bv_ = BatchView();
-    reads_.resize(n);
-    parallel_ranges(n, policy_threads_, [&](uint64_t a, uint64_t b) {
-        for (uint64_t i = a; i < b; i++) reads_[i] = read_view(reads, i);
-    });
-    pair_records_by_name(*reads, true, rec_read_);
-    bv_.rec_read = rec_read_.data();
-    max_qlen_ = 1;
-    bv_.reads = ReadSpan{reads_.data(), reads_.size()};
-    for (auto& r : reads_) max_qlen_ = std::max(max_qlen_, r.len);
-    h2d_bytes_ = 0;
-    upload_reads(bv_.reads);
-    SA_CUDA(cudaStreamSynchronize(st_));
-    have_batch_ = true;
+    prepare_interleaved(reads);
+    upload_all();
     stats_.seconds_upload = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+}
+
+// A prepared batch mapped while its bases are uploaded, a part at a time.
+void Mapper::map_prepared(std::chrono::steady_clock::time_point t0, sa_output* out) {
+    const uint64_t h2d = h2d_bytes_;
+    const double tu = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    pending_ = true;
+    try {
+        map_uploaded(out);
+    } catch (...) {
+        // some parts may not be on the device
+        pending_ = false;
+        have_batch_ = false;
+        throw;
+    }
+    pending_ = false;
+    stats_.seconds_upload = tu;
+    stats_.h2d_bytes += h2d;
+    stats_.seconds_total = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
 }
 
 void Mapper::map_interleaved(const sa_read_batch* reads, sa_output* out) {
     auto t0 = std::chrono::steady_clock::now();
-    upload_interleaved(reads);
-    uint64_t h2d = h2d_bytes_;
-    double tu = stats_.seconds_upload;
-    map_uploaded(out);
-    stats_.seconds_upload = tu;
-    stats_.h2d_bytes += h2d;
-    stats_.seconds_total = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    prepare_interleaved(reads);
+    map_prepared(t0, out);
 }
 
 void Mapper::map(const sa_read_batch* r1, const sa_read_batch* r2, sa_output* out) {
     auto t0 = std::chrono::steady_clock::now();
-    upload(r1, r2);
-    uint64_t h2d = h2d_bytes_;
-    double tu = stats_.seconds_upload;
-    map_uploaded(out);
-    stats_.seconds_upload = tu;
-    stats_.h2d_bytes += h2d;
-    stats_.seconds_total = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+    prepare(r1, r2);
+    map_prepared(t0, out);
 }
 
 // Continuous batching of extension work.  Chunks are independent (fresh RNG and
@@ -310,28 +350,38 @@ uint32_t Mapper::schedule(std::vector<ChunkState>& chunks, uint32_t& launches, u
     std::vector<bool> is_seeded(nchunks, false);
     bool nam_done = false;  // every part's NAMs are in (the plain form waits for it)
 
-    // NAM pipelines part by part; a part's chunks become ready once its NAMs are in
-    std::thread nam_thread([&]() {
+    // NAM pipelines, a part at a time on each lane; a part's chunks become ready once its
+    // NAMs are in.  The plain form and profiled maps (their events time one stream) use one.
+    const unsigned n_lanes = overlap_ && !kt_nam_.enabled && n_parts_ > 1 ? NAM_LANES : 1;
+    size_t next_part = 0, parts_done = 0;
+    std::vector<std::thread> nam_threads;
+    auto nam_lane = [&](unsigned l) {
         try {
-            for (size_t pi = 0; pi < n_parts_; pi++) {
+            SA_CUDA(cudaSetDevice(idx_->device));
+            for (;;) {
+                size_t pi;
                 {
                     std::lock_guard<std::mutex> g(mu);
-                    if (stop) return;
+                    if (stop || next_part >= n_parts_) return;
+                    pi = next_part++;
                 }
                 Part& p = *parts_[pi];
-                part_nams(p, nam_launches);
-                if (!overlap_) continue;  // the plain form starts the policy after the last part
+                uint32_t nl = 0;
+                part_nams(p, lanes_[l], nl);
                 std::lock_guard<std::mutex> g(mu);
-                for (size_t c = p.chunk_lo; c < p.chunk_hi; c++) ready.push_back(c);
+                nam_launches += nl;
+                parts_done++;
+                if (overlap_)
+                    for (size_t c = p.chunk_lo; c < p.chunk_hi; c++) ready.push_back(c);
+                if (parts_done == n_parts_) {
+                    // the plain form starts the policy after the last part
+                    if (!overlap_)
+                        for (size_t c = 0; c < nchunks; c++) ready.push_back(c);
+                    nam_done = true;
+                }
                 cv_work.notify_all();
                 cv_ext.notify_one();
             }
-            std::lock_guard<std::mutex> g(mu);
-            if (!overlap_)
-                for (size_t c = 0; c < nchunks; c++) ready.push_back(c);
-            nam_done = true;
-            cv_work.notify_all();
-            cv_ext.notify_one();
         } catch (...) {
             std::lock_guard<std::mutex> g(mu);
             if (!err) err = std::current_exception();
@@ -339,7 +389,8 @@ uint32_t Mapper::schedule(std::vector<ChunkState>& chunks, uint32_t& launches, u
             cv_work.notify_all();
             cv_ext.notify_all();
         }
-    });
+    };
+    for (unsigned l = 0; l < n_lanes; l++) nam_threads.emplace_back(nam_lane, l);
 
     auto worker = [&]() {
         // one policy per thread, bound to each chunk's part in turn
@@ -515,7 +566,7 @@ uint32_t Mapper::schedule(std::vector<ChunkState>& chunks, uint32_t& launches, u
         cv_work.notify_all();
     }
     for (auto& t : th) t.join();
-    nam_thread.join();
+    for (auto& t : nam_threads) t.join();
     if (err) std::rethrow_exception(err);
     return waves;
 }
@@ -702,12 +753,9 @@ void Mapper::map_uploaded(sa_output* out) {
     {
         uint64_t rs = 0, an = 0, nn = 0;
         for (size_t pi = 0; pi < n_parts_; pi++) {
-            const Part& p = *parts_[pi];
-            nn += p.n_nams;
-            for (uint32_t i = 0; i < p.read_hi - p.read_lo; i++) {
-                rs += p.details.p[i].n_randstrobes;
-                an += p.details.p[i].n_anchors;
-            }
+            nn += parts_[pi]->n_nams;
+            rs += parts_[pi]->n_randstrobes;
+            an += parts_[pi]->n_anchors;
         }
         stats_.n_nams = nn;
         stats_.n_anchors = an;

@@ -34,7 +34,6 @@ class Mapper {
     NamWorkspace& nam_ws() { return nws_; }
     ExtWorkspace& ext_ws() { return ews_; }
     cudaStream_t stream() const { return st_; }
-    void upload_reads(const ReadSpan& reads);
     uint32_t n_reads() const { return n_reads_; }
     uint64_t total_bases() const { return total_bases_; }
     uint64_t h2d_bytes() const { return h2d_bytes_; }
@@ -91,10 +90,26 @@ class Mapper {
         PinnedBuf<NamRec> nams;
         PinnedBuf<NamDetailsRec> details;
         PinnedBuf<uint64_t> anc_off, anc;  // single-end piecewise: NAM chain anchors
-        uint64_t n_nams = 0;
+        uint64_t n_nams = 0, n_randstrobes = 0, n_anchors = 0;
         double seconds = 0;
     };
-    void part_nams(Part& p, uint32_t& launches);
+    // The stream and buffers of a NAM pipeline.  Two parts run at once: the end of one
+    // (its longest cluster's serial chain, its copies to the host) leaves most of the
+    // device to the next one's seeding and lookups.
+    struct NamLane {
+        cudaStream_t st = nullptr;  // highest priority
+        NamWorkspace ws;
+        PinnedBuf<uint64_t> off;  // the part's local read offsets
+    };
+    static constexpr unsigned NAM_LANES = 2;
+    void part_nams(Part& p, NamLane& lane, uint32_t& launches);
+    void prepare(const sa_read_batch* r1, const sa_read_batch* r2);
+    void prepare_interleaved(const sa_read_batch* reads);
+    // view(i) sets record i's read views and offsets and returns its longest read's length
+    template <class View>
+    void prepare_reads(uint64_t n_rec, unsigned per_rec, uint64_t total, View view);
+    void upload_all();
+    void map_prepared(std::chrono::steady_clock::time_point t0, sa_output* out);
     std::shared_ptr<const WaveResults> run_wave(const ExtJob* jobs, uint32_t nj, uint32_t max_qlen,
                                                 uint32_t& launches, const uint32_t* anchors, size_t anchor_words,
                                                 uint32_t max_anchors);
@@ -105,6 +120,7 @@ class Mapper {
     // empty for uniform batches
     std::vector<uint32_t> rec_read_;
     bool have_batch_ = false;
+    bool pending_ = false;  // the batch's bases are uploaded part by part, by the NAM pipelines
     uint32_t max_qlen_ = 1;
     sa_mapper_stats stats_{};
     double t_ext_ = 0;
@@ -126,7 +142,6 @@ class Mapper {
     std::string rg_id_;
     PolicyConfig pcfg_;
     cudaStream_t st_ = nullptr;   // uploads and extension waves
-    cudaStream_t stn_ = nullptr;  // NAM pipelines of the parts (highest priority)
     DevBuf<uint64_t> d_words_, d_woff_;
     DevBuf<uint32_t> d_clen_;
     DevRefs refs_view_{};
@@ -142,8 +157,7 @@ class Mapper {
     std::vector<std::unique_ptr<Part>> parts_;  // grow-only; pinned buffers reused across batches
     size_t n_parts_ = 0;
     uint32_t parts_target_ = 8;
-    NamWorkspace pws_;            // NAM pipeline buffers of one part
-    PinnedBuf<uint64_t> h_poff_;  // a part's local read offsets
+    NamLane lanes_[NAM_LANES];
     double t_nams_ = 0;
     std::chrono::steady_clock::time_point t_map0_;  // start of the current map (trace times)
     PodArray<uint32_t> wave_anchors_;  // a wave's piecewise anchors (query, reference start pairs)
