@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) k_seed(const uint8_t* __restrict__ seq, c
 
 // ------------------------------------------------------------------ hits
 struct HitsCounts {
-    uint32_t fnf, ff, ffound, pnf, pf, pfound, rescued;
+    uint32_t fnf = 0, ff = 0, ffound = 0, pnf = 0, pf = 0, pfound = 0, rescued = 0;
 };
 
 __device__ __forceinline__ uint32_t warp_sum(uint32_t v) {
@@ -293,16 +293,11 @@ __global__ void __launch_bounds__(256) k_probe(DevIndex ix, const uint64_t* __re
             const uint64_t slot = ori * total + o + (j - ori * n0);
             const uint64_t h = qr_hash[slot];
             uint64_t pos;
-            bool filtered;
-            idx_full_probe(ix, h, qr_hash_rc[slot], cutoff, pos, filtered);
+            bool filtered, partial;
+            idx_full_probe(ix, h, qr_hash_rc[slot], cutoff, mcs == SA_MCS_ALWAYS, pos, filtered, partial);
             uint32_t flags = 0;
-            if (pos != UINT64_MAX) {
-                flags = PROBE_FULL | (filtered ? PROBE_FILTERED : 0u);
-            } else if (mcs == SA_MCS_ALWAYS) {
-                pos = idx_get_masked_from(ix, h, ix.p.main_mask, false, 0);
-                if (pos != UINT64_MAX)
-                    flags = PROBE_PARTIAL | (idx_too_frequent_partial(ix, pos, cutoff) ? PROBE_FILTERED : 0u);
-            }
+            if (pos != UINT64_MAX)
+                flags = (partial ? PROBE_PARTIAL : PROBE_FULL) | (filtered ? PROBE_FILTERED : 0u);
             hit_pos[slot] = pos;
             hit_info[slot] = flags;
         }
@@ -311,7 +306,9 @@ __global__ void __launch_bounds__(256) k_probe(DevIndex ix, const uint64_t* __re
 
 // find_hits (src/hit.rs:129-333) for both orientations of each read, then the
 // orientation heuristic (src/chainer.rs:205-216, src/hit.rs:76-81).  The first pass
-// reads k_probe's per-slot answers.
+// reads k_probe's per-slot answers.  Counts come from ballots, and the walk over filtered
+// stretches, hit after hit on one lane, is entered only when some stretch is long enough
+// (0.7 M reads: 2.0 ms with six warp sums per orientation and the walk for every read, 1.1 ms).
 __global__ void __launch_bounds__(256) k_hits(DevIndex ix, const uint64_t* __restrict__ off, uint32_t n,
                                               uint64_t total, uint32_t mcs, uint32_t rescue_distance,
                                               const uint64_t* qr_hash, const uint64_t* qr_hash_rc,
@@ -329,7 +326,7 @@ __global__ void __launch_bounds__(256) k_hits(DevIndex ix, const uint64_t* __res
             const uint64_t b = ori * total + o;
             const uint32_t nr = n_rs[2 * r + ori];
             uint32_t nh = 0;
-            uint32_t fnf = 0, ff = 0, ffound = 0, pnf = 0, pf = 0, pfound = 0;
+            HitsCounts d;  // the same in every lane: counted by ballots
             const bool do_full = mcs != SA_MCS_FIRST_STROBE;
             // pass 1: full lookups (with partial fallback under MCS always), probed by
             // k_probe; compacted in place (a slot is written only after every lane of
@@ -337,42 +334,35 @@ __global__ void __launch_bounds__(256) k_hits(DevIndex ix, const uint64_t* __res
             if (do_full) {
                 for (uint32_t c = 0; c < nr; c += 32) {
                     uint32_t i = c + lane;
-                    bool is_hit = false, partial = false, filtered = false;
+                    uint32_t fl = 0;
                     uint64_t pos = UINT64_MAX;
                     if (i < nr) {
-                        const uint32_t fl = hit_info[b + i];
+                        fl = hit_info[b + i];
                         pos = hit_pos[b + i];
-                        filtered = fl & PROBE_FILTERED;
-                        if (fl & PROBE_FULL) {
-                            is_hit = true;
-                            if (filtered) ff++;
-                            else ffound++;
-                        } else {
-                            fnf++;
-                            if (mcs == SA_MCS_ALWAYS) {
-                                if (fl & PROBE_PARTIAL) {
-                                    is_hit = partial = true;
-                                    if (filtered) pf++;
-                                    else pfound++;
-                                } else {
-                                    pnf++;
-                                }
-                            }
-                        }
                     }
-                    uint32_t bal = __ballot_sync(FULL, is_hit);
+                    const bool filtered = fl & PROBE_FILTERED, partial = fl & PROBE_PARTIAL;
+                    const bool is_hit = fl & (PROBE_FULL | PROBE_PARTIAL);
+                    const uint32_t in = __ballot_sync(FULL, i < nr), full = __ballot_sync(FULL, fl & PROBE_FULL),
+                                   part = __ballot_sync(FULL, partial), filt = __ballot_sync(FULL, filtered);
+                    d.ff += __popc(full & filt);
+                    d.ffound += __popc(full & ~filt);
+                    d.fnf += __popc(in & ~full);
+                    if (mcs == SA_MCS_ALWAYS) {
+                        d.pf += __popc(part & filt);
+                        d.pfound += __popc(part & ~filt);
+                        d.pnf += __popc(in & ~full & ~part);
+                    }
+                    const uint32_t bal = full | part;
                     __syncwarp();
                     if (is_hit) {
                         uint32_t idx = nh + __popc(bal & lanemask_lt());
                         hit_pos[b + idx] = pos;
                         hit_info[b + idx] = (i << 3) | (filtered ? 4u : 0u) | (partial ? 2u : 0u) | 1u;
-                        cache[b + idx] = 0xffffffffu;
                     }
                     nh += __popc(bal);
                 }
             }
-            uint32_t full_hits = warp_sum(ff + ffound);
-            bool partial_pass = mcs == SA_MCS_FIRST_STROBE || (mcs == SA_MCS_RESCUE && full_hits == 0);
+            bool partial_pass = mcs == SA_MCS_FIRST_STROBE || (mcs == SA_MCS_RESCUE && d.ff + d.ffound == 0);
             if (partial_pass) {
                 for (uint32_t c = 0; c < nr; c += 32) {
                     uint32_t i = c + lane;
@@ -383,43 +373,68 @@ __global__ void __launch_bounds__(256) k_hits(DevIndex ix, const uint64_t* __res
                         if (pos != UINT64_MAX) {
                             is_hit = true;
                             filtered = idx_too_frequent_partial(ix, pos, cutoff);
-                            if (filtered) pf++;
-                            else pfound++;
-                        } else {
-                            pnf++;
                         }
                     }
                     uint32_t bal = __ballot_sync(FULL, is_hit);
+                    const uint32_t in = __ballot_sync(FULL, i < nr), filt = __ballot_sync(FULL, filtered);
+                    d.pf += __popc(bal & filt);
+                    d.pfound += __popc(bal & ~filt);
+                    d.pnf += __popc(in & ~bal);
                     if (is_hit) {
                         uint32_t idx = nh + __popc(bal & lanemask_lt());
                         hit_pos[b + idx] = pos;
                         hit_info[b + idx] = (i << 3) | (filtered ? 4u : 0u) | 2u | 1u;
-                        cache[b + idx] = 0xffffffffu;
                     }
                     nh += __popc(bal);
                 }
             }
             __syncwarp();
-            HitsCounts d;
-            d.fnf = warp_sum(fnf);
-            d.ff = warp_sum(ff);
-            d.ffound = warp_sum(ffound);
-            d.pnf = warp_sum(pnf);
-            d.pf = warp_sum(pf);
-            d.pfound = warp_sum(pfound);
-            d.rescued = 0;
             // rescue (src/hit.rs:270-304)
             uint32_t total_hits = d.pf + d.pfound + d.ff + d.ffound;
             uint32_t nonrep = d.ffound + d.pfound;
             float frac = total_hits > 0 ? __fdiv_rn(__uint2float_rn(nonrep), __uint2float_rn(total_hits)) : 1.0f;
             if (rescue_distance > 0) {
-                if (frac < 0.7f && nonrep < 5)
+                // counts of the hits that a rescue may look at, none known yet
+                bool counts_ready = false;
+                auto ready = [&]() {
+                    if (!counts_ready)
+                        for (uint32_t h = lane; h < nh; h += 32) cache[b + h] = 0xffffffffu;
+                    counts_ready = true;
+                    __syncwarp();
+                };
+                if (frac < 0.7f && nonrep < 5) {
+                    ready();
                     d.rescued += warp_rescue_least_frequent(ix, 0, nh, 5, 1000, hit_pos + b, hit_info + b, cache + b,
                                                             qr_hash_rc + b);
+                }
+                // most reads have no filtered stretch to rescue: tested for all hits at once
+                // (the walk below reads hit after hit)
+                bool stretch = false;
+                {
+                    uint32_t last = 0, lq = 0;
+                    for (uint32_t c = 0; c < nh; c += 32) {
+                        const uint32_t h = c + lane;
+                        uint32_t qs = 0;
+                        bool unf = false;
+                        if (h < nh) {
+                            const uint32_t info = hit_info[b + h];
+                            qs = qr_start[b + (info >> 3)];
+                            unf = !(info & 4);
+                        }
+                        const uint32_t um = __ballot_sync(FULL, unf), lower = um & lanemask_lt();
+                        const uint32_t pq = __shfl_sync(FULL, qs, lower ? 31 - __clz(lower) : 0);
+                        stretch = stretch || __any_sync(FULL, unf && qs > (lower ? pq : last) + rescue_distance);
+                        const uint32_t lu = __shfl_sync(FULL, qs, um ? 31 - __clz(um) : 0);
+                        if (um) last = lu;
+                        lq = __shfl_sync(FULL, qs, (nh - 1 < c + 31 ? nh - 1 - c : 31));
+                    }
+                    if (nh > 0 && lq - last > rescue_distance) stretch = true;
+                }
+                if (stretch) ready();
                 // local rescue over filtered stretches (src/hit.rs:232-268); an interval is
                 // processed as soon as it is found, which only touches hits already scanned
                 uint32_t scan = 0, last_unf = 0, first_f = 0;
-                for (;;) {
+                while (stretch) {
                     uint32_t is = 0, ie = 0, tr = 0, found = 0;
                     if (lane == 0) {
                         while (scan < nh) {
@@ -592,14 +607,19 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t& total) 
     return x - v;
 }
 
-template <bool FILL>
+// The anchors of each read orientation (src/chainer.rs:304-384): counted, then written to
+// the next free range of the anchor array while the table entries are still in the L1 (a
+// launch each for counts and anchors read the table's random sectors twice: 11.2 KB of
+// DRAM per read on a human-sized index; 3.0 ms for 0.7 M reads, 2.3 ms now).  The ranges'
+// order does not matter to the stages after.  Past the array's capacity nothing is written; *cursor then tells what it
+// takes.
 __global__ void __launch_bounds__(256) k_anchors(DevIndex ix, const uint64_t* __restrict__ off, uint32_t n,
                                                  uint64_t total, const uint64_t* qr_hash, const uint32_t* qr_start,
                                                  const uint32_t* qr_end, const uint64_t* hit_pos,
                                                  const uint32_t* hit_info, const uint32_t* n_hits,
                                                  const uint8_t* orient, uint32_t* hit_anchors_n, uint64_t* seg_count,
-                                                 const uint64_t* seg_off, uint64_t* anchors, AnchorPack ap,
-                                                 NamDetailsRec* details) {
+                                                 uint64_t* seg_off, unsigned long long* cursor, uint64_t* anchors,
+                                                 uint64_t capacity, AnchorPack ap, NamDetailsRec* details) {
     const uint32_t lane = lane_id();
     const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
     for (uint32_t r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; r < n; r += nwarps) {
@@ -609,54 +629,69 @@ __global__ void __launch_bounds__(256) k_anchors(DevIndex ix, const uint64_t* __
         for (int ori = 0; ori < 2; ori++) {
             const uint64_t b = ori * total + o;
             const uint32_t nh = (m >> ori) & 1 ? n_hits[2 * r + ori] : 0;
-            uint64_t acc = FILL ? seg_off[2 * r + ori] : 0;
-            AnchorPack aps = ap;
             uint32_t sum = 0;
-            for (uint32_t c = 0; c < nh; c += 32) {
-                uint32_t h = c + lane;
-                uint32_t cnt = 0, head = 0, minld = 0xffffffffu;
-                uint32_t info = 0, qs = 0, qe = 0;
-                uint64_t start = 0, fh = 0;
-                bool has_run = false, is_long = false;
-                if (h < nh) {
-                    info = hit_info[b + h];
-                    if (!(info & 4)) {
-                        const uint32_t ri = info >> 3;
-                        qs = qr_start[b + ri];
-                        qe = (info & 2) ? qs + ix.p.k : qr_end[b + ri];
-                        has_run = hit_run(ix, hit_pos[b + h], info, qr_hash[b + ri], start, fh);
-                        if (FILL) cnt = hit_anchors_n[b + h];
+            uint64_t base = 0;
+            // pass 0 counts, pass 1 writes; the counts of up to 32 hits stay in registers
+            uint32_t info = 0, qs = 0, qe = 0, cnt = 0;
+            uint64_t start = 0, fh = 0;
+            bool has_run = false;
+            for (int pass = 0; pass < 2 && nh; pass++) {
+                uint64_t acc = base;
+                for (uint32_t c = 0; c < nh; c += 32) {
+                    const uint32_t h = c + lane;
+                    if (pass == 0 || nh > 32) {
+                        has_run = false;
+                        cnt = 0;
+                        if (h < nh) {
+                            info = hit_info[b + h];
+                            if (!(info & 4)) {
+                                const uint32_t ri = info >> 3;
+                                qs = qr_start[b + ri];
+                                qe = (info & 2) ? qs + ix.p.k : qr_end[b + ri];
+                                has_run = hit_run(ix, hit_pos[b + h], info, qr_hash[b + ri], start, fh);
+                                if (pass) cnt = hit_anchors_n[b + h];
+                            }
+                        }
                     }
+                    uint32_t tot = 0, ex = 0;
+                    if (pass) ex = warp_excl_scan(cnt, tot);
+                    uint64_t* out = pass ? anchors + acc + ex : nullptr;
+                    // each lane its run's first 32 entries; longer runs continue with the
+                    // whole warp, one hit at a time
+                    uint32_t head = 0, minld = 0xffffffffu;
+                    bool is_long = false;
+                    if (has_run) is_long = !run_head(ix, start, fh, info & 2, qs, qe, ap, out, head, minld);
+                    for (uint32_t lm = __ballot_sync(FULL, is_long); lm; lm &= lm - 1) {
+                        const int L = __ffs(lm) - 1;
+                        const uint32_t hL = __shfl_sync(FULL, head, L);
+                        const uint32_t rest = warp_run_anchors(
+                            ix, __shfl_sync(FULL, start, L) + 32, __shfl_sync(FULL, fh, L),
+                            __shfl_sync(FULL, info, L) & 2, __shfl_sync(FULL, qs, L), __shfl_sync(FULL, qe, L), ap,
+                            pass ? anchors + acc + __shfl_sync(FULL, ex, L) + hL : nullptr, __shfl_sync(FULL, minld, L));
+                        if (lane == (uint32_t)L) head += rest;
+                    }
+                    if (!pass) {
+                        cnt = head;
+                        if (nh > 32 && has_run) hit_anchors_n[b + h] = cnt;
+                        else if (nh > 32 && h < nh && !(info & 4)) hit_anchors_n[b + h] = 0;
+                        warp_excl_scan(cnt, tot);
+                        sum += tot;
+                    }
+                    acc += tot;
                 }
-                uint32_t tot = 0, ex = 0;
-                if (FILL) ex = warp_excl_scan(cnt, tot);
-                // each lane its run's first 32 entries; longer runs continue with the
-                // whole warp, one hit at a time
-                if (has_run)
-                    is_long = !run_head(ix, start, fh, info & 2, qs, qe, aps, FILL ? anchors + acc + ex : nullptr, head,
-                                        minld);
-                const uint32_t lm = __ballot_sync(FULL, is_long);
-                for (uint32_t m = lm; m; m &= m - 1) {
-                    const int L = __ffs(m) - 1;
-                    const uint32_t hL = __shfl_sync(FULL, head, L);
-                    const uint32_t rest = warp_run_anchors(
-                        ix, __shfl_sync(FULL, start, L) + 32, __shfl_sync(FULL, fh, L), __shfl_sync(FULL, info, L) & 2,
-                        __shfl_sync(FULL, qs, L), __shfl_sync(FULL, qe, L), aps,
-                        FILL ? anchors + acc + __shfl_sync(FULL, ex, L) + hL : nullptr, __shfl_sync(FULL, minld, L));
-                    if (lane == (uint32_t)L) head += rest;
+                if (pass == 0) {
+                    if (lane == 0 && sum) base = atomicAdd(cursor, (unsigned long long)sum);
+                    base = __shfl_sync(FULL, base, 0);
+                    if (sum == 0 || base + sum > capacity) break;
                 }
-                if (!FILL) {
-                    cnt = head;
-                    if (h < nh && !(info & 4)) hit_anchors_n[b + h] = cnt;
-                    ex = warp_excl_scan(cnt, tot);
-                }
-                acc += tot;
-                sum += tot;
             }
-            if (!FILL && lane == 0) seg_count[2 * r + ori] = sum;
+            if (lane == 0) {
+                seg_count[2 * r + ori] = sum;
+                seg_off[2 * r + ori] = base;
+            }
             read_total += sum;
         }
-        if (!FILL && lane == 0) details[r].n_anchors = read_total;
+        if (lane == 0) details[r].n_anchors = read_total;
     }
 }
 
@@ -1586,7 +1621,7 @@ __device__ __forceinline__ uint32_t orientation_dedup(const uint64_t* sorted, ui
 // k_chain4 checks each small record cluster for the first anchor where the re-check
 // fires (recheck_first_fire) and scores again from there only.
 __global__ void __launch_bounds__(128) k_chain_long_prep(const uint64_t* __restrict__ off, const uint64_t* seg_off,
-                                                         const uint64_t* sorted, uint64_t* dedup, float* dp,
+                                                         const uint64_t* seg_count, const uint64_t* sorted, uint64_t* dedup, float* dp,
                                                          uint32_t* pred, uint32_t* aux, uint64_t total_anchors,
                                                          AnchorPack ap, ChainCtx cc, const uint32_t* long_list,
                                                          uint32_t n_long, uint32_t* long_n, uint32_t* long_c,
@@ -1596,7 +1631,7 @@ __global__ void __launch_bounds__(128) k_chain_long_prep(const uint64_t* __restr
     const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
     for (uint32_t u = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; u < n_long; u += nwarps) {
         const uint32_t sg = long_list[u];
-        const uint64_t b = seg_off[sg], e = seg_off[sg + 1];
+        const uint64_t b = seg_off[sg], e = b + seg_count[sg];
         const uint32_t N = orientation_dedup(sorted, dedup, b, e);
         __syncwarp();
         const uint32_t read_len = (uint32_t)(off[(sg >> 1) + 1] - off[sg >> 1]);
@@ -1930,7 +1965,7 @@ __global__ void __launch_bounds__(128) k_chain_long(const uint64_t* __restrict__
 
 template <bool RING>
 __global__ void __launch_bounds__(32 * CHAIN_WARPS, 8) k_chain4(const uint64_t* __restrict__ off, uint32_t n, const uint64_t* seg_off,
-                                                const uint64_t* sorted, uint64_t* dedup, float* dp, uint32_t* pred,
+                                                const uint64_t* seg_count, const uint64_t* sorted, uint64_t* dedup, float* dp, uint32_t* pred,
                                                 uint32_t* aux, uint64_t total_anchors, AnchorPack ap, ChainCtx cc,
                                                 NamRec* nam_out, uint32_t* nam_seg_count, uint64_t* anc_out,
                                                 uint64_t* anc_start, const uint32_t* seg_list, uint32_t n_list) {
@@ -1957,7 +1992,7 @@ __global__ void __launch_bounds__(32 * CHAIN_WARPS, 8) k_chain4(const uint64_t* 
         for (uint32_t q = 0; q < NG; q++) {
             const uint32_t sg = __shfl_sync(FULL, my_sg, q);
             if (sg == NONE) continue;
-            const uint64_t b = seg_off[sg], e = seg_off[sg + 1];
+            const uint64_t b = seg_off[sg], e = b + seg_count[sg];
             const uint32_t N = orientation_dedup(sorted, dedup, b, e);
             if (lane == q) {
                 my_n = N;
@@ -2325,15 +2360,6 @@ uint32_t run_nam_pipeline(const DevIndex& ix, const DevRefs& refs, const NamConf
     ws.hit_anchors.reserve(2 * total);
     ws.seg_count.reserve(2 * (size_t)n + 1);
     ws.seg_off.reserve(2 * (size_t)n + 1);
-    kt->begin(KS_ANCHORS, st);
-    k_anchors<false><<<warps_grid(n), 32 * WARPS_PER_BLOCK, 0, st>>>(
-        ix, ws.off.p, n, total, ws.qr_hash.p, ws.qr_start.p, ws.qr_end.p, ws.hit_pos.p, ws.hit_info.p, ws.n_hits.p,
-        ws.orient.p, ws.hit_anchors.p, ws.seg_count.p, nullptr, nullptr, ap, ws.details.p);
-    kt->end(st);
-    launches++;
-    SA_CUDA(cudaMemsetAsync(ws.seg_count.p + 2 * (size_t)n, 0, 8, st));
-    cub_excl_sum(ws, ws.seg_count.p, ws.seg_off.p, 2 * (uint64_t)n + 1, st);
-    launches++;
     // seg_list: short list [0, 2n), long list [2n, 4n), counts at 4n
     ws.seg_list.reserve(4 * (size_t)n + 4);
     ws.sort_begin.reserve(2 * (size_t)n);
@@ -2343,24 +2369,31 @@ uint32_t run_nam_pipeline(const DevIndex& ix, const DevRefs& refs, const NamConf
     ws.seg_key.reserve(4 * (size_t)n);
     ws.seg_key_alt.reserve(4 * (size_t)n);
     ws.seg_sorted.reserve(4 * (size_t)n);
-    SA_CUDA(cudaMemsetAsync(list_counts, 0, 12, st));
-    k_seg_list<<<warps_grid((2 * (uint64_t)n + 31) / 32), 32 * WARPS_PER_BLOCK, 0, st>>>(
-        ws.seg_count.p, ws.seg_off.p, 2 * n, ws.seg_list.p, long_list, list_counts, ws.sort_begin.p, ws.sort_end.p,
-        ws.seg_key.p, ws.seg_key.p + 2 * (size_t)n);
-    launches++;
+    unsigned long long* const cursor = reinterpret_cast<unsigned long long*>(ws.seg_count.p + 2 * (size_t)n);
     uint64_t total_anchors = 0;
     uint32_t n_list[3] = {0, 0, 0};
-    SA_CUDA(cudaMemcpyAsync(&total_anchors, ws.seg_off.p + 2 * (size_t)n, 8, cudaMemcpyDeviceToHost, st));
-    SA_CUDA(cudaMemcpyAsync(n_list, list_counts, 12, cudaMemcpyDeviceToHost, st));
-    SA_CUDA(cudaStreamSynchronize(st));
-    ws.anchors.reserve(total_anchors);
+    // about 40 anchors per 150 nt read of a human-sized genome
+    ws.anchors.reserve(std::max<uint64_t>(ws.anchors.n, total / 3 + 64 * (uint64_t)n));
+    for (;;) {
+        SA_CUDA(cudaMemsetAsync(cursor, 0, 8, st));
+        SA_CUDA(cudaMemsetAsync(list_counts, 0, 12, st));
+        kt->begin(KS_ANCHORS, st);
+        k_anchors<<<warps_grid(n), 32 * WARPS_PER_BLOCK, 0, st>>>(
+            ix, ws.off.p, n, total, ws.qr_hash.p, ws.qr_start.p, ws.qr_end.p, ws.hit_pos.p, ws.hit_info.p, ws.n_hits.p,
+            ws.orient.p, ws.hit_anchors.p, ws.seg_count.p, ws.seg_off.p, cursor, ws.anchors.p, ws.anchors.n, ap,
+            ws.details.p);
+        kt->end(st);
+        k_seg_list<<<warps_grid((2 * (uint64_t)n + 31) / 32), 32 * WARPS_PER_BLOCK, 0, st>>>(
+            ws.seg_count.p, ws.seg_off.p, 2 * n, ws.seg_list.p, long_list, list_counts, ws.sort_begin.p, ws.sort_end.p,
+            ws.seg_key.p, ws.seg_key.p + 2 * (size_t)n);
+        launches += 2;
+        SA_CUDA(cudaMemcpyAsync(&total_anchors, cursor, 8, cudaMemcpyDeviceToHost, st));
+        SA_CUDA(cudaMemcpyAsync(n_list, list_counts, 12, cudaMemcpyDeviceToHost, st));
+        SA_CUDA(cudaStreamSynchronize(st));
+        if (total_anchors <= ws.anchors.n) break;
+        ws.anchors.reserve(total_anchors);  // did not fit: once more with room for all
+    }
     ws.anchors_sorted.reserve(total_anchors);
-    kt->begin(KS_ANCHORS, st);
-    k_anchors<true><<<warps_grid(n), 32 * WARPS_PER_BLOCK, 0, st>>>(
-        ix, ws.off.p, n, total, ws.qr_hash.p, ws.qr_start.p, ws.qr_end.p, ws.hit_pos.p, ws.hit_info.p, ws.n_hits.p,
-        ws.orient.p, ws.hit_anchors.p, nullptr, ws.seg_off.p, ws.anchors.p, ap, ws.details.p);
-    kt->end(st);
-    launches++;
     if (n_list[1]) {
         // orientations with more than CHAIN_SORT_SMALL anchors; k_chain4 sorts the rest
         size_t tmp = 0;
@@ -2451,7 +2484,7 @@ uint32_t run_nam_pipeline(const DevIndex& ix, const DevRefs& refs, const NamConf
         const cudaStream_t sl = ws.side.fork(st);
         SA_CUDA(cudaMemsetAsync(ws.chain_big.p, 0, 4, sl));
         const unsigned pgrid = (unsigned)std::min<uint64_t>(((uint64_t)n_list[2] + 3) / 4, sm_count() * 16);
-        k_chain_long_prep<<<pgrid, 128, 0, sl>>>(ws.off.p, ws.seg_off.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p,
+        k_chain_long_prep<<<pgrid, 128, 0, sl>>>(ws.off.p, ws.seg_off.p, ws.seg_count.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p,
                                                  ws.pred.p, ws.aux.p, total_anchors, ap, cc, long_sorted, n_list[2],
                                                  long_n, long_c, ws.chain_big.p + 2, ws.chain_big.p, lane_max);
         const unsigned bgrid = (unsigned)(sm_count() * 8);
@@ -2466,7 +2499,7 @@ uint32_t run_nam_pipeline(const DevIndex& ix, const DevRefs& refs, const NamConf
     }
     if (n_list[0]) {
         (ring ? k_chain4<true> : k_chain4<false>)<<<chain_grid, 32 * CHAIN_WARPS, 0, st>>>(
-            ws.off.p, n, ws.seg_off.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p,
+            ws.off.p, n, ws.seg_off.p, ws.seg_count.p, ws.anchors_sorted.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p,
             total_anchors, ap, cc, ws.nam_scratch.p, ws.nam_seg_count.p, anc_out, anc_start, short_list, n_list[0]);
         launches++;
     }
