@@ -44,6 +44,44 @@ __device__ __forceinline__ uint8_t read_char(const uint8_t* s, uint32_t L, uint3
     return rc ? c_comp[s[L - 1 - i]] : s[i];
 }
 
+// Ranges of the wave's arena, CIGARs and banded scratch, taken from cursors in the counter
+// block (ALLOC_*, 64 bits each): the order of the ranges does not matter, so no scan has to
+// run between the sizes and the kernels that use them.  A wave of a few dozen jobs is bound by
+// launches and synchronisations, not by its kernels: with scans, five synchronisations and a
+// wide pass that mostly found nothing to do it took 0.55 ms, and now waits three times; mapping
+// 8 pairs went from 0.74 to 0.60 ms, 2000 pairs from 4.29 to 3.94 ms.
+constexpr int ALLOC_ARENA = 32, ALLOC_CIGAR = 34, ALLOC_H = 36, N_SSW = 38, ALLOC_USED = 40, N_COUNTERS = 48;
+
+__device__ __forceinline__ unsigned long long* cursor64(uint32_t* counters, int at) {
+    return reinterpret_cast<unsigned long long*>(counters + at);
+}
+
+// the start of this lane's range of `size` (whole warp, one addition per warp)
+__device__ __forceinline__ uint64_t warp_alloc(unsigned long long* cursor, uint64_t size) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint64_t incl = size;
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint64_t y = __shfl_up_sync(FULLM, (unsigned long long)incl, d);
+        if (lane >= d) incl += y;
+    }
+    unsigned long long base = 0;
+    if (lane == 31 && incl) base = atomicAdd(cursor, (unsigned long long)incl);
+    return __shfl_sync(FULLM, base, 31) + incl - size;
+}
+
+struct TaskSizes {
+    uint64_t arena, cigar, h;
+};
+__device__ __forceinline__ TaskSizes task_sizes(uint32_t type, uint32_t L, uint32_t wlen) {
+    if (type == 1) return {0, (uint64_t)L + 1, 0};
+    // piecewise: every op consumes a query or reference base
+    if (type == 3) return {(uint64_t)L + wlen, (uint64_t)L + wlen + 8, 0};
+    // SSW; the scratch: the literal pass's three rows; k_band_small's words of three widths,
+    // maxima and CIGAR
+    if (type == 2) return {(uint64_t)L + wlen, 2ull * L + wlen + 4, 8ull * (L > wlen ? L : wlen) + 24};
+    return {0, 0, 0};
+}
+
 // has_shared_substring (src/mapper.rs:1157-1168), warp per rescue job: the
 // window's substrings of length 2k/3 go into a shared-memory hash set (2-bit
 // codes, the window read straight from the packed reference), then every read
@@ -60,8 +98,7 @@ __device__ __forceinline__ uint32_t rescue_slot(uint64_t v, uint32_t bits) {
 __global__ void __launch_bounds__(64) k_rescue_filter(const uint32_t* __restrict__ list,
                                                       const uint32_t* __restrict__ n_list,
                                                       const uint8_t* __restrict__ seq, const uint64_t* __restrict__ off,
-                                                      DevRefs R, uint32_t k, PrepRec* prep, uint64_t* sz_arena,
-                                                      uint64_t* sz_cigar, uint64_t* sz_h) {
+                                                      DevRefs R, uint32_t k, PrepRec* prep, uint32_t* counters) {
     extern __shared__ unsigned long long rescue_tab[];
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x & 31, wpb = blockDim.x / 32;
     unsigned long long* tab = rescue_tab + warp * RESCUE_TAB_MAX;
@@ -126,12 +163,17 @@ __global__ void __launch_bounds__(64) k_rescue_filter(const uint32_t* __restrict
             found = __any_sync(FULLM, hit);
             __syncwarp();
         }
-        if (!found && lane == 0) {
-            prep[t].type = 0;
-            prep[t].cigar_cap = 0;
-            sz_arena[t] = 0;
-            sz_cigar[t] = 0;
-            sz_h[t] = 0;
+        if (lane == 0) {
+            if (found) {
+                const TaskSizes z = task_sizes(2, L, p.wlen);
+                prep[t].cigar_cap = (uint32_t)z.cigar;
+                prep[t].arena_off = atomicAdd(cursor64(counters, ALLOC_ARENA), (unsigned long long)z.arena);
+                prep[t].cigar_off = atomicAdd(cursor64(counters, ALLOC_CIGAR), (unsigned long long)z.cigar);
+                prep[t].h_off = atomicAdd(cursor64(counters, ALLOC_H), (unsigned long long)z.h);
+                atomicAdd(&counters[N_SSW], 1u);
+            } else {
+                prep[t].type = 0;
+            }
         }
     }
 }
@@ -176,11 +218,13 @@ __device__ __forceinline__ uint32_t hamming_distance(const DevRefs& R, const uin
 // Thread per job; the reference bases come 32 at a time from the packed words
 __global__ void k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restrict__ seq,
                           const uint64_t* __restrict__ off, DevRefs R, uint32_t k, const uint8_t* raw_refs,
-                          const uint64_t* raw_off, ExtResult* res, PrepRec* prep, uint64_t* sz_arena,
-                          uint64_t* sz_cigar, uint64_t* sz_h, uint32_t* rescue_list, uint32_t* n_rescue,
-                          uint32_t* max_pw_window) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        ExtJob jb = jobs[t];
+                          const uint64_t* raw_off, ExtResult* res, PrepRec* prep, uint32_t* rescue_list,
+                          uint32_t* n_rescue, uint32_t* max_pw_window, uint32_t* counters) {
+    const uint32_t lane = threadIdx.x & 31;
+    // whole warps: the ranges are taken a warp at a time
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t - lane < n; t += gridDim.x * blockDim.x) {
+        const bool in = t < n;
+        ExtJob jb = jobs[in ? t : n - 1];
         const uint8_t* s = seq + off[jb.read];
         const uint32_t L = (uint32_t)(off[jb.read + 1] - off[jb.read]);
         ExtResult r{};
@@ -248,7 +292,7 @@ __global__ void k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restr
                     p.wstart = ds;
                     p.wlen = de > ds ? (uint32_t)(de - ds) : 0;
                     p.type = (cons && jb.anc_n > 0 && L > 0) ? 3 : 0;
-                    if (p.type == 3) atomicMax(max_pw_window, p.wlen);
+                    if (p.type == 3 && in) atomicMax(max_pw_window, p.wlen);
                 }
             }
         } else if (jb.kind == JOB_RESCUE) {
@@ -260,32 +304,26 @@ __global__ void k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restr
             p.wlen = jb.ref_end - jb.ref_start;
             // extended only if has_shared_substring holds (k_rescue_filter)
             p.type = (p.wlen <= 2000 && L > 0) ? 2 : 0;
-            if (p.type == 2) rescue_list[atomicAdd(n_rescue, 1u)] = t;
+            if (p.type == 2 && in) rescue_list[atomicAdd(n_rescue, 1u)] = t;
         } else {  // JOB_ALIGN: raw reference bytes
             p.rc = 0;
             p.wstart = 0;
             p.wlen = (uint32_t)(raw_off[jb.ref_id + 1] - raw_off[jb.ref_id]);
             p.type = (p.wlen <= 2000 && L > 0) ? 2 : 0;
         }
-        uint64_t ab = 0, cap = 0, hs = 0;
-        if (p.type == 1) cap = L + 1;
-        if (p.type == 3) {
-            ab = (uint64_t)L + p.wlen;
-            cap = (uint64_t)L + p.wlen + 8;  // every op consumes a query or reference base
+        // a rescue job's ranges come from k_rescue_filter, if it is kept
+        const bool rescue = jb.kind == JOB_RESCUE;
+        const TaskSizes z = in && !rescue ? task_sizes(p.type, L, p.wlen) : TaskSizes{0, 0, 0};
+        p.cigar_cap = (uint32_t)z.cigar;
+        p.arena_off = warp_alloc(cursor64(counters, ALLOC_ARENA), z.arena);
+        p.cigar_off = warp_alloc(cursor64(counters, ALLOC_CIGAR), z.cigar);
+        p.h_off = warp_alloc(cursor64(counters, ALLOC_H), z.h);
+        const uint32_t ssw = __ballot_sync(FULLM, in && !rescue && p.type == 2);
+        if (lane == 0 && ssw) atomicAdd(&counters[N_SSW], (uint32_t)__popc(ssw));
+        if (in) {
+            res[t] = r;
+            prep[t] = p;
         }
-        if (p.type == 2) {
-            ab = (uint64_t)L + p.wlen;
-            cap = 2ull * L + p.wlen + 4;
-            uint64_t len = L > p.wlen ? L : p.wlen;
-            // the literal pass's three rows; k_band_small's words of three widths, maxima, CIGAR
-            hs = 8 * len + 24;
-        }
-        p.cigar_cap = (uint32_t)cap;
-        res[t] = r;
-        prep[t] = p;
-        sz_arena[t] = ab;
-        sz_cigar[t] = cap;
-        sz_h[t] = hs;
     }
 }
 
@@ -387,15 +425,10 @@ __device__ __forceinline__ uint32_t hamming_cigar_bits(const uint32_t* bits, uin
 // k_copy.
 __global__ void __launch_bounds__(256) k_fill(const ExtJob* jobs, uint32_t n, const uint8_t* __restrict__ seq,
                                               const uint64_t* __restrict__ off, DevRefs R, AlignScores sc,
-                                              PrepRec* prep, const uint64_t* off_arena, const uint64_t* off_cigar,
-                                              const uint64_t* off_h, uint32_t* cigar, ExtResult* res, SswTask* tasks,
+                                              const PrepRec* prep, uint32_t* cigar, ExtResult* res, SswTask* tasks,
                                               uint32_t* counters, uint32_t* pw_list) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        PrepRec p = prep[t];
-        p.arena_off = off_arena[t];
-        p.cigar_off = off_cigar[t];
-        p.h_off = off_h[t];
-        prep[t] = p;
+        const PrepRec p = prep[t];
         if (p.type == 1) {
             const uint8_t* s = seq + off[p.read];
             const uint32_t L = p.qlen;
@@ -2560,19 +2593,23 @@ __device__ __forceinline__ uint32_t warp_eq_runs(const uint8_t* q, const uint8_t
     return mm;
 }
 
+// With list: the tasks list[0 .. *n_tasks_ptr); without: all of them, but for those whose
+// traceback is still to come (pending: k_band_width_wide's).
 __global__ void __launch_bounds__(128) k_finalize(const SswTask* tasks, const uint32_t* n_tasks_ptr,
-                                                  const PrepRec* prep, const uint8_t* arena, const uint64_t* raw_off,
-                                                  const uint32_t* raw, const int32_t* hscratch, AlignScores sc,
-                                                  uint32_t* cigar, ExtResult* res) {
+                                                  const uint32_t* list, bool pending, const PrepRec* prep,
+                                                  const uint8_t* arena, const uint64_t* raw_off, const uint32_t* raw,
+                                                  const int32_t* hscratch, AlignScores sc, uint32_t* cigar,
+                                                  ExtResult* res) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t n = *n_tasks_ptr;
     const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
-    for (uint32_t ti = (blockIdx.x * blockDim.x + threadIdx.x) / 32; ti < n; ti += nwarps) {
+    for (uint32_t x = (blockIdx.x * blockDim.x + threadIdx.x) / 32; x < n; x += nwarps) {
+        const uint32_t ti = list ? list[x] : x;
         const SswTask tk = tasks[ti];
         const PrepRec p = prep[tk.job];
         ExtResult r = res[tk.job];
         r.valid = 0;
-        if (tk.ref_begin1 < 0 || tk.read_begin1 < 0 || tk.flag != 0) {
+        if (tk.ref_begin1 < 0 || tk.read_begin1 < 0 || tk.flag != 0 || (pending && tk.raw_off == RAW_FALLBACK)) {
             if (lane == 0) res[tk.job] = r;
             continue;
         }
@@ -3075,21 +3112,27 @@ __global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ l
     }
 }
 
-__global__ void k_cigar_used(const ExtResult* res, uint32_t n, uint64_t* used) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x)
-        used[t] = res[t].valid ? res[t].cigar_len : 0;
+// each valid job's place in the compact CIGAR array
+__global__ void k_cigar_used(const ExtResult* res, uint32_t n, uint64_t* at, uint32_t* counters) {
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t - lane < n; t += gridDim.x * blockDim.x) {
+        const uint64_t o = warp_alloc(cursor64(counters, ALLOC_USED), t < n && res[t].valid ? res[t].cigar_len : 0);
+        if (t < n) at[t] = o;
+    }
 }
 
-// copy each valid job's CIGAR into a compact array and point the result at it
-__global__ void k_cigar_gather(ExtResult* res, uint32_t n, const uint32_t* cigar, const uint64_t* off,
+// copy each valid job's CIGAR into the compact array and point the result at it, four
+// lanes a job
+__global__ void k_cigar_gather(ExtResult* res, uint32_t n, const uint32_t* cigar, const uint64_t* at,
                                uint32_t* compact) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        ExtResult r = res[t];
-        if (!r.valid) continue;
-        const uint64_t o = off[t];
-        for (uint32_t i = 0; i < r.cigar_len; i++) compact[o + i] = cigar[r.cigar_offset + i];
-        r.cigar_offset = (uint32_t)o;
-        res[t] = r;
+    const uint32_t sub = threadIdx.x & 3;
+    for (uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / 4; t < n; t += gridDim.x * blockDim.x / 4) {
+        if (!res[t].valid) continue;
+        const uint64_t o = at[t];
+        const uint32_t len = res[t].cigar_len, from = res[t].cigar_offset;
+        for (uint32_t i = sub; i < len; i += 4) compact[o + i] = cigar[from + i];
+        __syncwarp(0xfu << (threadIdx.x & 28));
+        if (sub == 0) res[t].cigar_offset = (uint32_t)o;
     }
 }
 
@@ -3239,22 +3282,18 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
     uint32_t launches = 0;
     ws.results.reserve(n);
     ws.prep.reserve(n);
-    ws.sizes.reserve(3 * ((size_t)n + 1));
-    ws.offs.reserve(3 * ((size_t)n + 1));
-    ws.counters.reserve(32);
+    ws.offs.reserve((size_t)n + 1);
+    ws.counters.reserve(N_COUNTERS);
     if (n == 0) {
         ws.h_results.clear();
         ws.h_cigar.clear();
         return 0;
     }
-    uint64_t* sz[3] = {ws.sizes.p, ws.sizes.p + n + 1, ws.sizes.p + 2 * ((size_t)n + 1)};
-    uint64_t* of[3] = {ws.offs.p, ws.offs.p + n + 1, ws.offs.p + 2 * ((size_t)n + 1)};
-    SA_CUDA(cudaMemsetAsync(ws.counters.p, 0, 32 * sizeof(uint32_t), st));
+    SA_CUDA(cudaMemsetAsync(ws.counters.p, 0, N_COUNTERS * sizeof(uint32_t), st));
     kt->begin(KS_PREPARE, st);
     ws.rescue_list.reserve(n);
     k_prepare<<<grid1(n), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, k, raw_refs, raw_off, ws.results.p, ws.prep.p,
-                                        sz[0], sz[1], sz[2], ws.rescue_list.p, ws.counters.p + 4,
-                                        ws.counters.p + 20);
+                                        ws.rescue_list.p, ws.counters.p + 4, ws.counters.p + 20, ws.counters.p);
     {
         static bool attr = false;
         const size_t smem = 2 * RESCUE_TAB_MAX * sizeof(unsigned long long);
@@ -3265,37 +3304,35 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
         uint64_t blocks = ((uint64_t)n + 1) / 2;
         if (blocks > sm_count() * 3) blocks = sm_count() * 3;
         k_rescue_filter<<<(unsigned)(blocks ? blocks : 1), 64, smem, st>>>(ws.rescue_list.p, ws.counters.p + 4, seq,
-                                                                           off, refs, k, ws.prep.p, sz[0], sz[1],
-                                                                           sz[2]);
+                                                                           off, refs, k, ws.prep.p, ws.counters.p);
     }
     kt->end(st);
     launches += 2;
-    // exclusive scans of arena bytes, CIGAR capacity and banded-DP scratch per job
-    uint64_t tot[3];
-    for (int c = 0; c < 3; c++) {
-        SA_CUDA(cudaMemsetAsync(sz[c] + n, 0, 8, st));
-        excl_sum(ws, sz[c], of[c], (uint64_t)n + 1, st);
-        SA_CUDA(cudaMemcpyAsync(&tot[c], of[c] + n, 8, cudaMemcpyDeviceToHost, st));
-    }
-    uint32_t max_pw_window = 0;
-    SA_CUDA(cudaMemcpyAsync(&max_pw_window, ws.counters.p + 20, 4, cudaMemcpyDeviceToHost, st));
-    launches += 3;
+    // what the ranges take, and the tasks that there will be
+    uint32_t hc[N_COUNTERS];
+    SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
     SA_CUDA(cudaStreamSynchronize(st));
-    ws.arena.reserve(tot[0] + 16);
-    ws.cigar.reserve(tot[1] + 1);
-    ws.hscratch.reserve(tot[2] + 1);
+    auto total_of = [&](int at) { return (uint64_t)hc[at] | (uint64_t)hc[at + 1] << 32; };
+    const uint32_t n_tasks = hc[N_SSW], max_pw_window = hc[20];
+    ws.arena.reserve(total_of(ALLOC_ARENA) + 16);
+    ws.cigar.reserve(total_of(ALLOC_CIGAR) + 1);
+    ws.hscratch.reserve(total_of(ALLOC_H) + 1);
     ws.tasks.reserve(n);
     ws.list_word.reserve(n);
     ws.list_rev_byte.reserve(n);
     ws.list_rev_word.reserve(n);
     kt->begin(KS_FILL, st);
     ws.pw_list.reserve(n);
-    k_fill<<<grid1(n), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, sc, ws.prep.p, of[0], of[1], of[2], ws.cigar.p,
-                                     ws.results.p, ws.tasks.p, ws.counters.p, ws.pw_list.p);
-    k_copy<<<grid1((uint64_t)n * 32), 256, 0, st>>>(ws.jobs.p, seq, off, refs, raw_refs, raw_off, ws.prep.p,
-                                                    ws.arena.p, ws.tasks.p, ws.pw_list.p, ws.counters.p);
+    k_fill<<<grid1(n), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, sc, ws.prep.p, ws.cigar.p, ws.results.p, ws.tasks.p,
+                                     ws.counters.p, ws.pw_list.p);
+    launches++;
+    if (n_tasks || max_pw_window) {
+        const uint64_t copies = max_pw_window ? n : n_tasks;
+        k_copy<<<grid1(copies * 32), 256, 0, st>>>(ws.jobs.p, seq, off, refs, raw_refs, raw_off, ws.prep.p, ws.arena.p,
+                                                   ws.tasks.p, ws.pw_list.p, ws.counters.p);
+        launches++;
+    }
     kt->end(st);
-    launches += 2;
     if (max_pw_window) {
         // single-end piecewise jobs: a warp per job, each warp with its own DP scratch
         if (!anchors) throw Error(SA_ERR_INVALID, "internal: piecewise jobs without anchors");
@@ -3323,10 +3360,33 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
         kt->end(st);
         launches++;
     }
-    uint32_t cnt[4];
-    SA_CUDA(cudaMemcpyAsync(cnt, ws.counters.p, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    SA_CUDA(cudaStreamSynchronize(st));
-    const uint32_t n_tasks = cnt[0];
+    const bool wide = sc.gap_open >= sc.gap_extend;
+    // directions and CIGARs of the tasks that dir_size / raw_size give sizes for
+    auto wide_scratch = [&]() {
+        ws.dir_off.reserve((size_t)n_tasks + 1);
+        ws.raw_off.reserve((size_t)n_tasks + 1);
+        SA_CUDA(cudaMemsetAsync(ws.dir_size.p + n_tasks, 0, 8, st));
+        SA_CUDA(cudaMemsetAsync(ws.raw_size.p + n_tasks, 0, 8, st));
+        excl_sum(ws, ws.dir_size.p, ws.dir_off.p, (uint64_t)n_tasks + 1, st);
+        excl_sum(ws, ws.raw_size.p, ws.raw_off.p, (uint64_t)n_tasks + 1, st);
+        uint64_t dtot = 0, rtot = 0;
+        SA_CUDA(cudaMemcpyAsync(&dtot, ws.dir_off.p + n_tasks, 8, cudaMemcpyDeviceToHost, st));
+        SA_CUDA(cudaMemcpyAsync(&rtot, ws.raw_off.p + n_tasks, 8, cudaMemcpyDeviceToHost, st));
+        SA_CUDA(cudaStreamSynchronize(st));
+        ws.dir.reserve(dtot + 16);
+        ws.raw.reserve(rtot + 1);
+        SA_CUDA(cudaMemsetAsync(ws.dir.p, 0, dtot + 16, st));
+        launches += 2;
+    };
+    auto finalize = [&](const uint32_t* n_ptr, uint32_t n_max, const uint32_t* list, bool pending) {
+        kt->begin(KS_FINALIZE, st);
+        // a warp per task
+        k_finalize<<<grid1((uint64_t)n_max * 32, 128), 128, 0, st>>>(ws.tasks.p, n_ptr, list, pending, ws.prep.p,
+                                                                     ws.arena.p, ws.raw_off.p, ws.raw.p, ws.hscratch.p,
+                                                                     sc, ws.cigar.p, ws.results.p);
+        kt->end(st);
+        launches++;
+    };
     const int bias = sc.mismatch;  // |min(matrix)| for the match/mismatch matrix (ext/ssw/ssw.c:802-806)
     if (n_tasks) {
         const int seg_b = ((int)max_qlen + 15) / 16, seg_w = ((int)max_qlen + 7) / 8;
@@ -3481,87 +3541,73 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
             kt->end(st);
             launches++;
         }
-        ws.dir_size.reserve((size_t)n_tasks + 1);
-        ws.dir_off.reserve((size_t)n_tasks + 1);
-        ws.raw_size.reserve((size_t)n_tasks + 1);
-        ws.raw_off.reserve((size_t)n_tasks + 1);
-        const bool wide = sc.gap_open >= sc.gap_extend;
-        const int maxc = 2 * (int)std::max<uint32_t>(2048, max_qlen) + 8;
-        const size_t band_smem = (size_t)4 * maxc * sizeof(int);
-        unsigned band_blocks = (unsigned)std::min<uint64_t>(n_tasks, sm_count() * 3);
-        if (!band_blocks) band_blocks = 1;
-        kt->begin(KS_BAND, st);
-        if (wide) {
-            static int attr_smem = 0;
-            if ((int)band_smem > attr_smem) {
-                SA_CUDA(cudaFuncSetAttribute(k_band_width_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)band_smem));
-                SA_CUDA(cudaFuncSetAttribute(k_band_trace_wide, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)band_smem));
-                attr_smem = (int)band_smem;
-            }
-            SA_CUDA(cudaMemsetAsync(ws.dir_size.p, 0, (size_t)n_tasks * 8, st));
-            SA_CUDA(cudaMemsetAsync(ws.raw_size.p, 0, (size_t)n_tasks * 8, st));
-            k_band_width_wide<<<band_blocks, 32, band_smem, st>>>(ws.tasks.p, ws.counters.p + 29, ws.wide_list.p,
-                                                                 ws.prep.p, ws.arena.p, sc, maxc, ws.dir_size.p,
-                                                                 ws.raw_size.p, ws.counters.p);
-        } else {
+        if (!wide) {
+            // the literal passes, a thread per task
+            ws.dir_size.reserve((size_t)n_tasks + 1);
+            ws.raw_size.reserve((size_t)n_tasks + 1);
+            kt->begin(KS_BAND, st);
             k_band_width<<<grid1(n_tasks, 128), 128, 0, st>>>(ws.tasks.p, ws.counters.p, ws.prep.p, ws.arena.p,
                                                               ws.hscratch.p, sc, ws.dir_size.p, ws.raw_size.p);
-        }
-        kt->end(st);
-        launches++;
-        SA_CUDA(cudaMemsetAsync(ws.dir_size.p + n_tasks, 0, 8, st));
-        SA_CUDA(cudaMemsetAsync(ws.raw_size.p + n_tasks, 0, 8, st));
-        excl_sum(ws, ws.dir_size.p, ws.dir_off.p, (uint64_t)n_tasks + 1, st);
-        excl_sum(ws, ws.raw_size.p, ws.raw_off.p, (uint64_t)n_tasks + 1, st);
-        launches += 2;
-        uint64_t dtot = 0, rtot = 0;
-        SA_CUDA(cudaMemcpyAsync(&dtot, ws.dir_off.p + n_tasks, 8, cudaMemcpyDeviceToHost, st));
-        SA_CUDA(cudaMemcpyAsync(&rtot, ws.raw_off.p + n_tasks, 8, cudaMemcpyDeviceToHost, st));
-        SA_CUDA(cudaStreamSynchronize(st));
-        ws.dir.reserve(dtot + 16);
-        ws.raw.reserve(rtot + 1);
-        SA_CUDA(cudaMemsetAsync(ws.dir.p, 0, dtot + 16, st));
-        kt->begin(KS_BAND, st);
-        if (wide)
-            k_band_trace_wide<<<band_blocks, 32, band_smem, st>>>(ws.tasks.p, ws.counters.p + 29, ws.wide_list.p,
-                                                                 ws.prep.p, ws.arena.p, sc, maxc, ws.dir_off.p,
-                                                                 ws.dir.p, ws.raw_off.p, ws.raw.p, ws.counters.p);
-        else
+            kt->end(st);
+            launches++;
+            wide_scratch();
+            kt->begin(KS_BAND, st);
             k_band_trace_literal<<<grid1(n_tasks, 128), 128, 0, st>>>(ws.tasks.p, ws.counters.p, ws.prep.p, ws.arena.p,
-                                                              ws.hscratch.p, sc, ws.dir_off.p, ws.dir.p, ws.raw_off.p,
-                                                              ws.raw.p);
-        kt->end(st);
-        kt->begin(KS_FINALIZE, st);
-        // a warp per task
-        k_finalize<<<grid1((uint64_t)n_tasks * 32, 128), 128, 0, st>>>(ws.tasks.p, ws.counters.p, ws.prep.p, ws.arena.p,
-                                                        ws.raw_off.p, ws.raw.p, ws.hscratch.p, sc, ws.cigar.p,
-                                                        ws.results.p);
-        kt->end(st);
-        launches += 2;
+                                                                      ws.hscratch.p, sc, ws.dir_off.p, ws.dir.p,
+                                                                      ws.raw_off.p, ws.raw.p);
+            kt->end(st);
+            launches++;
+        }
+        finalize(ws.counters.p, n_tasks, nullptr, wide);
     }
-    // compact the CIGARs that were written and copy back results + used ops only
-    k_cigar_used<<<grid1(n), 256, 0, st>>>(ws.results.p, n, sz[0]);
-    SA_CUDA(cudaMemsetAsync(sz[0] + n, 0, 8, st));
-    excl_sum(ws, sz[0], of[0], (uint64_t)n + 1, st);
-    uint64_t used = 0;
-    SA_CUDA(cudaMemcpyAsync(&used, of[0] + n, 8, cudaMemcpyDeviceToHost, st));
+    // the CIGARs' places in the compact array; then the tasks whose band outgrew a warp, if
+    // there are any, and the places again
+    ws.offs.reserve(n);
+    k_cigar_used<<<grid1(n), 256, 0, st>>>(ws.results.p, n, ws.offs.p, ws.counters.p);
+    launches++;
+    SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
     SA_CUDA(cudaStreamSynchronize(st));
+    if (const uint32_t n_wide = hc[29]) {
+        const int maxc = 2 * (int)std::max<uint32_t>(2048, max_qlen) + 8;
+        const size_t band_smem = (size_t)4 * maxc * sizeof(int);
+        const unsigned band_blocks = (unsigned)std::min<uint64_t>(n_wide, sm_count() * 3);
+        SA_CUDA(cudaFuncSetAttribute(k_band_width_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)band_smem));
+        SA_CUDA(cudaFuncSetAttribute(k_band_trace_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)band_smem));
+        ws.dir_size.reserve((size_t)n_tasks + 1);
+        ws.raw_size.reserve((size_t)n_tasks + 1);
+        kt->begin(KS_BAND, st);
+        SA_CUDA(cudaMemsetAsync(ws.dir_size.p, 0, (size_t)n_tasks * 8, st));
+        SA_CUDA(cudaMemsetAsync(ws.raw_size.p, 0, (size_t)n_tasks * 8, st));
+        k_band_width_wide<<<band_blocks, 32, band_smem, st>>>(ws.tasks.p, ws.counters.p + 29, ws.wide_list.p, ws.prep.p,
+                                                             ws.arena.p, sc, maxc, ws.dir_size.p, ws.raw_size.p,
+                                                             ws.counters.p);
+        kt->end(st);
+        wide_scratch();
+        kt->begin(KS_BAND, st);
+        k_band_trace_wide<<<band_blocks, 32, band_smem, st>>>(ws.tasks.p, ws.counters.p + 29, ws.wide_list.p, ws.prep.p,
+                                                             ws.arena.p, sc, maxc, ws.dir_off.p, ws.dir.p,
+                                                             ws.raw_off.p, ws.raw.p, ws.counters.p);
+        kt->end(st);
+        finalize(ws.counters.p + 29, n_wide, ws.wide_list.p, false);
+        SA_CUDA(cudaMemsetAsync(ws.counters.p + ALLOC_USED, 0, 8, st));
+        k_cigar_used<<<grid1(n), 256, 0, st>>>(ws.results.p, n, ws.offs.p, ws.counters.p);
+        launches += 3;
+        SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
+        SA_CUDA(cudaStreamSynchronize(st));
+    }
+    const uint64_t used = total_of(ALLOC_USED);
     ws.raw.reserve(std::max<uint64_t>(used, 1));  // reused as the compact CIGAR buffer
-    k_cigar_gather<<<grid1(n), 256, 0, st>>>(ws.results.p, n, ws.cigar.p, of[0], ws.raw.p);
-    launches += 3;
+    k_cigar_gather<<<grid1((uint64_t)n * 4), 256, 0, st>>>(ws.results.p, n, ws.cigar.p, ws.offs.p, ws.raw.p);
+    launches++;
     SA_CUDA(cudaGetLastError());
     ws.h_results.resize(n);
     ws.h_cigar.resize(used);
     SA_CUDA(cudaMemcpyAsync(ws.h_results.data(), ws.results.p, (size_t)n * sizeof(ExtResult), cudaMemcpyDeviceToHost,
                             st));
     if (used) SA_CUDA(cudaMemcpyAsync(ws.h_cigar.data(), ws.raw.p, used * 4, cudaMemcpyDeviceToHost, st));
-    SA_CUDA(cudaMemcpyAsync(ws.cells, ws.counters.p + 8, 5 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
-    SA_CUDA(cudaMemcpyAsync(ws.cells + 5, ws.counters.p + 24, 2 * sizeof(uint64_t), cudaMemcpyDeviceToHost, st));
     SA_CUDA(cudaStreamSynchronize(st));
-    tot[1] = used;
-    ws.total_cigar = tot[1];
+    for (int c = 0; c < 7; c++) ws.cells[c] = total_of(c < 5 ? 8 + 2 * c : 24 + 2 * (c - 5));
+    ws.total_cigar = used;
     return launches;
 }
 

@@ -47,15 +47,18 @@ struct ExtWorkspace {
     DevBuf<ExtJob> jobs;
     DevBuf<ExtResult> results;
     DevBuf<PrepRec> prep;
-    DevBuf<uint64_t> sizes;     // 3 per job: arena bytes, cigar ops, h ints
-    DevBuf<uint64_t> offs;      // 3 per job (+3)
+    DevBuf<uint64_t> offs;      // per job: its CIGAR's place in the compact array
     DevBuf<uint8_t> arena;
     DevBuf<uint32_t> cigar;
     DevBuf<int32_t> hscratch;
     DevBuf<SswTask> tasks;
     DevBuf<uint32_t> band_list, wide_list;  // tasks left by k_band_small / by k_band_warp
     DevBuf<uint32_t> band_buckets;          // tasks by starting band width, then the counts
-    DevBuf<uint32_t> counters;  // [0] n_tasks [1] n_word [2] n_rev_byte [3] n_rev_word [4] n_rescue, [5]-[7] [18] [21]-[23] [30] task queues, [19] n_piecewise, [20] widest piecewise window, [31] n_redo, u64 cells at [8], u64 band cells at [24], band list sizes at [28] and [29]
+    // [0] n_tasks [1] n_word [2] n_rev_byte [3] n_rev_word [4] n_rescue, [5]-[7] [18] [21]-[23]
+    // [30] task queues, u64 cells at [8], [19] n_piecewise, [20] widest piecewise window, u64
+    // band cells at [24], band list sizes at [28] and [29], [31] n_redo, then the wave's
+    // u64 range cursors and its task count (ALLOC_*, N_SSW in extend.cu)
+    DevBuf<uint32_t> counters;
     DevBuf<uint32_t> rescue_list;
     DevBuf<uint32_t> list_word, list_rev_byte, list_rev_word;
     DevBuf<uint32_t> order;  // task order of the fused SSW kernel
