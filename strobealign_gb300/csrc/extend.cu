@@ -2713,13 +2713,20 @@ __global__ void __launch_bounds__(128) k_finalize(const SswTask* tasks, const ui
 // piecewise unit vectors agree with.  Beyond those vectors and the goldens this path is
 // parity-unpinned.
 //
-// A piece's DP runs row by row on the warp, the columns in chunks of 32 lanes: F and
-// the diagonal come from the previous row (shared memory), and the row's E chain
-// E(j) = max(H(j-1) - gO, E(j-1) - gE) is a max-plus scan of max(diag, F) - gO over the
-// lanes (exact for gap_open >= gap_extend, since H(j-1) = max(that, E(j-1))).  Each cell
-// keeps four direction bits for the traceback.
+// A piece's DP is a wavefront: a lane owns R query rows of a strip of 32 R, lane l is l columns
+// behind lane 0, and a step takes the row above's H and F from the lane above by two shuffles.
+// The strip's last row goes to the next strip through the row buffer (shared memory).  What
+// bounds it is the instructions issued, with 28 warps per SM: a step is about 30 for one cell a
+// lane, 45 for two, against about 90 for 32 columns of a row when the warp ran along the rows
+// (the row's E chain as a scan, the best cell by a reduction per row).  One row a lane up to 32
+// query bases, two beyond: a step of two costs half as much again, and halves the lanes that a
+// short piece keeps busy.  With that, the 32-wide traceback and the anchors of a chain looked
+// at 32 at a time, a wave of 14500 reads of 50..500 nt takes 0.3 ms instead of 0.9.  E takes max(diagonal, F) where H would do: the same for
+// gap_open >= gap_extend.  Each cell keeps four direction bits, stored by wavefront so that a
+// step's are contiguous; the traceback looks at 32 of them at a time, along the diagonal or the
+// gap.
 constexpr int PW_NEG = -(1 << 28);
-constexpr uint8_t PW_DIAG = 1, PW_FROM_E = 2, PW_EEXT = 4, PW_FEXT = 8, PW_FROM_F = 16;
+constexpr uint8_t PW_FROM_E = 2, PW_EEXT = 4, PW_FEXT = 8, PW_FROM_F = 16;
 
 struct PwPiece {
     int score;
@@ -2727,160 +2734,206 @@ struct PwPiece {
     int nops;    // traceback ops, last op first (OP codes of src/cigar.rs)
 };
 
-// q: n query bytes, r: m reference bytes (REV: both read backwards).  LOCAL: best cell
-// (strict >, row-major, from 0) with the end bonus on the last query row; otherwise the
-// end is (n, m).  ops receives the traceback from the end cell back to (0, 0).
-template <bool LOCAL, bool REV>
-__device__ PwPiece pw_dp(const uint8_t* q, int n, const uint8_t* r, int m, const AlignScores& sc, int* rowbuf,
-                         uint8_t* dirs, uint8_t* ops) {
+// bytes of direction bits of a piece of n query and m reference bases (grows with both)
+__host__ __device__ __forceinline__ uint64_t pw_dir_bytes(uint64_t n, uint64_t m) {
+    return (n <= 32 ? 32 : (n + 63) / 64 * 64) * (m + 31);
+}
+
+// q: n query bytes, r: m reference bytes (step -1: both start at their last base and are
+// read backwards).  local: best cell (strict >, row-major, from 0) with the end bonus on the
+// last query row; otherwise the end is (n, m).
+template <int R>
+__device__ __noinline__ PwPiece pw_fill(const uint8_t* q, int n, const uint8_t* r, int m, int step, bool local,
+                                        int match, int mism, int go, int ge, int end_bonus, int2* row,
+                                        uint8_t* dirs) {
     const int lane = threadIdx.x & 31;
-    const int go = sc.gap_open, ge = sc.gap_extend, match = sc.match, mism = sc.mismatch;
-    const int W = m + 1;
-    int* Hp = rowbuf;
-    int* Fp = rowbuf + W;
-    int* Hc = rowbuf + 2 * W;
-    int* Fc = rowbuf + 3 * W;
-    auto qv = [&](int i) { return REV ? q[n - 1 - i] : q[i]; };
-    auto rv = [&](int j) { return REV ? r[m - 1 - j] : r[j]; };
-    for (int j = lane; j <= m; j += 32) {
-        Hp[j] = j == 0 ? 0 : -go - (j - 1) * ge;
-        Fp[j] = PW_NEG;
-        uint8_t d = 0;
-        if (j >= 1) {
-            d |= PW_FROM_E;                        // H(0, j) = E(0, j)
-            if (j >= 2 && go != ge) d |= PW_EEXT;  // E(0, j) extends E(0, j-1), not opened from H
-        }
-        dirs[j] = d;
-    }
+    for (int j = lane; j <= m; j += 32) row[j] = make_int2(j == 0 ? 0 : -go - (j - 1) * ge, PW_NEG);
     __syncwarp();
-    int best = 0, bi = 0, bj = 0;
-    for (int i = 1; i <= n; i++) {
-        const int hcol0 = -go - (i - 1) * ge;  // H(i, 0) = F(i, 0)
-        if (lane == 0) {
-            Hc[0] = hcol0;
-            Fc[0] = hcol0;
-            dirs[(size_t)i * W] = (i >= 2 && go != ge) ? PW_FEXT : 0;
-        }
-        const int qc = qv(i - 1);
-        const int bonus = (LOCAL && i == n) ? (int)sc.end_bonus : 0;
-        int carryT = hcol0 - go, carryE = PW_NEG, carryH = hcol0;
-        for (int c = 0; c * 32 < m; c++) {
-            const int j = 1 + 32 * c + lane;
-            const bool act = j <= m;
-            int F = PW_NEG, D = PW_NEG, B = PW_NEG;
-            bool fext = false;
-            if (act) {
-                const int hu = Hp[j], fu = Fp[j];
-                const int f1 = hu - go, f2 = fu - ge;
-                F = f1 > f2 ? f1 : f2;
-                fext = F == fu - ge && F != hu - go;
-                D = Hp[j - 1] + (qc == rv(j - 1) ? match : -mism) + bonus;
-                B = D > F ? D : F;
-            }
-            int T = act ? B - go : PW_NEG;
+    auto col0 = [&](int i) { return i == 0 ? 0 : -go - (i - 1) * ge; };  // H(i, 0) = F(i, 0)
+    PwPiece res;
+    res.score = res.bi = res.bj = res.nops = 0;
+    for (int base = 0; base < n; base += 32 * R) {
+        const int i0 = base + R * lane + 1;  // this lane's first row
+        const int lanes = n - base >= 32 * R ? 32 : (n - base + R - 1) / R;
+        const int steps = m + lanes - 1;
+        const bool more = base + 32 * R < n;
+        int H[R], B[R], E[R], dg[R], F = PW_NEG, qc[R], eqs[R], nes[R], best[R], bcol[R];
 #pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int Tp = __shfl_up_sync(FULLM, T, d);
-                const int cc = Tp - d * ge;
-                if (lane >= d && cc > T) T = cc;
-            }
-            {
-                const int cc = carryT - (lane + 1) * ge;
-                if (cc > T) T = cc;
-            }
-            int E = __shfl_up_sync(FULLM, T, 1);
-            if (lane == 0) E = carryT;
-            const int H = B > E ? B : E;
-            int El = __shfl_up_sync(FULLM, E, 1), Hl = __shfl_up_sync(FULLM, H, 1);
+        for (int x = 0; x < R; x++) {
+            const int i = i0 + x;
+            H[x] = B[x] = col0(i);
+            E[x] = PW_NEG;
+            dg[x] = col0(i - 1);
+            qc[x] = i <= n ? q[(long long)step * (i - 1)] : 0;
+            const int bonus = local && i == n ? end_bonus : 0;
+            eqs[x] = match + bonus;
+            nes[x] = bonus - mism;
+            best[x] = i <= n ? 0 : 0x7fffffff;
+            bcol[x] = 0;
+        }
+        // the columns behind lane 0's: t = column - 1
+        int t = -lane;
+        const unsigned cols = i0 <= n ? (unsigned)m : 0u;
+        bool act = (unsigned)t < cols;
+        const uint8_t* rp = r + (long long)step * t;
+        int rc = act ? *rp : 0;
+        uint8_t* dp = dirs + (size_t)(base / (32 * R)) * (m + 31) * (32 * R) + lane * R;
+        int2 up = row[1 <= m ? 1 : m];
+        for (int s = 0; s < steps; s++) {
+            int hu = __shfl_up_sync(FULLM, H[R - 1], 1), fu = __shfl_up_sync(FULLM, F, 1);
             if (lane == 0) {
-                El = carryE;
-                Hl = carryH;
+                hu = up.x;
+                fu = up.y;
             }
-            const bool eext = E == El - ge && E != Hl - go;
+            up = row[s + 2 <= m ? s + 2 : m];
+            rp += step;
+            const bool nact = (unsigned)(t + 1) < cols;
+            const int rn = nact ? *rp : 0;
             if (act) {
-                uint8_t d = 0;
-                if (H == D) d |= PW_DIAG;
-                if (H == E) d |= PW_FROM_E;
-                if (H == F) d |= PW_FROM_F;
-                if (eext) d |= PW_EEXT;
-                if (fext) d |= PW_FEXT;
-                dirs[(size_t)i * W + j] = d;
-                Hc[j] = H;
-                Fc[j] = F;
-            }
-            if (LOCAL) {
-                int v = act ? H : PW_NEG;
-                for (int d = 16; d > 0; d >>= 1) {
-                    const int o = __shfl_xor_sync(FULLM, v, d);
-                    v = v > o ? v : o;
+                uint32_t dir = 0;
+#pragma unroll
+                for (int x = 0; x < R; x++) {
+                    const int f1 = hu - go, f2 = fu - ge;
+                    F = f1 > f2 ? f1 : f2;
+                    const int D = dg[x] + (qc[x] == rc ? eqs[x] : nes[x]);
+                    dg[x] = hu;
+                    const int e1 = B[x] - go, e2 = E[x] - ge;
+                    const int e = e1 > e2 ? e1 : e2;
+                    const bool eext = e == e2 && e != H[x] - go;
+                    B[x] = D > F ? D : F;
+                    E[x] = e;
+                    H[x] = B[x] > e ? B[x] : e;
+                    uint32_t d = eext ? PW_EEXT : 0;
+                    if (f2 > f1) d |= PW_FEXT;
+                    if (H[x] == e) d |= PW_FROM_E;
+                    if (H[x] == F) d |= PW_FROM_F;
+                    dir |= d << (8 * x);
+                    if (H[x] > best[x]) {
+                        best[x] = H[x];
+                        bcol[x] = t + 1;
+                    }
+                    hu = H[x];
+                    fu = F;
                 }
-                if (v > best) {
-                    const unsigned at = __ballot_sync(FULLM, act && H == v);
-                    best = v;
-                    bi = i;
-                    bj = 1 + 32 * c + (__ffs(at) - 1);
-                }
+                if (R == 1) *dp = (uint8_t)dir;
+                else *reinterpret_cast<uint16_t*>(dp) = (uint16_t)dir;
+                if (more && lane == 31) row[t + 1] = make_int2(H[R - 1], F);
             }
-            carryT = __shfl_sync(FULLM, T, 31);
-            carryE = __shfl_sync(FULLM, E, 31);
-            carryH = __shfl_sync(FULLM, H, 31);
+            dp += 32 * R;
+            t++;
+            act = nact;
+            rc = rn;
+        }
+        if (local) {
+            int bv = best[0], brow = i0, bc = bcol[0];
+            if (R == 2 && best[R - 1] > bv && i0 + 1 <= n) {
+                bv = best[R - 1];
+                brow = i0 + 1;
+                bc = bcol[R - 1];
+            }
+            if (i0 > n) bv = 0;
+            const int top = __reduce_max_sync(FULLM, bv);
+            if (top > res.score) {
+                const int from = __ffs(__ballot_sync(FULLM, bv == top)) - 1;
+                res.score = top;
+                res.bi = __shfl_sync(FULLM, brow, from);
+                res.bj = __shfl_sync(FULLM, bc, from);
+            }
+        } else if (!more) {
+            const int from = (n - 1 - base) / R;
+            const int h0 = __shfl_sync(FULLM, H[0], from), h1 = __shfl_sync(FULLM, H[R - 1], from);
+            res.score = (n - 1 - base) % R ? h1 : h0;
         }
         __syncwarp();
-        int* t = Hp;
-        Hp = Hc;
-        Hc = t;
-        t = Fp;
-        Fp = Fc;
-        Fc = t;
     }
-    if (!LOCAL) {
-        best = Hp[m];
-        bi = n;
-        bj = m;
+    if (!local) {
+        if (n == 0) res.score = col0(m);
+        res.bi = n;
+        res.bj = m;
     }
-    __syncwarp();
-    PwPiece res;
-    res.score = best;
-    res.bi = bi;
-    res.bj = bj;
-    res.nops = 0;
-    if (lane == 0) {
-        int i = bi, j = bj, state = 0, nops = 0;
-        const int limit = 2 * (n + m) + 4;
-        for (int it = 0; (i > 0 || j > 0) && it < limit; it++) {
-            const uint8_t d = dirs[(size_t)i * W + j];
-            if (state == 0) {
-                // a deletion, then an insertion, before the diagonal on ties: a gap
-                // that ties with matches goes to the end of the run (the reference's
-                // extend_piecewise_complex vector, src/piecewisealigner.rs:1672-1710)
-                if (j > 0 && (d & PW_FROM_E)) {
-                    state = 1;
-                } else if (i > 0 && (j == 0 || (d & PW_FROM_F))) {
-                    state = 2;
-                } else {
-                    ops[nops++] = qv(i - 1) == rv(j - 1) ? 7 : 8;  // = / X
-                    i--;
-                    j--;
-                }
-            } else if (state == 1) {
-                ops[nops++] = 2;  // D
-                const bool ext = j > 1 && (d & PW_EEXT);
-                j--;
-                state = ext ? 1 : 0;
-                if (i == 0 && j > 0) state = 1;
-            } else {
-                ops[nops++] = 1;  // I
-                const bool ext = i > 1 && (d & PW_FEXT);
-                i--;
-                state = ext ? 2 : 0;
-                if (j == 0 && i > 0) state = 2;
-            }
+    return res;
+}
+
+// ops receives the traceback from the end cell back to (0, 0)
+template <bool LOCAL, bool REV>
+__device__ __forceinline__ PwPiece pw_dp(const uint8_t* q, int n, const uint8_t* r, int m, const AlignScores& sc,
+                                         int2* row, uint8_t* dirs, uint8_t* ops) {
+    const int lane = threadIdx.x & 31, step = REV ? -1 : 1;
+    const int go = sc.gap_open, ge = sc.gap_extend, match = sc.match, mism = sc.mismatch, bonus = sc.end_bonus;
+    const uint8_t* q0 = REV ? q + (n - 1) : q;
+    const uint8_t* r0 = REV ? r + (m - 1) : r;
+    PwPiece res = n <= 32 ? pw_fill<1>(q0, n, r0, m, step, LOCAL, match, mism, go, ge, bonus, row, dirs)
+                          : pw_fill<2>(q0, n, r0, m, step, LOCAL, match, mism, go, ge, bonus, row, dirs);
+    const int rs = n <= 32 ? 0 : 1;  // log2 of the rows a lane
+    const int strip_bytes = (m + 31) * (32 << rs);
+    auto bits = [&](int i, int j) -> uint32_t {  // i, j >= 1
+        const int x = i - 1, l = (x >> rs) & 31;
+        return dirs[(size_t)(x >> (5 + rs)) * strip_bytes + ((j - 1 + l) << (5 + rs)) + (x & ((32 << rs) - 1))];
+    };
+    int i = res.bi, j = res.bj, nops = 0;
+    while (i > 0 && j > 0) {
+        // a deletion, then an insertion, before the diagonal on ties: a gap that ties with
+        // matches goes to the end of the run (the reference's extend_piecewise_complex
+        // vector, src/piecewisealigner.rs:1672-1710)
+        const bool in = lane < i && lane < j;
+        const uint32_t d = in ? bits(i - lane, j - lane) : 0;
+        const uint32_t stop = __ballot_sync(FULLM, !in || (d & (PW_FROM_E | PW_FROM_F)));
+        const int run = stop ? __ffs(stop) - 1 : 32;
+        if (lane < run)
+            ops[nops + lane] = q0[(long long)step * (i - lane - 1)] == r0[(long long)step * (j - lane - 1)] ? 7 : 8;
+        nops += run;
+        i -= run;
+        j -= run;
+        if (run == 32 || i == 0 || j == 0) continue;
+        const bool del = __shfl_sync(FULLM, d, run) & PW_FROM_E;
+        // the gap goes on to the first cell that opens it (column or row 1 at the latest)
+        for (bool open = false; !open;) {
+            const int left = (del ? j : i) - lane;
+            const bool ext = left > 1 && (bits(del ? i : i - lane, del ? j - lane : j) & (del ? PW_EEXT : PW_FEXT));
+            const uint32_t end = __ballot_sync(FULLM, !ext);
+            open = end != 0;
+            const int len = open ? __ffs(end) : 32;
+            if (lane < len) ops[nops + lane] = del ? 2 : 1;
+            nops += len;
+            if (del) j -= len;
+            else i -= len;
         }
-        res.nops = nops;
     }
-    res.nops = __shfl_sync(FULLM, res.nops, 0);
+    // the rest lies along an edge: deletions in row 0, insertions in column 0
+    for (int x = lane; x < i + j; x += 32) ops[nops + x] = j > 0 ? 2 : 1;
+    res.nops = nops + i + j;
     __syncwarp();
     return res;
+}
+
+// the piece's ops, from its first base on (fwd: ops is a backward piece's, last op first in
+// the piece's direction is the read's first): runs found 32 ops at a time, pushed by lane 0
+__device__ __forceinline__ void pw_push_ops(const uint8_t* ops, int nops, bool fwd, CigarWriter& w) {
+    const int lane = threadIdx.x & 31;
+    for (int c = 0; c < nops; c += 32) {
+        const int x = c + lane, cnt = nops - c < 32 ? nops - c : 32;
+        const uint32_t op = x < nops ? ops[fwd ? x : nops - 1 - x] : 0;
+        const uint32_t before = __shfl_up_sync(FULLM, op, 1);
+        uint32_t heads = __ballot_sync(FULLM, x < nops && (lane == 0 || op != before));
+        while (heads) {
+            const int at = __ffs(heads) - 1;
+            heads &= heads - 1;
+            const uint32_t o = __shfl_sync(FULLM, op, at);
+            if (lane == 0) w.push(o, (uint32_t)((heads ? __ffs(heads) - 1 : cnt) - at));
+        }
+    }
+}
+
+// mismatches, insertions and deletions of a finished CIGAR (lane 0's)
+__device__ __forceinline__ uint32_t pw_edits(const CigarWriter& w) {
+    const uint32_t lane = threadIdx.x & 31, n = __shfl_sync(FULLM, w.n, 0);
+    __syncwarp();
+    uint32_t ed = 0;
+    for (uint32_t x = lane; x < n; x += 32) {
+        const uint32_t op = w.out[x] & 15;
+        if (op == 8 || op == 1 || op == 2) ed += w.out[x] >> 4;
+    }
+    return __reduce_add_sync(FULLM, ed);
 }
 
 // remove_spurious_anchors (src/piecewisealigner.rs:596-719) on anchors held as
@@ -2940,6 +2993,47 @@ __device__ void prune_spurious_anchors(int* anc, int& na) {
     }
 }
 
+// The same by a warp: a chain with an indel beyond the tolerance goes through the serial
+// passes; in all others only the ends are looked at, 32 anchors at a time.
+__device__ __forceinline__ void prune_spurious_anchors_warp(int*& anc, int& na) {
+    if (na < 2) return;
+    const int lane = threadIdx.x & 31;
+    // query less reference step from anchor x to x - 1
+    auto indel = [&](int x) {
+        return ((long long)anc[2 * (x - 1)] - anc[2 * x]) - ((long long)anc[2 * (x - 1) + 1] - anc[2 * x + 1]);
+    };
+    bool far = false;
+    for (int x = 1 + lane; x < na; x += 32) {
+        const long long d = indel(x);
+        far |= (d < 0 ? -d : d) > 5;
+    }
+    if (__any_sync(FULLM, far)) {
+        if (lane == 0) prune_spurious_anchors(anc, na);
+        na = __shfl_sync(FULLM, na, 0);
+        __syncwarp();
+        return;
+    }
+    const int max_prune = (int)ceilf(__fmul_rn((float)na, 0.20f));
+    const int lim = na < max_prune ? na : max_prune;
+    for (int c = 1; c < lim; c += 32) {
+        const uint32_t at = __ballot_sync(FULLM, c + lane < lim && indel(c + lane) != 0);
+        if (at) {
+            const int x = c + __ffs(at) - 1;
+            anc += 2 * x;
+            na -= x;
+            break;
+        }
+    }
+    const int lo = (na > max_prune ? na - max_prune : 0) + 1;
+    for (int c = na - 1; c >= lo; c -= 32) {
+        const uint32_t at = __ballot_sync(FULLM, c - lane >= lo && indel(c - lane) != 0);
+        if (at) {
+            na = c - (__ffs(at) - 1);
+            break;
+        }
+    }
+}
+
 // hamming_align_global's score (src/aligner.rs:261-291): matches minus mismatches over
 // equal-length pieces, floored at 0.
 __device__ __forceinline__ int hamming_global_score(const uint8_t* q, const uint8_t* r, int n, const AlignScores& sc) {
@@ -2951,19 +3045,22 @@ __device__ __forceinline__ int hamming_global_score(const uint8_t* q, const uint
 // The DP rows of a piece live in shared memory when the piece is at most smem_w - 1
 // columns wide (PW_SMEM_W: small enough that 32 single-warp blocks fit on an SM), else in
 // the block's slice of global scratch.
-constexpr uint32_t PW_SMEM_W = 256;
-__global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ list, const uint32_t* n_list_ptr,
+constexpr uint32_t PW_SMEM_W = 512;
+// anchors of a chain that are held in shared memory (longer chains: in the ops scratch)
+constexpr uint32_t PW_SMEM_ANCHORS = 64;
+constexpr size_t pw_smem_bytes(uint32_t smem_w) { return 8 * ((size_t)smem_w + PW_SMEM_ANCHORS); }
+__global__ void __launch_bounds__(32, 28) k_piecewise(const uint32_t* __restrict__ list, const uint32_t* n_list_ptr,
                                                   const ExtJob* jobs, const PrepRec* prep, const uint8_t* arena,
                                                   const uint32_t* __restrict__ anchors, AlignScores sc, uint32_t k,
                                                   uint8_t* scratch, uint64_t cells_bytes, uint64_t ops_bytes,
                                                   uint64_t rows_bytes, uint32_t smem_w, uint32_t* cigar,
                                                   ExtResult* res, uint32_t* counters) {
-    extern __shared__ int pw_rows[];
+    extern __shared__ int2 pw_rows[];
     const int lane = threadIdx.x & 31;
     const uint32_t n_list = *n_list_ptr;
     uint8_t* dirs = scratch + (size_t)blockIdx.x * (cells_bytes + ops_bytes + rows_bytes);
     uint8_t* ops = dirs + cells_bytes;
-    int* grows = reinterpret_cast<int*>(ops + ops_bytes);
+    int2* grows = reinterpret_cast<int2*>(ops + ops_bytes);
     auto rows_for = [&](int m) { return (uint32_t)m + 1 <= smem_w ? pw_rows : grows; };
     for (;;) {
         uint32_t li = 0;
@@ -2978,18 +3075,18 @@ __global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ l
         const int L = (int)p.qlen, RL = (int)p.wlen;
         const int padding = L / 10;
         // anchors (last to first) as (query start, reference start in dref); the
-        // pruning below rewrites them in this task's slice of the ops scratch
-        int* anc = reinterpret_cast<int*>(ops + (((size_t)L + RL + 8 + 15) & ~(size_t)15));
+        // pruning below rewrites them in place
         const int na0 = (int)jb.anc_n;
+        int* anc = (uint32_t)na0 <= PW_SMEM_ANCHORS
+                       ? reinterpret_cast<int*>(pw_rows + smem_w)
+                       : reinterpret_cast<int*>(ops + (((size_t)L + RL + 8 + 15) & ~(size_t)15));
         for (int a = lane; a < na0; a += 32) {
             anc[2 * a] = (int)anchors[2 * ((size_t)jb.anc_off + a)];
             anc[2 * a + 1] = (int)anchors[2 * ((size_t)jb.anc_off + a) + 1] - (int)p.wstart;
         }
         __syncwarp();
         int na = na0;
-        if (lane == 0) prune_spurious_anchors(anc, na);
-        na = __shfl_sync(FULLM, na, 0);
-        __syncwarp();
+        prune_spurious_anchors_warp(anc, na);
         CigarWriter w{cigar + p.cigar_off, 0, p.cigar_cap, false};
         auto push = [&](uint32_t op, int len) {
             if (lane == 0 && len > 0) w.push(op, (uint32_t)len);
@@ -3009,7 +3106,7 @@ __global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ l
                 pre_qs = fqs - pc.bi;
                 pre_rs = rs + (frs - rs) - pc.bj;
                 score = pc.score;
-                for (int x = 0; x < pc.nops; x++) push(ops[x], 1);
+                pw_push_ops(ops, pc.nops, true, w);
             }
         } else {
             pre_qs = fqs;
@@ -3019,6 +3116,24 @@ __global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ l
         score += K * (int)sc.match;
         push(7, K);
         for (int i = na - 1; i >= 1; i--) {
+            // overlapping anchors on one diagonal: as many as there are, up to 32 at a time
+            {
+                const int x = i - lane;
+                bool plain = false;
+                if (x >= 1) {
+                    const int step = anc[2 * (x - 1)] - anc[2 * x];
+                    plain = step >= 0 && step <= K && step == anc[2 * (x - 1) + 1] - anc[2 * x + 1];
+                }
+                const uint32_t other = __ballot_sync(FULLM, !plain);
+                const int run = other ? __ffs(other) - 1 : 32;
+                if (run) {
+                    const int mp = anc[2 * (i - run)] - anc[2 * i];
+                    score += mp * (int)sc.match;
+                    push(7, mp);
+                    i -= run - 1;
+                    continue;
+                }
+            }
             const int cqs = anc[2 * (i - 1)], crs = anc[2 * (i - 1) + 1];
             const int pqe = anc[2 * i] + K, prre = anc[2 * i + 1] + K;
             const int qd = cqs - pqe, rd = crs - prre;
@@ -3040,7 +3155,7 @@ __global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ l
                 }
                 const PwPiece pc = pw_dp<false, false>(q + pqe, qd, dref + prre, rd, sc, rows_for(rd), dirs, ops);
                 score += pc.score;
-                for (int x = pc.nops; x-- > 0;) push(ops[x], 1);
+                pw_push_ops(ops, pc.nops, false, w);
                 score += K * (int)sc.match;
                 push(7, K);
             } else if (rd < qd) {
@@ -3077,7 +3192,7 @@ __global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ l
             } else {
                 post_qe = lqe + pc.bi;
                 post_re = lre + pc.bj;
-                for (int x = pc.nops; x-- > 0;) push(ops[x], 1);
+                pw_push_ops(ops, pc.nops, false, w);
             }
             score += pc.score;
         } else {
@@ -3086,15 +3201,11 @@ __global__ void __launch_bounds__(32) k_piecewise(const uint32_t* __restrict__ l
             score += lqe == L ? (int)sc.end_bonus : 0;
         }
         if (lane == 0) w.finish();
+        const uint32_t ed = pw_edits(w);
         if (lane == 0) {
             ExtResult r = res[t];
             r.valid = 0;
             if (score > 0 && !w.overflow) {
-                uint32_t ed = 0;
-                for (uint32_t x = 0; x < w.n; x++) {
-                    const uint32_t op = w.out[x] & 15;
-                    if (op == 8 || op == 1 || op == 2) ed += w.out[x] >> 4;
-                }
                 r.valid = 1;
                 r.score = (uint32_t)score;
                 r.edit_distance = ed;
@@ -3215,37 +3326,32 @@ __global__ void __launch_bounds__(32) k_stage_pieces(uint32_t n, const uint32_t*
                                                      const uint64_t* qo, const uint8_t* r, const uint64_t* ro,
                                                      AlignScores sc, uint8_t* scratch, const uint64_t* scr_off,
                                                      StageAlignment* out, uint32_t* cigar, const uint64_t* cig_off) {
-    extern __shared__ int pw_rows[];
+    extern __shared__ int2 pw_rows[];
     const int lane = threadIdx.x & 31;
     for (uint32_t t = blockIdx.x; t < n; t += gridDim.x) {
         const uint8_t* a = q + qo[t];
         const uint8_t* b = r + ro[t];
         const int L = (int)(qo[t + 1] - qo[t]), RL = (int)(ro[t + 1] - ro[t]);
         uint8_t* dirs = scratch + scr_off[t];
-        uint8_t* ops = dirs + (size_t)(L + 1) * (RL + 1);
+        uint8_t* ops = dirs + pw_dir_bytes(L, RL);
         PwPiece pc;
         if (kinds[t] == 0) pc = pw_dp<false, false>(a, L, b, RL, sc, pw_rows, dirs, ops);
         else if (kinds[t] == 1) pc = pw_dp<true, false>(a, L, b, RL, sc, pw_rows, dirs, ops);
         else pc = pw_dp<true, true>(a, L, b, RL, sc, pw_rows, dirs, ops);
+        CigarWriter w{cigar + cig_off[t], 0, (uint32_t)(cig_off[t + 1] - cig_off[t]), false};
+        pw_push_ops(ops, pc.nops, kinds[t] == 2, w);
+        if (lane == 0) w.finish();
+        const uint32_t ed = pw_edits(w);
         if (lane == 0) {
             StageAlignment o{};
-            CigarWriter w{cigar + cig_off[t], 0, (uint32_t)(cig_off[t + 1] - cig_off[t]), false};
             if (kinds[t] == 2) {
-                for (int x = 0; x < pc.nops; x++) w.push(ops[x], 1);
                 o.query_start = (uint32_t)(L - pc.bi);
                 o.ref_start = (uint32_t)(RL - pc.bj);
                 o.query_end = (uint32_t)L;
                 o.ref_end = (uint32_t)RL;
             } else {
-                for (int x = pc.nops; x-- > 0;) w.push(ops[x], 1);
                 o.query_end = (uint32_t)pc.bi;
                 o.ref_end = (uint32_t)pc.bj;
-            }
-            w.finish();
-            uint32_t ed = 0;
-            for (uint32_t x = 0; x < w.n; x++) {
-                const uint32_t op = w.out[x] & 15;
-                if (op == 8 || op == 1 || op == 2) ed += w.out[x] >> 4;
             }
             o.valid = !w.overflow;
             o.score = pc.score;
@@ -3337,17 +3443,17 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
         // single-end piecewise jobs: a warp per job, each warp with its own DP scratch
         if (!anchors) throw Error(SA_ERR_INVALID, "internal: piecewise jobs without anchors");
         auto a16 = [](uint64_t x) { return (x + 15) & ~(uint64_t)15; };
-        const uint64_t cells = a16(((uint64_t)max_qlen + 1) * ((uint64_t)max_pw_window + 1));
+        const uint64_t cells = a16(pw_dir_bytes(max_qlen, max_pw_window));
         const uint64_t opsb = a16((uint64_t)max_qlen + max_pw_window + 8) + a16(8ull * (max_anchors + 1));
         // single-warp blocks, 28 per SM (the registers of 28 fit): the per-job work is
         // mostly serial (anchor pruning, gap checks, traceback pushes, a row at a time), so
         // more resident warps hide its latency; the rows of wide pieces go to global
         // scratch so that the shared rows stay small
         const unsigned blocks = (unsigned)std::min<uint64_t>(n, sm_count() * 28);
-        const uint64_t rowsb = a16(16ull * ((uint64_t)max_pw_window + 2));
+        const uint64_t rowsb = a16(8ull * ((uint64_t)max_pw_window + 2));
         ws.pw_scratch.reserve((cells + opsb + rowsb) * blocks);
         const uint32_t smem_w = (uint32_t)std::min<uint64_t>((uint64_t)max_pw_window + 2, PW_SMEM_W);
-        const size_t smem = 16 * (size_t)smem_w;
+        const size_t smem = pw_smem_bytes(smem_w);
         static size_t attr = 0;
         if (smem > attr) {
             SA_CUDA(cudaFuncSetAttribute(k_piecewise, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -3678,7 +3784,7 @@ void stage_pieces(uint32_t n, const uint32_t* kinds, const uint8_t* q, const uin
     uint64_t max_r = 0;
     for (uint32_t i = 0; i < n; i++) {
         const uint64_t L = qo[i + 1] - qo[i], R = ro[i + 1] - ro[i];
-        so[i + 1] = so[i] + (((L + 1) * (R + 1) + L + R + 8 + 15) & ~15ull);
+        so[i + 1] = so[i] + ((pw_dir_bytes(L, R) + L + R + 8 + 15) & ~15ull);
         max_r = std::max(max_r, R);
     }
     DevBuf<uint8_t> scratch;
@@ -3761,13 +3867,13 @@ void stage_piecewise(uint32_t n, const uint8_t* q, const uint64_t* qo, const uin
     SA_CUDA(cudaMemcpyAsync(d_counters.p + 19, &n, 4, cudaMemcpyHostToDevice, st));
     SA_CUDA(cudaMemsetAsync(d_res.p, 0, std::max<uint32_t>(n, 1) * sizeof(ExtResult), st));
     auto a16 = [](uint64_t x) { return (x + 15) & ~(uint64_t)15; };
-    const uint64_t cells = a16((max_q + 1) * (max_w + 1));
+    const uint64_t cells = a16(pw_dir_bytes(max_q, max_w));
     const uint64_t opsb = a16(max_q + max_w + 8) + a16(8ull * (max_a + 1));
     const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(n, 1024));
-    const uint64_t rowsb = a16(16ull * (max_w + 2));
+    const uint64_t rowsb = a16(8ull * (max_w + 2));
     d_scratch.reserve((cells + opsb + rowsb) * blocks);
     const uint32_t smem_w = (uint32_t)std::min<uint64_t>(max_w + 2, PW_SMEM_W);
-    const size_t smem = 16 * (size_t)smem_w;
+    const size_t smem = pw_smem_bytes(smem_w);
     if (n)
         k_piecewise<<<blocks, 32, smem, st>>>(d_list.p, d_counters.p + 19, d_jobs.p, d_prep.p, d_arena.p, d_anc.p, sc,
                                               k, d_scratch.p, cells, opsb, rowsb, smem_w, d_cigar.p, d_res.p,
