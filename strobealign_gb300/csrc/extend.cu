@@ -2,9 +2,9 @@
 // rescue_align (src/mapper.rs:1094-1153) and Aligner::align (src/aligner.rs:80-151)
 // for a list of jobs.
 //
-//   k_prepare   thread per job: NAM consistency / orientation repair
+//   k_prepare   eight lanes per job: NAM consistency / orientation repair
 //               (src/nam.rs:49-135), projected window, Hamming eligibility
-//   k_fill      thread per job: Hamming fast path (src/aligner.rs:166-259), or an SSW /
+//   k_fill      eight lanes per job: Hamming fast path (src/aligner.rs:166-259), or an SSW /
 //               piecewise task (its query and reference bytes: k_copy, a warp per task)
 //   k_sw        SSW (ext/ssw/ssw.c:163-596) with the library's striped semantics:
 //               one lane per SSE lane, 16 lanes per task in byte mode and 8 in word
@@ -191,40 +191,58 @@ __device__ __forceinline__ uint64_t ref_codes32(const DevRefs& R, uint32_t c, ui
 // "ACGT"[code]
 __device__ __forceinline__ uint8_t code_char(uint32_t code) { return (uint8_t)(0x54474341u >> (8 * code)); }
 
-// Mismatches of read positions [qs, qs + cnt) (cnt <= 32) against the reference from pos
-__device__ __forceinline__ uint32_t mismatches32(const DevRefs& R, uint32_t c, uint64_t pos, const uint8_t* s,
-                                                 uint32_t L, uint32_t qs, uint32_t cnt, bool rc) {
-    const uint64_t v = ref_codes32(R, c, pos);
-    uint32_t mm = 0;
-    for (uint32_t b = 0; b < cnt; b++) mm += read_char(s, L, qs + b, rc) != code_char((uint32_t)(v >> (2 * b)) & 3);
-    return mm;
+// Ungapped comparisons by a group of eight lanes, 32 bases a step, four a lane.  A thread per job
+// is bound by the latency of its byte loads: waves of 20 to 22,000 jobs of 50..500 nt took 52 us
+// in k_prepare and 78 us in k_fill that way, with 85 blocks on the device, and 39 and 49 us this
+// way; mapping 8 pairs takes 0.659 instead of 0.669 ms, 2000 pairs 3.44 instead of 3.48 ms,
+// larger batches the same within 2 %.
+constexpr uint32_t JOB_LANES = 8, JOBS_PER_BLOCK = 32;
+__device__ __forceinline__ uint32_t job_group_mask() { return 0xffu << (threadIdx.x & 24); }
+
+// this lane's bits of the positions [qs + x, qs + x + 32) that match the reference from
+// pos + x (positions from qs + cnt on: 0); bit b is position qs + x + b
+__device__ __forceinline__ uint32_t group_match_bits(const DevRefs& R, uint32_t c, uint64_t pos, const uint8_t* s,
+                                                     uint32_t L, uint32_t qs, uint32_t x, uint32_t cnt, bool rc) {
+    const uint32_t b0 = 4 * (threadIdx.x & (JOB_LANES - 1));
+    const uint64_t v = ref_codes32(R, c, pos + x) >> (2 * b0);
+    uint32_t m = 0;
+#pragma unroll
+    for (uint32_t b = 0; b < 4; b++)
+        if (x + b0 + b < cnt)
+            m |= (uint32_t)(read_char(s, L, qs + x + b0 + b, rc) == code_char((uint32_t)(v >> (2 * b)) & 3)) << (b0 + b);
+    return m;
+}
+
+// Mismatches of read positions [qs, qs + cnt) against the reference from pos (whole group)
+__device__ __forceinline__ uint32_t group_mismatches(const DevRefs& R, uint32_t c, uint64_t pos, const uint8_t* s,
+                                                     uint32_t L, uint32_t qs, uint32_t cnt, bool rc) {
+    uint32_t eq = 0;
+    for (uint32_t x = 0; x < cnt; x += 32) eq += __popc(group_match_bits(R, c, pos, s, L, qs, x, cnt, rc));
+    for (uint32_t d = 1; d < JOB_LANES; d <<= 1) eq += __shfl_xor_sync(job_group_mask(), eq, d);
+    return cnt - eq;
 }
 
 // Nam::is_consistent (src/nam.rs:49-69): the k-mers at both ends of the NAM match (k < 32)
 __device__ __forceinline__ bool nam_consistent(const DevRefs& R, const uint8_t* s, uint32_t L, uint32_t ref_id,
                                                uint32_t rs, uint32_t re, uint32_t qs, uint32_t qe, bool rc,
                                                uint32_t k) {
-    return mismatches32(R, ref_id, rs, s, L, qs, k, rc) == 0 && mismatches32(R, ref_id, re - k, s, L, qe - k, k, rc) == 0;
+    return group_mismatches(R, ref_id, rs, s, L, qs, k, rc) == 0 &&
+           group_mismatches(R, ref_id, re - k, s, L, qe - k, k, rc) == 0;
 }
 
-// Mismatches of the read against the reference from ref_start
-__device__ __forceinline__ uint32_t hamming_distance(const DevRefs& R, const uint8_t* s, uint32_t L, uint32_t ref_id,
-                                                     uint32_t ref_start, bool rc) {
-    uint32_t hd = 0;
-    for (uint32_t c = 0; c < L; c += 32) hd += mismatches32(R, ref_id, (uint64_t)ref_start + c, s, L, c, L - c < 32 ? L - c : 32, rc);
-    return hd;
-}
-
-// Thread per job; the reference bases come 32 at a time from the packed words
-__global__ void k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restrict__ seq,
+// A group of eight lanes per job
+__global__ void __launch_bounds__(JOB_LANES * JOBS_PER_BLOCK) k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restrict__ seq,
                           const uint64_t* __restrict__ off, DevRefs R, uint32_t k, const uint8_t* raw_refs,
                           const uint64_t* raw_off, ExtResult* res, PrepRec* prep, uint32_t* rescue_list,
                           uint32_t* n_rescue, uint32_t* max_pw_window, uint32_t* counters) {
-    const uint32_t lane = threadIdx.x & 31;
-    // whole warps: the ranges are taken a warp at a time
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t - lane < n; t += gridDim.x * blockDim.x) {
-        const bool in = t < n;
-        ExtJob jb = jobs[in ? t : n - 1];
+    __shared__ TaskSizes ranges[JOBS_PER_BLOCK];  // sizes, then starts
+    const uint32_t lane = threadIdx.x & 31, job_in_block = threadIdx.x / JOB_LANES;
+    // whole blocks: the ranges are taken for a block's 32 jobs at once, by its first warp (by
+    // every warp for its four, 60,000 jobs queue up on the cursors)
+    for (uint32_t t0 = blockIdx.x * JOBS_PER_BLOCK; t0 < n; t0 += gridDim.x * JOBS_PER_BLOCK) {
+        const uint32_t t = t0 + job_in_block;
+        const bool in = t < n && lane % JOB_LANES == 0;  // the lane that writes
+        const ExtJob jb = jobs[t < n ? t : n - 1];
         const uint8_t* s = seq + off[jb.read];
         const uint32_t L = (uint32_t)(off[jb.read + 1] - off[jb.read]);
         ExtResult r{};
@@ -262,7 +280,7 @@ __global__ void k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restr
             uint32_t pre = (uint32_t)(pre64 < clen ? pre64 : clen);
             bool hamming = false;
             if ((uint64_t)prs + L == pre && cons) {
-                const uint32_t hd = hamming_distance(R, s, L, jb.ref_id, prs, rc);
+                const uint32_t hd = group_mismatches(R, jb.ref_id, prs, s, L, 0, L, rc);
                 if (__fdiv_rn(__uint2float_rn(hd), __uint2float_rn(L)) < 0.05f) hamming = true;
             }
             if (hamming) {
@@ -312,18 +330,28 @@ __global__ void k_prepare(const ExtJob* jobs, uint32_t n, const uint8_t* __restr
             p.type = (p.wlen <= 2000 && L > 0) ? 2 : 0;
         }
         // a rescue job's ranges come from k_rescue_filter, if it is kept
-        const bool rescue = jb.kind == JOB_RESCUE;
-        const TaskSizes z = in && !rescue ? task_sizes(p.type, L, p.wlen) : TaskSizes{0, 0, 0};
-        p.cigar_cap = (uint32_t)z.cigar;
-        p.arena_off = warp_alloc(cursor64(counters, ALLOC_ARENA), z.arena);
-        p.cigar_off = warp_alloc(cursor64(counters, ALLOC_CIGAR), z.cigar);
-        p.h_off = warp_alloc(cursor64(counters, ALLOC_H), z.h);
-        const uint32_t ssw = __ballot_sync(FULLM, in && !rescue && p.type == 2);
-        if (lane == 0 && ssw) atomicAdd(&counters[N_SSW], (uint32_t)__popc(ssw));
+        const bool own = t < n && jb.kind != JOB_RESCUE;
+        if (lane % JOB_LANES == 0) ranges[job_in_block] = own ? task_sizes(p.type, L, p.wlen) : TaskSizes{0, 0, 0};
+        const int ssw = __syncthreads_count(in && own && p.type == 2);
+        p.cigar_cap = (uint32_t)ranges[job_in_block].cigar;
+        __syncthreads();
+        if (threadIdx.x < JOBS_PER_BLOCK) {
+            TaskSizes z = ranges[lane];
+            z.arena = warp_alloc(cursor64(counters, ALLOC_ARENA), z.arena);
+            z.cigar = warp_alloc(cursor64(counters, ALLOC_CIGAR), z.cigar);
+            z.h = warp_alloc(cursor64(counters, ALLOC_H), z.h);
+            ranges[lane] = z;
+            if (lane == 0 && ssw) atomicAdd(&counters[N_SSW], (uint32_t)ssw);
+        }
+        __syncthreads();
+        p.arena_off = ranges[job_in_block].arena;
+        p.cigar_off = ranges[job_in_block].cigar;
+        p.h_off = ranges[job_in_block].h;
         if (in) {
             res[t] = r;
             prep[t] = p;
         }
+        __syncthreads();
     }
 }
 
@@ -419,57 +447,108 @@ __device__ __forceinline__ uint32_t hamming_cigar_bits(const uint32_t* bits, uin
     return mm;
 }
 
-// A thread per job: Hamming jobs (hamming_align, src/aligner.rs:181-259) are run (the match
-// bits of the read against the reference, 32 bases per pair of packed reference words, then
-// the best segment and its =/X runs from the bits); SSW and piecewise jobs are listed for
-// k_copy.
-__global__ void __launch_bounds__(256) k_fill(const ExtJob* jobs, uint32_t n, const uint8_t* __restrict__ seq,
+// highest_scoring_segment from the match bits: a run of matches only raises the score, so
+// it is taken at once (match > 0); everything else a position at a time.
+__device__ __forceinline__ int32_t best_segment_bits(const uint32_t* bits, uint32_t L, const AlignScores& sc,
+                                                     uint32_t& bs, uint32_t& be) {
+    int32_t score = (int32_t)sc.end_bonus, best = 0;
+    uint32_t start = 0;
+    bs = be = 0;
+    for (uint32_t i = 0; i < L;) {
+        const uint32_t gap = ~bits[i >> 5] >> (i & 31);  // mismatches from i on, in this word
+        uint32_t len = 1;
+        if (gap & 1) {
+            score -= (int32_t)sc.mismatch;
+            if (score < 0) { start = i + 1; score = 0; }
+        } else {
+            if (sc.match) {
+                len = gap ? (uint32_t)(__ffs(gap) - 1) : 32 - (i & 31);
+                if (len > L - i) len = L - i;
+            }
+            score += (int32_t)(len * sc.match);
+        }
+        i += len;
+        if (score > best) { bs = start; best = score; be = i; }
+    }
+    if (score + (int32_t)sc.end_bonus > best) {
+        best = score + (int32_t)sc.end_bonus;
+        be = L;
+        bs = start;
+    }
+    return best;
+}
+
+// A group of eight lanes per job: Hamming jobs (hamming_align, src/aligner.rs:181-259) are run
+// (the match bits of the read against the reference, then by one lane the best segment and
+// its =/X runs from the bits); SSW and piecewise jobs are listed for k_copy.
+__global__ void __launch_bounds__(JOB_LANES * JOBS_PER_BLOCK) k_fill(const ExtJob* jobs, uint32_t n, const uint8_t* __restrict__ seq,
                                               const uint64_t* __restrict__ off, DevRefs R, AlignScores sc,
                                               const PrepRec* prep, uint32_t* cigar, ExtResult* res, SswTask* tasks,
                                               uint32_t* counters, uint32_t* pw_list) {
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-        const PrepRec p = prep[t];
-        if (p.type == 1) {
+    __shared__ uint32_t match_bits[JOBS_PER_BLOCK][MAX_READ_LEN / 32 + 1];  // an odd stride: a bank each
+    __shared__ uint32_t task_at[JOBS_PER_BLOCK];
+    __shared__ uint64_t task_cells[JOBS_PER_BLOCK];  // 0: no SSW task
+    const uint32_t lane = threadIdx.x & 31, gl = lane % JOB_LANES, job_in_block = threadIdx.x / JOB_LANES;
+    uint32_t* bits = match_bits[job_in_block];
+    for (uint32_t t0 = blockIdx.x * JOBS_PER_BLOCK; t0 < n; t0 += gridDim.x * JOBS_PER_BLOCK) {
+        const uint32_t t = t0 + job_in_block;
+        const bool in = t < n;
+        const PrepRec p = prep[in ? t : n - 1];
+        const bool ssw = in && gl == 0 && p.type == 2;
+        // the block's SSW tasks in one addition
+        if (__syncthreads_or(ssw)) {
+            if (gl == 0) task_cells[job_in_block] = ssw ? (uint64_t)p.qlen * p.wlen + 1 : 0;
+            __syncthreads();
+            if (threadIdx.x < JOBS_PER_BLOCK) {
+                unsigned long long cells = task_cells[lane];
+                const uint32_t m = __ballot_sync(FULLM, cells != 0);
+                if (cells) cells--;
+                for (uint32_t d = 1; d < 32; d <<= 1) cells += __shfl_xor_sync(FULLM, cells, d);
+                uint32_t ti = 0;
+                if (lane == 0) {
+                    ti = atomicAdd(&counters[0], (uint32_t)__popc(m));
+                    atomicAdd(reinterpret_cast<unsigned long long*>(counters + 8), cells);
+                }
+                task_at[lane] = __shfl_sync(FULLM, ti, 0) + __popc(m & ((1u << lane) - 1));
+            }
+            __syncthreads();
+            if (ssw) {
+                SswTask tk{};
+                tk.job = t;
+                tk.raw_off = RAW_FALLBACK;
+                tk.ref_begin1 = -1;
+                tk.read_begin1 = -1;
+                tasks[task_at[job_in_block]] = tk;
+            }
+        }
+        if (in && gl == 0 && p.type == 3) pw_list[atomicAdd(&counters[19], 1u)] = t;
+        if (in && p.type == 1) {
             const uint8_t* s = seq + off[p.read];
             const uint32_t L = p.qlen;
-            uint32_t bits[MAX_READ_LEN / 32];
-            const uint32_t nw = (L + 31) / 32;
-            for (uint32_t w = 0; w < nw; w++) {
-                const uint64_t v = ref_codes32(R, p.ref_id, (uint64_t)p.wstart + 32 * w);
-                const uint32_t cnt = L - 32 * w < 32 ? L - 32 * w : 32;
-                uint32_t m = 0;
-                for (uint32_t b = 0; b < cnt; b++)
-                    m |= (uint32_t)(read_char(s, L, 32 * w + b, p.rc) == code_char((uint32_t)(v >> (2 * b)) & 3)) << b;
-                bits[w] = m;
+            for (uint32_t x = 0; x < L; x += 32) {
+                uint32_t m = group_match_bits(R, p.ref_id, p.wstart, s, L, 0, x, L, p.rc);
+                for (uint32_t d = 1; d < JOB_LANES; d <<= 1) m |= __shfl_xor_sync(job_group_mask(), m, d);
+                if (gl == 0) bits[x / 32] = m;
             }
-            auto eq = [&](uint32_t i) { return (bool)((bits[i >> 5] >> (i & 31)) & 1); };
-            uint32_t bs, be;
-            const int32_t best = highest_scoring_segment(eq, L, sc, bs, be);
-            CigarWriter cw{cigar + p.cigar_off, 0, p.cigar_cap, false};
-            const uint32_t mm = hamming_cigar_bits(bits, bs, be, cw);
-            ExtResult r = res[t];
-            r.valid = cw.overflow ? 0 : 1;
-            r.score = (uint32_t)best;
-            r.edit_distance = mm;
-            r.ref_start = p.wstart + bs;
-            r.length = be - bs;
-            r.soft_clip_left = bs;
-            r.soft_clip_right = L - be;
-            r.cigar_offset = (uint32_t)p.cigar_off;
-            r.cigar_len = cw.n;
-            res[t] = r;
-        } else if (p.type == 3) {
-            pw_list[atomicAdd(&counters[19], 1u)] = t;
-        } else if (p.type == 2) {
-            const uint32_t ti = atomicAdd(&counters[0], 1u);
-            atomicAdd(reinterpret_cast<unsigned long long*>(counters + 8), (unsigned long long)p.qlen * p.wlen);
-            SswTask tk{};
-            tk.job = t;
-            tk.raw_off = RAW_FALLBACK;
-            tk.ref_begin1 = -1;
-            tk.read_begin1 = -1;
-            tasks[ti] = tk;
+            if (gl == 0) {
+                uint32_t bs, be;
+                const int32_t best = best_segment_bits(bits, L, sc, bs, be);
+                CigarWriter cw{cigar + p.cigar_off, 0, p.cigar_cap, false};
+                const uint32_t mm = hamming_cigar_bits(bits, bs, be, cw);
+                ExtResult r = res[t];
+                r.valid = cw.overflow ? 0 : 1;
+                r.score = (uint32_t)best;
+                r.edit_distance = mm;
+                r.ref_start = p.wstart + bs;
+                r.length = be - bs;
+                r.soft_clip_left = bs;
+                r.soft_clip_right = L - be;
+                r.cigar_offset = (uint32_t)p.cigar_off;
+                r.cigar_len = cw.n;
+                res[t] = r;
+            }
         }
+        __syncthreads();
     }
 }
 
@@ -2720,11 +2799,11 @@ __global__ void __launch_bounds__(128) k_finalize(const SswTask* tasks, const ui
 // lane, 45 for two, against about 90 for 32 columns of a row when the warp ran along the rows
 // (the row's E chain as a scan, the best cell by a reduction per row).  One row a lane up to 32
 // query bases, two beyond: a step of two costs half as much again, and halves the lanes that a
-// short piece keeps busy.  With that, the 32-wide traceback and the anchors of a chain looked
-// at 32 at a time, a wave of 14500 reads of 50..500 nt takes 0.3 ms instead of 0.9.  E takes max(diagonal, F) where H would do: the same for
-// gap_open >= gap_extend.  Each cell keeps four direction bits, stored by wavefront so that a
-// step's are contiguous; the traceback looks at 32 of them at a time, along the diagonal or the
-// gap.
+// short piece keeps busy.  With that, the 32-wide traceback and the anchors of a chain looked at
+// 32 at a time, a wave of 14500 reads of 50..500 nt takes 0.3 ms instead of 0.9.  E takes
+// max(diagonal, F) where H would do: the same for gap_open >= gap_extend.  Each cell keeps four
+// direction bits, stored by wavefront so that a step's are contiguous; the traceback looks at 32
+// of them at a time, along the diagonal or the gap.
 constexpr int PW_NEG = -(1 << 28);
 constexpr uint8_t PW_FROM_E = 2, PW_EEXT = 4, PW_FEXT = 8, PW_FROM_F = 16;
 
@@ -3398,8 +3477,9 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
     SA_CUDA(cudaMemsetAsync(ws.counters.p, 0, N_COUNTERS * sizeof(uint32_t), st));
     kt->begin(KS_PREPARE, st);
     ws.rescue_list.reserve(n);
-    k_prepare<<<grid1(n), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, k, raw_refs, raw_off, ws.results.p, ws.prep.p,
-                                        ws.rescue_list.p, ws.counters.p + 4, ws.counters.p + 20, ws.counters.p);
+    k_prepare<<<grid1((uint64_t)n * JOB_LANES), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, k, raw_refs, raw_off,
+                                                              ws.results.p, ws.prep.p, ws.rescue_list.p,
+                                                              ws.counters.p + 4, ws.counters.p + 20, ws.counters.p);
     {
         static bool attr = false;
         const size_t smem = 2 * RESCUE_TAB_MAX * sizeof(unsigned long long);
@@ -3429,8 +3509,8 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
     ws.list_rev_word.reserve(n);
     kt->begin(KS_FILL, st);
     ws.pw_list.reserve(n);
-    k_fill<<<grid1(n), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, sc, ws.prep.p, ws.cigar.p, ws.results.p, ws.tasks.p,
-                                     ws.counters.p, ws.pw_list.p);
+    k_fill<<<grid1((uint64_t)n * JOB_LANES), 256, 0, st>>>(ws.jobs.p, n, seq, off, refs, sc, ws.prep.p, ws.cigar.p,
+                                                           ws.results.p, ws.tasks.p, ws.counters.p, ws.pw_list.p);
     launches++;
     if (n_tasks || max_pw_window) {
         const uint64_t copies = max_pw_window ? n : n_tasks;
