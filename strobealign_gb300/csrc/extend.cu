@@ -3495,8 +3495,10 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
     kt->end(st);
     launches += 2;
     // what the ranges take, and the tasks that there will be
-    uint32_t hc[N_COUNTERS];
-    SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    // read back into pinned memory where the workspace keeps some
+    uint32_t own_counters[N_COUNTERS];
+    uint32_t* hc = ws.h_counters.p ? ws.h_counters.p : own_counters;
+    SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, N_COUNTERS * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     SA_CUDA(cudaStreamSynchronize(st));
     auto total_of = [&](int at) { return (uint64_t)hc[at] | (uint64_t)hc[at + 1] << 32; };
     const uint32_t n_tasks = hc[N_SSW], max_pw_window = hc[20];
@@ -3751,7 +3753,7 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
     ws.offs.reserve(n);
     k_cigar_used<<<grid1(n), 256, 0, st>>>(ws.results.p, n, ws.offs.p, ws.counters.p);
     launches++;
-    SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
+    SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, N_COUNTERS * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     SA_CUDA(cudaStreamSynchronize(st));
     if (const uint32_t n_wide = hc[29]) {
         const int maxc = 2 * (int)std::max<uint32_t>(2048, max_qlen) + 8;
@@ -3778,7 +3780,7 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
         SA_CUDA(cudaMemsetAsync(ws.counters.p + ALLOC_USED, 0, 8, st));
         k_cigar_used<<<grid1(n), 256, 0, st>>>(ws.results.p, n, ws.offs.p, ws.counters.p);
         launches += 3;
-        SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, sizeof(hc), cudaMemcpyDeviceToHost, st));
+        SA_CUDA(cudaMemcpyAsync(hc, ws.counters.p, N_COUNTERS * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         SA_CUDA(cudaStreamSynchronize(st));
     }
     const uint64_t used = total_of(ALLOC_USED);
@@ -3800,6 +3802,7 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
 uint32_t run_extension(const DevRefs& refs, const NamWorkspace& nws, uint32_t k, const AlignScores& sc, uint32_t n,
                        ExtWorkspace& ws, uint32_t max_qlen, cudaStream_t st, KernelTimers* kt, const uint32_t* anchors,
                        uint32_t max_anchors) {
+    ws.h_counters.reserve(N_COUNTERS);
     return run_extension_raw(refs, nws.seq.p, nws.off.p, nullptr, nullptr, k, sc, n, ws, max_qlen, st, kt, anchors,
                              max_anchors);
 }

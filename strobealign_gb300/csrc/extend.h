@@ -72,6 +72,7 @@ struct ExtWorkspace {
     DevBuf<uint8_t> cub_tmp;
     // host mirrors (capacity kept across waves; the callers swap them with pooled
     // wave buffers)
+    PinnedBuf<uint32_t> h_counters;  // the counters read back; kept by mapping workspaces only
     PodArray<ExtResult> h_results;
     PodArray<uint32_t> h_cigar;
     uint64_t total_cigar = 0;

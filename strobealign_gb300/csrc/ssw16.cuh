@@ -48,6 +48,8 @@ constexpr uint32_t FULLM = 0xffffffffu;
 constexpr int KEY_BITS = 5;
 constexpr uint32_t ROW_BITS = 0x001f001fu;
 constexpr uint32_t CODE_NONE = 5;       // no column here
+constexpr uint32_t NO_BASE = 256;       // its index in the code table (CODE_TABLE uint4)
+constexpr int CODE_TABLE = 17;
 constexpr int T16 = 8;                  // threads per task
 constexpr int SSW16_WARPS = 2;          // per block
 
@@ -81,7 +83,13 @@ __device__ __forceinline__ uint32_t addmax2(uint32_t a, uint32_t b, uint32_t c) 
 // mode); they sit in the last n of the NB registers, the d0 before them unused.  Only the
 // first SKIP rows test for that: 0 when every group of the warp uses all registers, 4 when
 // none leaves out more.
-template <int NB, bool BYTE, int SKIP, class GP>
+// AHEAD: the columns' codes and the first rows' profiles are read a step ahead, lane 0's
+// base two steps ahead. A warp that is alone on its scheduler waits for each of these reads
+// in every step otherwise (waves of 14 to 500 tasks of 150 nt: 97 to 180 us, 140 to 245
+// before). Where other warps fill the waits it only costs registers: with the base alone
+// read ahead, 140 for 127 at 20 rows and 188 for 152 at 32, and 60,000 tasks of 100-300 nt
+// lost 5 %.
+template <int NB, bool BYTE, int SKIP, bool AHEAD, class GP>
 __device__ __forceinline__ End16 wave16(const uint8_t* r, int rlen, bool r_rev, int qlen, bool check_term,
                                         int terminate, int bias, GP gp, const uint4* prof, const uint8_t* code, int n,
                                         int seg, int d0) {
@@ -106,18 +114,32 @@ __device__ __forceinline__ End16 wave16(const uint8_t* r, int rlen, bool r_rev, 
     const int dir = r_rev ? -1 : 1;
     const uint8_t* rp = r + (r_rev ? rlen - 1 : 0);
     uint32_t b_next = gl == 0 && rlen > 0 ? code[*rp] * STEP : NONE;
+    // AHEAD: b_lo, b_hi and the first rows' profiles are this step's already
+    uint32_t base_next = NO_BASE;
+    uint4 L_next, U_next;
+    if (AHEAD) {
+        b_lo = b_next;
+        L_next = prof[b_lo];
+        U_next = prof[6 * STEP + b_hi];
+        rp += dir;
+        b_next = rlen > 1 ? code[*rp] * STEP : NONE;
+        rp += dir;
+        if (rlen > 2) base_next = *rp;
+    }
     int steps = __reduce_max_sync(FULLM, limit ? limit + V - 1 : 0);
     const int thr = ((BYTE && !check_term ? 255 - bias : terminate) << KEY_BITS);
     for (int s = 0; s < steps; s++) {
         const uint32_t w = __shfl_up_sync(FULLM, __byte_perm(hO, xO, 0x7632), 1, T);
         uint32_t bin = __shfl_up_sync(FULLM, b_hi, 1, T);
-        b_hi = b_lo;
-        if (gl == 0) {
-            bin = b_next;
-            rp += dir;
-            b_next = s + 1 < rlen ? code[*rp] * STEP : NONE;
+        if (!AHEAD) {
+            b_hi = b_lo;
+            if (gl == 0) {
+                bin = b_next;
+                rp += dir;
+                b_next = s + 1 < rlen ? code[*rp] * STEP : NONE;
+            }
+            b_lo = bin;
         }
-        b_lo = bin;
         const uint32_t win = gl == 0 ? 0 : w;
         const uint32_t hin = __byte_perm(win, hO, 0x5410);
         uint32_t gb = __byte_perm(win, SPLIT ? gO : xO, 0x5432);
@@ -132,9 +154,20 @@ __device__ __forceinline__ End16 wave16(const uint8_t* r, int rlen, bool r_rev, 
         uint32_t f_last = 0;
         uint32_t gj = gb;
         uint4 L, U;
+        if (AHEAD) {
+            L = L_next;
+            U = U_next;
+            b_hi = b_lo;
+            b_lo = gl == 0 ? b_next : bin;
+            b_next = code[base_next] * STEP;
+            rp += dir;
+            base_next = s + 3 < rlen ? *rp : NO_BASE;
+            L_next = prof[b_lo];
+            U_next = prof[6 * STEP + b_hi];
+        }
 #pragma unroll
         for (int j = 0; j < NB; j++) {
-            if ((j & 7) == 0) {
+            if ((j & 7) == 0 && (j > 0 || !AHEAD)) {
                 L = pl[(j >> 3) * 32];
                 U = ph[(j >> 3) * 32];
             }
@@ -261,20 +294,21 @@ __device__ __forceinline__ void profile16(const uint8_t* q, int qlen, bool q_rev
 // A pass of the groups that run: with NB registers per piece where that is enough for
 // the warp's longest lane (the next size otherwise, MAXNB at last), the profiles of their
 // pieces, then the wavefront.
-template <int NB, int MAXNB, bool BYTE, class GP>
+template <int NB, int MAXNB, bool BYTE, bool AHEAD, class GP>
 __device__ __forceinline__ End16 pass16(bool run, const uint8_t* q, int qlen, bool q_rev, const uint8_t* r, int rlen,
                                         bool r_rev, bool check_term, int terminate, int match, int mismatch, int bias,
                                         GP gp, uint4* prof, const uint8_t* code, int n, int seg, int nmax, int nmin) {
     if constexpr (NB < MAXNB) {
         constexpr int NEXT = NB == 8 ? 10 : NB == 10 ? 12 : NB + 4;
         if (NB - nmin > 4 || nmax > NB)
-            return pass16<NEXT, MAXNB, BYTE, GP>(run, q, qlen, q_rev, r, rlen, r_rev, check_term, terminate, match,
-                                                 mismatch, bias, gp, prof, code, n, seg, nmax, nmin);
+            return pass16<NEXT, MAXNB, BYTE, AHEAD, GP>(run, q, qlen, q_rev, r, rlen, r_rev, check_term, terminate,
+                                                        match, mismatch, bias, gp, prof, code, n, seg, nmax, nmin);
     }
     const int d0 = run ? NB - n : 0;
     if (run) profile16<NB, BYTE>(q, qlen, q_rev, match, mismatch, prof, code, n, seg, d0);
 #define SA_W16(S) \
-    wave16<NB, BYTE, S, GP>(r, run ? rlen : 0, r_rev, qlen, check_term, terminate, bias, gp, prof, code, n, seg, d0)
+    wave16<NB, BYTE, S, AHEAD, GP>(r, run ? rlen : 0, r_rev, qlen, check_term, terminate, bias, gp, prof, code, n, seg, \
+                                   d0)
     if constexpr (std::is_same_v<GP, DefaultGaps>) {
         if (nmin == NB) return SA_W16(0);
         if (NB < MAXNB || NB - nmin <= 4) return SA_W16(4);
@@ -283,7 +317,7 @@ __device__ __forceinline__ End16 pass16(bool run, const uint8_t* q, int qlen, bo
 #undef SA_W16
 }
 
-template <int MAXNB, bool BYTE, class GP>
+template <int MAXNB, bool BYTE, bool AHEAD, class GP>
 __device__ __forceinline__ End16 pass16(bool run, const uint8_t* q, int qlen, bool q_rev, const uint8_t* r, int rlen,
                                         bool r_rev, bool check_term, int terminate, int match, int mismatch, int bias,
                                         GP gp, uint4* prof, const uint8_t* code) {
@@ -300,8 +334,8 @@ __device__ __forceinline__ End16 pass16(bool run, const uint8_t* q, int qlen, bo
     const int nmax = __reduce_max_sync(FULLM, n), nmin = __reduce_min_sync(FULLM, run ? n : nmax);
     // other gap penalties: one size, all rows tested
     constexpr int FIRST = std::is_same_v<GP, DefaultGaps> ? 8 : MAXNB;
-    const End16 e = pass16<FIRST, MAXNB, BYTE, GP>(run, q, qlen, q_rev, r, rlen, r_rev, check_term, terminate, match,
-                                                   mismatch, bias, gp, prof, code, n, seg, nmax, nmin);
+    const End16 e = pass16<FIRST, MAXNB, BYTE, AHEAD, GP>(run, q, qlen, q_rev, r, rlen, r_rev, check_term, terminate,
+                                                          match, mismatch, bias, gp, prof, code, n, seg, nmax, nmin);
     return run ? e : z;
 }
 
@@ -361,7 +395,8 @@ __device__ __forceinline__ int diag_bound(bool run, const uint8_t* q, int qlen, 
 // PAIR: a block's two warps share four tasks, the first for the byte passes, the second
 // for the word passes: the forward passes of a task run at once, whether the byte pass
 // overflows or not.  More work but less latency, for launches that leave SMs idle: 140
-// rescue tasks (windows of up to 600 columns) 0.21 ms, 0.35 ms without.
+// rescue tasks (windows of up to 600 columns) 0.15 ms; 0.21 ms without the reads
+// ahead, 0.35 ms with the passes one after the other.
 template <int NB, bool PAIR, class GP>
 __global__ void __launch_bounds__(32 * SSW16_WARPS, NB > 20 ? 4 : 6)
     k_ssw16(SswTask* tasks, const uint32_t* order, uint32_t n_tasks, const PrepRec* prep, const uint8_t* arena,
@@ -377,9 +412,10 @@ __global__ void __launch_bounds__(32 * SSW16_WARPS, NB > 20 ? 4 : 6)
         const char u = (char)(i & 0xdf);
         code[i] = i >= 128 ? 4 : u == 'A' || u == 'U' ? 0 : u == 'C' ? 1 : u == 'G' ? 2 : u == 'T' ? 3 : 4;
     }
+    if (threadIdx.x == 0) code[NO_BASE] = CODE_NONE;
     __syncthreads();
     const int lane = threadIdx.x & 31, gi = lane / T, gl = lane % T, wib = threadIdx.x / 32;
-    uint4* prof = s16_smem + 16 + wib * (2 * 6 * NW * 32) + lane;
+    uint4* prof = s16_smem + CODE_TABLE + wib * (2 * 6 * NW * 32) + lane;
     unsigned long long* cells = reinterpret_cast<unsigned long long*>(counters + 8);
     for (;;) {
         uint32_t base = 0;
@@ -412,20 +448,21 @@ __global__ void __launch_bounds__(32 * SSW16_WARPS, NB > 20 ? 4 : 6)
         }
         const uint8_t* r = q + qlen;
         // a byte pass that must overflow is skipped: the word pass alone gives the same
-        // results (the task's diagonal bound reaches 255 - bias)
-        const bool try_bound = have && d0 != NO_DIAG && qlen * (int)sc.match >= 255 - bias;
+        // results (the task's diagonal bound reaches 255 - bias).  Where the two run side by
+        // side, the bound would only come before both (22 us at 150 nt).
+        const bool try_bound = !PAIR && have && d0 != NO_DIAG && qlen * (int)sc.match >= 255 - bias;
         bool certain = false;
-        if (__any_sync(FULLM, try_bound))
+        if (!PAIR && __any_sync(FULLM, try_bound))
             certain = diag_bound<T>(try_bound, q, qlen, r, wlen, (int)d0, sc.match, sc.mismatch, sc.gap_open,
                                     sc.gap_extend, gl, code) >= 255 - bias;
         // forward: byte, word on overflow (ext/ssw/ssw.c:840-862)
         End16 e, ew;
         if (!PAIR || wib == 0)
-            e = pass16<NB, true, GP>(have && !certain, q, qlen, false, r, wlen, false, false, 0, sc.match, sc.mismatch,
-                                     bias, gp, prof, code);
+            e = pass16<NB, true, PAIR, GP>(have && !certain, q, qlen, false, r, wlen, false, false, 0, sc.match,
+                                           sc.mismatch, bias, gp, prof, code);
         if (!PAIR || wib == 1)
-            ew = pass16<NB, false, GP>(have && (PAIR || certain || e.score == 255), q, qlen, false, r, wlen, false,
-                                       false, 0, sc.match, sc.mismatch, bias, gp, prof, code);
+            ew = pass16<NB, false, PAIR, GP>(have && (PAIR || certain || e.score == 255), q, qlen, false, r, wlen,
+                                             false, false, 0, sc.match, sc.mismatch, bias, gp, prof, code);
         if (PAIR) {
             if (gl == 0) s_end[wib][gi] = wib ? ew : e;
             __syncthreads();
@@ -440,11 +477,11 @@ __global__ void __launch_bounds__(32 * SSW16_WARPS, NB > 20 ? 4 : 6)
         const bool rev = have && e.ref >= 0;
         End16 b;
         if (!PAIR || wib == 0)
-            b = pass16<NB, true, GP>(rev && !word, q, e.read + 1, true, r, e.ref + 1, true, true, e.score, sc.match,
-                                     sc.mismatch, bias, gp, prof, code);
+            b = pass16<NB, true, PAIR, GP>(rev && !word, q, e.read + 1, true, r, e.ref + 1, true, true, e.score,
+                                           sc.match, sc.mismatch, bias, gp, prof, code);
         if (!PAIR || wib == 1) {
-            const End16 bw = pass16<NB, false, GP>(rev && word, q, e.read + 1, true, r, e.ref + 1, true, true, e.score,
-                                                   sc.match, sc.mismatch, bias, gp, prof, code);
+            const End16 bw = pass16<NB, false, PAIR, GP>(rev && word, q, e.read + 1, true, r, e.ref + 1, true, true,
+                                                         e.score, sc.match, sc.mismatch, bias, gp, prof, code);
             if (word) b = bw;
         }
         if (!rev) {
@@ -510,7 +547,7 @@ inline Gaps other_gaps(const AlignScores& sc) {
 template <int NB, bool PAIR, class GP>
 void launch_one(const Ssw16Args& a, GP gp) {
     constexpr int NW = (NB + 7) / 8, G = 32 / T16;
-    const size_t smem = (16 + (size_t)SSW16_WARPS * 2 * 6 * NW * 32) * sizeof(uint4);
+    const size_t smem = (CODE_TABLE + (size_t)SSW16_WARPS * 2 * 6 * NW * 32) * sizeof(uint4);
     SA_CUDA(cudaFuncSetAttribute(k_ssw16<NB, PAIR, GP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint64_t per_block = (uint64_t)(PAIR ? 1 : SSW16_WARPS) * G;
     const uint64_t blocks = std::min<uint64_t>((a.n_tasks + per_block - 1) / per_block, sm_count() * 32);
