@@ -40,14 +40,10 @@ constexpr int WARPS_PER_BLOCK = 8;
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 __device__ __forceinline__ uint32_t lanemask_lt() { return (1u << lane_id()) - 1; }
 
-__device__ __forceinline__ uint8_t nt_code(uint8_t c) {
-    switch (c) {
-        case 'A': case 'a': return 0;
-        case 'C': case 'c': return 1;
-        case 'G': case 'g': return 2;
-        case 'T': case 't': case 'U': case 'u': return 3;
-        default: return 4;
-    }
+// A, C, G, T or U, in either case: 0 to 3; anything else 4
+__device__ __forceinline__ uint32_t nt_code(uint8_t c) {
+    const uint32_t u = c & 0xdfu, x = u - 'A';
+    return x < 32 && ((0x180045u >> x) & 1) ? ((u >> 1) ^ (u >> 2)) & 3 : 4;
 }
 
 // ------------------------------------------------------------------ seeding
@@ -63,9 +59,9 @@ __device__ __forceinline__ uint64_t spread_bits(uint32_t v) {
     return x;
 }
 __device__ __forceinline__ uint64_t window_bits(const uint64_t* packed, uint32_t q) {
-    const uint32_t w = q >> 5, sh = 2 * (q & 31);
-    const uint64_t lo = packed[w] >> sh;
-    return sh ? lo | (packed[w + 1] << (64 - sh)) : lo;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(packed) + (q >> 4);
+    const uint32_t sh = 2 * (q & 15), w1 = w[1];
+    return (uint64_t)__funnelshift_r(w1, w[2], sh) << 32 | __funnelshift_r(w[0], w1, sh);
 }
 __device__ __forceinline__ uint32_t window_n(const uint32_t* nflags, uint32_t q) {
     const uint32_t w = q >> 5;
@@ -85,6 +81,14 @@ __device__ __forceinline__ void kmer_codes(uint64_t w, uint32_t n, uint64_t& fw,
 
 // src/seeding/syncmers.rs:171-237: a syncmer at p requires an N-free k-mer window
 // and the (t-1)-th of its k-s+1 s-mer hashes to equal their minimum.
+// Bound by the instructions issued. The bases are packed for 32 words at a time by a lane
+// each; the windows' minima take log2 steps; the k-mers of syncmers are hashed once their
+// positions are gathered, by full warps; and the syncmers stay in shared memory, unless a
+// read has more than SEED_SYNCMERS (104, what the warp's 2 KB leave room for), whose
+// syncmers all go to global memory. 100,000 reads of 150 nt take 0.207 ms; 0.300 ms (2850
+// warp instructions a read) with a shuffle per window position, each chunk's few syncmers
+// hashed at once and the syncmers in global memory.
+constexpr uint32_t SEED_SYNCMERS = 104;
 // CHECKED (offsets supplied by a caller, not built here): a read whose offsets are
 // decreasing, end past `total` or span more than MAX_READ_LEN gets the count
 // UINT32_MAX in both orientations and is not touched otherwise.
@@ -94,11 +98,15 @@ __global__ void __launch_bounds__(256) k_seed(const uint8_t* __restrict__ seq, c
                                               uint64_t* qr_hash, uint64_t* qr_hash_rc, uint32_t* qr_start,
                                               uint32_t* qr_end, uint64_t total, uint32_t* n_rs) {
     extern __shared__ uint8_t smem[];
-    // per warp: packed bases (MAX_READ_LEN / 32 + 2 words) then N flags
+    // per warp: packed bases and N flags (MAX_READ_LEN / 32 + 2 words each), then syncmers
+    constexpr uint32_t WORDS = MAX_READ_LEN / 32 + 2;
+    static_assert(WORDS * 12 + SEED_SYNCMERS * 12 <= MAX_READ_LEN && WORDS % 2 == 0, "a warp's shared memory");
     uint64_t* packed = reinterpret_cast<uint64_t*>(smem + (threadIdx.x / 32) * MAX_READ_LEN);
-    uint32_t* nflags = reinterpret_cast<uint32_t*>(packed + MAX_READ_LEN / 32 + 2);
+    uint32_t* nflags = reinterpret_cast<uint32_t*>(packed + WORDS);
+    uint64_t* sh_hash = reinterpret_cast<uint64_t*>(nflags + WORDS);
+    uint32_t* sh_pos = reinterpret_cast<uint32_t*>(sh_hash + SEED_SYNCMERS);
     const uint32_t lane = lane_id();
-    const uint32_t span = p.k - p.s, step = 32 - span;
+    const uint32_t span = p.k - p.s, step = 32 - span, all = (uint32_t)low_mask(span + 1);
     const uint32_t nwarps = gridDim.x * (blockDim.x / 32);
     for (uint32_t r = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32; r < n; r += nwarps) {
         const uint64_t o = off[r];
@@ -114,14 +122,23 @@ __global__ void __launch_bounds__(256) k_seed(const uint8_t* __restrict__ seq, c
         }
         const uint32_t L = (uint32_t)(off[r + 1] - o);
         const uint32_t nwords = (L + 31) / 32;
-        for (uint32_t w = 0; w <= nwords; w++) {
-            const uint32_t i = w * 32 + lane;
-            const uint32_t cc = i < L ? nt_code(seq[o + i]) : 0;
-            const uint32_t b0 = __ballot_sync(FULL, cc & 1), b1 = __ballot_sync(FULL, (cc >> 1) & 1);
-            const uint32_t bn = __ballot_sync(FULL, cc > 3);
-            if (lane == 0) {
-                packed[w] = spread_bits(b0) | (spread_bits(b1) << 1);
-                nflags[w] = bn;
+        for (uint32_t w0 = 0; w0 <= nwords; w0 += 32) {
+            uint32_t b0 = 0, b1 = 0, bn = 0;
+            const uint32_t wn = nwords + 1 - w0 < 32 ? nwords + 1 - w0 : 32;
+            for (uint32_t w = 0; w < wn; w++) {
+                const uint32_t i = (w0 + w) * 32 + lane;
+                const uint32_t cc = i < L ? nt_code(seq[o + i]) : 0;
+                const uint32_t v0 = __ballot_sync(FULL, cc & 1), v1 = __ballot_sync(FULL, cc & 2);
+                const uint32_t vn = __ballot_sync(FULL, cc > 3);
+                if (lane == w) {
+                    b0 = v0;
+                    b1 = v1;
+                    bn = vn;
+                }
+            }
+            if (lane < wn) {
+                packed[w0 + lane] = spread_bits(b0) | (spread_bits(b1) << 1);
+                nflags[w0 + lane] = bn;
             }
         }
         __syncwarp();
@@ -134,49 +151,58 @@ __global__ void __launch_bounds__(256) k_seed(const uint8_t* __restrict__ seq, c
                 v = (window_n(nflags, q) & (uint32_t)low_mask(p.s)) == 0;
                 kmer_codes(window_bits(packed, q), p.s, fw, rc);
             }
-            uint64_t hs = v ? xxh64_u64(fw < rc ? fw : rc) : 0;
-            bool ok = true;
-            uint64_t mn = UINT64_MAX, ht = 0;
-            for (uint32_t d = 0; d <= span; d++) {
-                uint64_t h = __shfl_down_sync(FULL, hs, d);
-                bool vv = __shfl_down_sync(FULL, v, d);
-                ok = ok && vv;
+            const uint64_t hs = v ? xxh64_u64(fw < rc ? fw : rc) : 0;
+            const uint32_t good = __ballot_sync(FULL, v) >> lane;
+            // the window's minimum (lanes >= step: not used)
+            uint64_t mn = hs;
+            uint32_t len = 1;
+            for (; 2 * len <= span + 1; len *= 2) {
+                const uint64_t h = __shfl_down_sync(FULL, mn, len);
                 mn = h < mn ? h : mn;
-                if (d == p.t - 1) ht = h;
             }
-            const uint32_t pos = c + lane;
-            bool is_syn = lane < step && pos + p.k <= L && ok && ht == mn;
-            uint64_t kh = 0;
-            uint32_t fwd = 0;
-            if (is_syn) {
-                uint64_t kf, kr;
-                kmer_codes(window_bits(packed, pos), p.k, kf, kr);
-                kh = xxh64_u64(kf < kr ? kf : kr);
-                fwd = kf <= kr;
+            if (len <= span) {
+                const uint64_t h = __shfl_down_sync(FULL, mn, span + 1 - len);
+                mn = h < mn ? h : mn;
             }
-            uint32_t bal = __ballot_sync(FULL, is_syn);
+            const uint64_t ht = p.t - 1 <= span ? __shfl_down_sync(FULL, hs, p.t - 1) : 0;
+            const bool is_syn = lane < step && q + p.k <= L && (good & all) == all && ht == mn;
+            const uint32_t bal = __ballot_sync(FULL, is_syn);
             if (is_syn) {
-                uint32_t idx = nsyn + __popc(bal & lanemask_lt());
-                syn_hash[o + idx] = kh;
-                syn_pos[o + idx] = (pos << 1) | fwd;
+                const uint32_t idx = nsyn + __popc(bal & lanemask_lt());
+                if (idx < SEED_SYNCMERS) sh_pos[idx] = q;
+                else syn_pos[o + idx] = q;
             }
             nsyn += __popc(bal);
+        }
+        __syncwarp();
+        const bool in_shared = nsyn <= SEED_SYNCMERS;
+        if (!in_shared)
+            for (uint32_t i = lane; i < SEED_SYNCMERS; i += 32) syn_pos[o + i] = sh_pos[i];
+        uint32_t* spos = in_shared ? sh_pos : syn_pos + o;
+        uint64_t* shash = in_shared ? sh_hash : syn_hash + o;
+        __syncwarp();
+        for (uint32_t i = lane; i < nsyn; i += 32) {
+            const uint32_t pos = spos[i];
+            uint64_t kf, kr;
+            kmer_codes(window_bits(packed, pos), p.k, kf, kr);
+            shash[i] = xxh64_u64(kf < kr ? kf : kr);
+            spos[i] = (pos << 1) | (uint32_t)(kf <= kr);
         }
         __syncwarp();
         const uint32_t nr = L < p.w_max ? 0 : nsyn;
         // forward randstrobes (src/seeding/strobes.rs:145-176)
         for (uint32_t i = lane; i < nr; i += 32) {
-            uint64_t h1 = syn_hash[o + i];
-            uint32_t p1 = syn_pos[o + i];
+            uint64_t h1 = shash[i];
+            uint32_t p1 = spos[i];
             uint32_t pos1 = p1 >> 1;
-            uint64_t best = UINT64_MAX;
+            uint32_t best = UINT32_MAX;
             uint64_t h2 = h1;
             uint32_t p2 = p1;
             for (uint32_t j = i + p.w_min; j <= i + p.w_max && j < nsyn; j++) {
-                uint32_t pj = syn_pos[o + j];
+                uint32_t pj = spos[j];
                 if ((pj >> 1) > pos1 + p.max_dist) break;
-                uint64_t hj = syn_hash[o + j];
-                uint64_t ones = (uint64_t)__popcll((h1 ^ hj) & p.q);
+                uint64_t hj = shash[j];
+                const uint32_t ones = __popcll((h1 ^ hj) & p.q);
                 if (ones < best) { best = ones; h2 = hj; p2 = pj; }
             }
             uint64_t f1 = p1 & 1, f2 = p2 & 1;
@@ -188,20 +214,20 @@ __global__ void __launch_bounds__(256) k_seed(const uint8_t* __restrict__ seq, c
         // reverse-complement randstrobes from the reversed syncmer list (src/seeding/mod.rs:53-73)
         for (uint32_t ir = lane; ir < nr; ir += 32) {
             uint32_t i = nsyn - 1 - ir;
-            uint64_t h1 = syn_hash[o + i];
-            uint32_t p1 = syn_pos[o + i];
+            uint64_t h1 = shash[i];
+            uint32_t p1 = spos[i];
             uint32_t pos1 = L - (p1 >> 1) - p.k;
             uint32_t f1 = (p1 & 1) ^ 1;
-            uint64_t best = UINT64_MAX;
+            uint32_t best = UINT32_MAX;
             uint64_t h2 = h1;
             uint32_t pos2 = pos1, f2 = f1;
             for (uint32_t d = p.w_min; d <= p.w_max && d <= i; d++) {
                 uint32_t j = i - d;
-                uint32_t pj = syn_pos[o + j];
+                uint32_t pj = spos[j];
                 uint32_t posj = L - (pj >> 1) - p.k;
                 if (posj > pos1 + p.max_dist) break;
-                uint64_t hj = syn_hash[o + j];
-                uint64_t ones = (uint64_t)__popcll((h1 ^ hj) & p.q);
+                uint64_t hj = shash[j];
+                const uint32_t ones = __popcll((h1 ^ hj) & p.q);
                 if (ones < best) { best = ones; h2 = hj; pos2 = posj; f2 = (pj & 1) ^ 1; }
             }
             qr_hash[total + o + ir] = randstrobe_hash(h1, h2, f1, f2, p);
