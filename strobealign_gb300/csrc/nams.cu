@@ -300,10 +300,12 @@ __device__ uint32_t warp_rescue_least_frequent(const DevIndex& ix, uint32_t s, u
 // Per-randstrobe index probes of find_hits' first pass (src/hit.rs:143-187), ahead of
 // k_hits: lanes run over both orientations' randstrobes of a read together, each lane
 // one probe with the latency-parallel lookups.  Writes, per randstrobe slot, the table
-// position (UINT64_MAX if absent) and PROBE_* flags; k_hits compacts them in place.
+// position (UINT64_MAX if absent) and PROBE_* flags; k_hits compacts them in place.  Bound by
+// the latency of random table sectors: five blocks an SM in 48 registers (four in 57: 100,000
+// reads spend 1.62 ms in the NAM stage instead of 1.59; six in 40 spill: 1.63).
 constexpr uint32_t PROBE_FULL = 1, PROBE_PARTIAL = 2, PROBE_FILTERED = 4;
 
-__global__ void __launch_bounds__(256) k_probe(DevIndex ix, const uint64_t* __restrict__ off, uint32_t n,
+__global__ void __launch_bounds__(256, 5) k_probe(DevIndex ix, const uint64_t* __restrict__ off, uint32_t n,
                                                uint64_t total, uint32_t mcs, const uint64_t* __restrict__ qr_hash,
                                                const uint64_t* __restrict__ qr_hash_rc,
                                                const uint32_t* __restrict__ n_rs, uint64_t* __restrict__ hit_pos,
@@ -633,13 +635,14 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t& total) 
     return x - v;
 }
 
-// The anchors of each read orientation (src/chainer.rs:304-384): counted, then written to
-// the next free range of the anchor array while the table entries are still in the L1 (a
-// launch each for counts and anchors read the table's random sectors twice: 11.2 KB of
-// DRAM per read on a human-sized index; 3.0 ms for 0.7 M reads, 2.3 ms now).  The ranges'
-// order does not matter to the stages after.  Past the array's capacity nothing is written; *cursor then tells what it
-// takes.
-__global__ void __launch_bounds__(256) k_anchors(DevIndex ix, const uint64_t* __restrict__ off, uint32_t n,
+// The anchors of each read orientation (src/chainer.rs:304-384): counted, then written to the
+// next free range of the anchor array while the table entries are still in the L1 (a launch
+// each for counts and anchors read the table's random sectors twice: 11.2 KB of DRAM per read
+// on a human-sized index; 3.0 ms for 0.7 M reads, 2.3 ms now).  The ranges' order does not
+// matter to the stages after.  Past the array's capacity nothing is written; *cursor then
+// tells what it takes. Five blocks an SM in 48 registers: the NAM stage of 100,000 reads takes
+// 1.60 ms, with four in 64 registers 1.62 ms; six gain nothing more.
+__global__ void __launch_bounds__(256, 5) k_anchors(DevIndex ix, const uint64_t* __restrict__ off, uint32_t n,
                                                  uint64_t total, const uint64_t* qr_hash, const uint32_t* qr_start,
                                                  const uint32_t* qr_end, const uint64_t* hit_pos,
                                                  const uint32_t* hit_info, const uint32_t* n_hits,
