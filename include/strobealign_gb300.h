@@ -445,7 +445,9 @@ int32_t sa_map_uploaded(sa_mapper* m, sa_output* out);
  * parts whose NAM pipelines overlap the extension waves and the policy:
  * seconds_nams sums the parts' pipelines, seconds_extension the waves, and
  * seconds_policy is the rest of seconds_total after the waves and the first part's
- * pipeline. */
+ * pipeline.  seconds_upload is what precedes: the preparation of the batch on the host, and
+ * for sa_mapper_upload also the copies (sa_map_batch copies part by part inside the
+ * pipelines). */
 typedef struct {
     double seconds_upload, seconds_nams, seconds_extension, seconds_policy, seconds_total;
     uint64_t n_jobs, n_waves, n_launches;
@@ -505,10 +507,13 @@ int32_t sa_mapper_set_schedule(sa_mapper* m, const sa_schedule_params* p);
 /* Tuning knobs of a mapper, chosen by sa_mapper_autotune.  No counterpart in the
  * reference; output bytes never depend on them.
  *   parts, wave_min_jobs, max_wave_jobs  as in sa_schedule_params
- *   ssw_wave_max_qlen       SSW tasks of reads up to this length (at most 192) run on
- *                           the lane-wavefront kernel, longer ones a warp per task
+ *   ssw_wave_max_qlen       SSW tasks of reads up to this length run on the
+ *                           lane-wavefront kernels, longer ones a warp per task; 192, the
+ *                           largest value, stands for all reads that the 16-bit kernel
+ *                           takes (511 nt with the default scores)
  *   chain_lane_cluster_max  clusters of a long read orientation's anchors up to this
- *                           size are chained by one thread, larger ones by a warp
+ *                           size (at least 2) are chained by one thread, larger ones by a
+ *                           block
  *   l2_fetch_bytes          the context's L2 fetch granularity for DRAM reads
  *                           (cudaLimitMaxL2FetchGranularity: 32, 64 or 128; 0 keeps the
  *                           value the context had when the mapper was created).  It is a

@@ -3121,9 +3121,9 @@ __device__ __forceinline__ int hamming_global_score(const uint8_t* q, const uint
     return hs > 0 ? hs : 0;
 }
 
-// The DP rows of a piece live in shared memory when the piece is at most smem_w - 1
-// columns wide (PW_SMEM_W: small enough that 32 single-warp blocks fit on an SM), else in
-// the block's slice of global scratch.
+// The row between a piece's strips lives in shared memory when the piece is at most
+// smem_w - 1 columns wide (PW_SMEM_W: 4 KB a block, so that 28 single-warp blocks leave the
+// L1 half of the SM's memory), else in the block's slice of global scratch.
 constexpr uint32_t PW_SMEM_W = 512;
 // anchors of a chain that are held in shared memory (longer chains: in the ops scratch)
 constexpr uint32_t PW_SMEM_ANCHORS = 64;
@@ -3527,10 +3527,9 @@ uint32_t run_extension_raw(const DevRefs& refs, const uint8_t* seq, const uint64
         auto a16 = [](uint64_t x) { return (x + 15) & ~(uint64_t)15; };
         const uint64_t cells = a16(pw_dir_bytes(max_qlen, max_pw_window));
         const uint64_t opsb = a16((uint64_t)max_qlen + max_pw_window + 8) + a16(8ull * (max_anchors + 1));
-        // single-warp blocks, 28 per SM (the registers of 28 fit): the per-job work is
-        // mostly serial (anchor pruning, gap checks, traceback pushes, a row at a time), so
-        // more resident warps hide its latency; the rows of wide pieces go to global
-        // scratch so that the shared rows stay small
+        // single-warp blocks, 28 per SM (72 registers; what spills is outside the wavefront's
+        // loop): a job is one serial chain of pieces, so more resident warps hide its latency;
+        // the rows of wide pieces go to global scratch so that the shared rows stay small
         const unsigned blocks = (unsigned)std::min<uint64_t>(n, sm_count() * 28);
         const uint64_t rowsb = a16(8ull * ((uint64_t)max_pw_window + 2));
         ws.pw_scratch.reserve((cells + opsb + rowsb) * blocks);

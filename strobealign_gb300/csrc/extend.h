@@ -76,8 +76,8 @@ struct ExtWorkspace {
     PodArray<ExtResult> h_results;
     PodArray<uint32_t> h_cigar;
     uint64_t total_cigar = 0;
-    // tuning (output-invariant): SSW tasks of reads up to wave_qmax nt (at most 192) run
-    // on the lane-wavefront kernel, longer ones a warp per task
+    // tuning (output-invariant): SSW tasks of reads up to wave_qmax nt run on the
+    // lane-wavefront kernels, longer ones a warp per task; 192: all that k_ssw16 takes
     uint32_t wave_qmax = 192;
     // SW cells: canonical, then computed forward byte / word, reverse byte / word; then
     // banded cells: every pass's, and the final pass's

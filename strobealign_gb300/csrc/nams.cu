@@ -3,9 +3,11 @@
 //
 //   k_seed          warp per read: canonical syncmers + forward / reverse-complement
 //                   randstrobes (src/seeding/{syncmers,strobes,mod}.rs)
-//   k_hits          warp per read: index probes with the repeat filter, global and
-//                   local rescue, orientation choice (src/hit.rs, src/chainer.rs:205-216)
-//   k_anchors       warp per read: anchor count, then fill (src/chainer.rs:304-384)
+//   k_probe         warp per read, a randstrobe per lane: index probes with the repeat
+//                   filter (src/hit.rs)
+//   k_hits          warp per read: hits, global and local rescue, orientation choice
+//                   (src/hit.rs, src/chainer.rs:205-216)
+//   k_anchors       warp per read: anchors counted and written (src/chainer.rs:304-384)
 //   segmented sort  (ref_id, ref_start, query_start) packed in a u64 key
 //   k_chain_long_prep, k_chain_big, k_chain_long   orientations of over 96 anchors, their
 //                   position clusters scored apart, beside k_chain4
