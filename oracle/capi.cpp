@@ -107,6 +107,20 @@ void* ora_index_from_fasta(const char* path, size_t read_length, int32_t bits, d
     return o;
 }
 
+// An index over a given table (sorted) and bucket directory, without reference sequences
+void* ora_index_from_table(size_t read_length, uint32_t bits, size_t filter_cutoff, const uint64_t* table, size_t n,
+                           const uint64_t* buckets) {
+    auto* o = new OraIndex();
+    o->index.params = SeedingParameters::from_read_length(read_length);
+    o->index.bits = (uint8_t)bits;
+    o->index.filter_cutoff = filter_cutoff;
+    for (size_t i = 0; i < n; i++)
+        o->index.randstrobes.push_back(
+            RefRandstrobe{table[2 * i], (uint32_t)table[2 * i + 1], (uint32_t)(table[2 * i + 1] >> 32)});
+    o->index.bucket_starts.assign(buckets, buckets + ((size_t)1 << bits) + 1);
+    return o;
+}
+
 // The same from contigs in memory (ASCII bases), built on `threads` threads;
 // *seconds = the index build time.
 void* ora_index_from_buffers(size_t n, const char* const* names, const char* const* seqs, const size_t* lens,

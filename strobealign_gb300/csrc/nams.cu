@@ -24,6 +24,7 @@
 // intrinsics (no contraction) and log2(d + 1) from a table built with the host's
 // log2f, the function the reference calls.
 #include <cub/cub.cuh>
+#include <type_traits>
 
 #include <cmath>
 #include <mutex>
@@ -1636,21 +1637,19 @@ __device__ __forceinline__ uint32_t orientation_dedup(const uint64_t* sorted, ui
 // reference changes or the position jumps by max_ref_gap or more.  A predecessor scan
 // never crosses into an earlier cluster (the reference's scan breaks there or skips
 // without contributing), so a cluster's DP depends on the others only through the
-// best-index re-check (src/chainer.rs:150-165), which can fire only once the cluster
-// holds the running best, a strict maximum over all earlier anchors.  So the clusters
-// are scored at once, the small ones without the re-check, here, the large ones with
-// their own running best (k_chain_big), and k_chain4 then takes them in order.  A small
-// cluster whose maximum beats the running best of those before it is scored again from
-// the first anchor where the re-check fires; a large one only if it first fired while an
-// earlier cluster still held the running best (a cluster of thousands of anchors would
-// otherwise run its serial DP twice).
+// best-index re-check (src/chainer.rs:150-165), which can change a score only once the
+// cluster holds the running best, a strict maximum over all earlier anchors.  So the
+// clusters are scored at once: the small ones without the re-check, here, the large ones
+// both without it and with their own running best (k_chain_big).  k_chain_long then takes
+// them in order.  A cluster scored without the re-check whose maximum beats the running best
+// of those before it is scored again from the first anchor where the re-check fires
+// (recheck_first_fire); a large one whose own running best was ahead by then has its scores
+// already (a cluster of thousands of anchors would otherwise run its serial DP twice).
 //
 // k_chain_long_prep: a warp per long orientation u: the dedup, the cluster starts
 // (aux[b ..]), and the clusters of up to lane_max anchors scored a thread each (maxima
 // at aux[T + b ..] as floats); the larger ones are queued as (u, cluster) items for
-// k_chain_big, a warp each.  long_n[u] / long_c[u]: anchors after dedup, clusters.
-// k_chain4 checks each small record cluster for the first anchor where the re-check
-// fires (recheck_first_fire) and scores again from there only.
+// k_chain_big, a block each.  long_n[u] / long_c[u]: anchors after dedup, clusters.
 __global__ void __launch_bounds__(128) k_chain_long_prep(const uint64_t* __restrict__ off, const uint64_t* seg_off,
                                                          const uint64_t* seg_count, const uint64_t* sorted, uint64_t* dedup, float* dp,
                                                          uint32_t* pred, uint32_t* aux, uint64_t total_anchors,
@@ -1722,26 +1721,31 @@ struct BigCluster {
 };
 
 // The queued large clusters for max_lookback < 64, a block each (their maxima into
-// aux[T + b + cluster]), with the re-check against the cluster's own running best.  That
-// is the reference's score of every anchor if the best of the clusters before is already
-// beaten when the re-check first changes a score (BigCluster::fire), and in any case up to
-// that anchor; k_chain_long scores the rest again where it is not.
+// aux[T + b + cluster]), scored twice side by side: by the first warp with the re-check
+// against the cluster's own running best (dp, pred), by the second without it (plain: the
+// score's bits, the predecessor).  The first is the reference's score of every anchor if the
+// best of the clusters before is already beaten when the re-check first changes a score
+// (BigCluster::fire), and in any case up to that anchor; otherwise the second is from there
+// on, until the cluster beats that best.  Neither bounds the other: a score that the
+// re-check raised can end the scan of a later anchor on the same diagonal before a better
+// predecessor, so that with it the cluster's maximum is lower.
 //
 // A cluster is one serial chain of anchors and the kernel lasts as long as its longest
-// cluster (a tandem repeat's: thousands of anchors), so what counts is the first warp's
-// instructions from one anchor's score to the next.  The other warps prepare, 32 anchors
+// cluster (a tandem repeat's: thousands of anchors), so what counts is a scoring warp's
+// instructions from one anchor's score to the next.  The other three warps prepare, 32 anchors
 // ahead in shared memory, everything that does not depend on scores: the pair scores
 // (gap, ratio test, chain_score) against the 64 anchors before, and which of them lie on
-// the same diagonal.  The first warp holds those anchors' scores two per lane.
+// the same diagonal.  A scoring warp holds those anchors' scores two per lane.
 //
 // The longest clusters of 53k-read parts on a 310 Mbp human-shaped genome (up to 3,100
 // anchors): 0.34 ms a launch on average, 0.56 at most; with the whole DP in one warp 1.06
-// and 1.69 ms, and 1.1 and 1.9 ms with the predecessors in shared memory.
-constexpr uint32_t BIG_CHUNK = 32;
+// and 1.69 ms, and 1.1 and 1.9 ms with the predecessors in shared memory.  The second scoring
+// costs nothing that shows (200k pairs to PAF 19.0 ms, 19.3 with the first alone).
+constexpr uint32_t BIG_CHUNK = 32, BIG_SCORING = 2, BIG_WARPS = 5;
 
-__global__ void __launch_bounds__(128) k_chain_big(const uint64_t* __restrict__ off, const uint64_t* seg_off,
+__global__ void __launch_bounds__(32 * BIG_WARPS) k_chain_big(const uint64_t* __restrict__ off, const uint64_t* seg_off,
                                                    const uint64_t* __restrict__ dedup, float* dp, uint32_t* pred,
-                                                   uint32_t* aux, uint64_t total_anchors, AnchorPack ap, ChainCtx cc,
+                                                   uint2* plain, uint32_t* aux, uint64_t total_anchors, AnchorPack ap, ChainCtx cc,
                                                    const uint32_t* long_list, const uint32_t* long_n,
                                                    const uint32_t* long_c, const uint32_t* big_items,
                                                    const uint32_t* n_big) {
@@ -1765,9 +1769,9 @@ __global__ void __launch_bounds__(128) k_chain_big(const uint64_t* __restrict__ 
         const uint64_t b = seg_b + lo;  // anchors 0 .. n of the cluster
         const uint32_t read_len = (uint32_t)(off[(sg >> 1) + 1] - off[sg >> 1]);
         const uint32_t max_ref_gap = cc.cp.max_ref_gap ? cc.cp.max_ref_gap : read_len;
-        // pair scores of chunk q's anchors, by warps w0 .. 3
+        // pair scores of chunk q's anchors, by the warps from w0 on
         auto prepare = [&](uint32_t q, uint32_t w0) {
-            for (uint32_t a = w - w0; a < BIG_CHUNK; a += 4 - w0) {
+            for (uint32_t a = w - w0; a < BIG_CHUNK; a += BIG_WARPS - w0) {
                 const uint32_t i = q * BIG_CHUNK + a;
                 if (i >= n) break;
                 const uint64_t ki = s_key[i & 127];
@@ -1804,62 +1808,57 @@ __global__ void __launch_bounds__(128) k_chain_big(const uint64_t* __restrict__ 
         uint64_t best_key = 0;
         float dA = 0.0f, dB = 0.0f;
         const uint32_t chunks = (n + BIG_CHUNK - 1) / BIG_CHUNK;
-        for (uint32_t q = 0; q < chunks; q++) {
-            if (w > 0) {
-                // the keys of chunk q + 2 take the slots of chunk q - 2
-                const uint32_t j = (q + 2) * BIG_CHUNK + lane;
-                uint64_t kn = 0;
-                if (w == 1 && j < n) kn = dedup[b + j];
-                if (q + 1 < chunks) prepare(q + 1, 1);
-                if (w == 1 && j < n) s_key[j & 127] = kn;
-            } else {
-                // Most anchors take the nearest candidate on their diagonal.  Its score dj
-                // is fetched an anchor ahead (it is the last one's only for distance 0), so
-                // that path needs one addition, one comparison and one vote from the last
-                // anchor's score to this one's.
-                const uint32_t i0 = q * BIG_CHUNK, m = n - i0 < BIG_CHUNK ? n - i0 : BIG_CHUNK;
-                const bool high = q & 1;
-                float sA = s_pair[q & 1][0][lane], sB = s_pair[q & 1][0][lane + 32];
-                uint2 near = s_near[q & 1][0];
-                uint2 pos = s_pos[q & 1][0];
-                uint32_t slot = (i0 - 1 - near.x) & 63;
-                float dj = __shfl_sync(FULL, slot & 32 ? dB : dA, slot & 31);
-                uint32_t my_pred = 0xffffffffu;
-                for (uint32_t a = 0; a < m; a++) {
-                    const uint32_t i = i0 + a;
-                    const float v0 = __fadd_rn(dj, __uint_as_float(near.y));  // -inf without one
-                    const float vA = __fadd_rn(dA, sA), vB = __fadd_rn(dB, sB);
-                    const uint32_t t0 = near.x;
-                    const uint2 here = pos;
-                    const uint32_t a1 = a + 1 < m ? a + 1 : a;
-                    sA = s_pair[q & 1][a1][lane];
-                    sB = s_pair[q & 1][a1][lane + 32];
-                    near = s_near[q & 1][a1];
-                    pos = s_pos[q & 1][a1];
-                    slot = (i - near.x) & 63;
-                    dj = __shfl_sync(FULL, slot & 32 ? dB : dA, slot & 31);
-                    // the re-check's score needs only the best before
-                    float cur = v0, ns = 0.0f;
-                    uint32_t cur_pred = i - 1 - t0;
-                    const bool again = here.x - best_pos < max_ref_gap && best_index != 0xffffffffu &&
-                                       recheck_score(s_key[i & 127], here.x, here.y, best_key, best_score, max_ref_gap,
-                                                     cc, ap, ns);
-                    if (__any_sync(FULL, vA > v0 || vB > v0) || !(v0 >= kf))
-                        scan_outcome(i, vA, vB, s_diag[q & 1][a], kf, cur, cur_pred);
-                    if (again && ns > cur) {
-                        cur = ns;
-                        cur_pred = best_index;
-                        if (fire == 0xffffffffu) {
-                            fire = i;
-                            fire_best = best_score;
-                        }
+        // Chunk q's scores.  Most anchors take the nearest candidate on their diagonal.  Its
+        // score dj is fetched an anchor ahead (it is the last one's only for distance 0), so
+        // that path needs one addition, one comparison and one vote from the last anchor's
+        // score to this one's.
+        auto score = [&](auto recheck, uint32_t q, uint32_t m) -> uint32_t {
+            const uint32_t i0 = q * BIG_CHUNK;
+            const bool high = q & 1;
+            float sA = s_pair[q & 1][0][lane], sB = s_pair[q & 1][0][lane + 32];
+            uint2 near = s_near[q & 1][0];
+            uint2 pos = s_pos[q & 1][0];
+            uint32_t slot = (i0 - 1 - near.x) & 63;
+            float dj = __shfl_sync(FULL, slot & 32 ? dB : dA, slot & 31);
+            uint32_t my_pred = 0xffffffffu;
+            for (uint32_t a = 0; a < m; a++) {
+                const uint32_t i = i0 + a;
+                const float v0 = __fadd_rn(dj, __uint_as_float(near.y));  // -inf without one
+                const float vA = __fadd_rn(dA, sA), vB = __fadd_rn(dB, sB);
+                const uint32_t t0 = near.x;
+                const uint2 here = pos;
+                const uint32_t a1 = a + 1 < m ? a + 1 : a;
+                sA = s_pair[q & 1][a1][lane];
+                sB = s_pair[q & 1][a1][lane + 32];
+                near = s_near[q & 1][a1];
+                pos = s_pos[q & 1][a1];
+                slot = (i - near.x) & 63;
+                dj = __shfl_sync(FULL, slot & 32 ? dB : dA, slot & 31);
+                float cur = v0, ns = 0.0f;
+                uint32_t cur_pred = i - 1 - t0;
+                bool again = false;
+                // the re-check's score needs only the best before
+                if constexpr (decltype(recheck)::value)
+                    again = here.x - best_pos < max_ref_gap && best_index != 0xffffffffu &&
+                            recheck_score(s_key[i & 127], here.x, here.y, best_key, best_score, max_ref_gap, cc, ap,
+                                          ns);
+                if (__any_sync(FULL, vA > v0 || vB > v0) || !(v0 >= kf))
+                    scan_outcome(i, vA, vB, s_diag[q & 1][a], kf, cur, cur_pred);
+                if (again && ns > cur) {
+                    cur = ns;
+                    cur_pred = best_index;
+                    if (fire == 0xffffffffu) {
+                        fire = i;
+                        fire_best = best_score;
                     }
-                    if (lane == a) {
-                        if (high) dB = cur;
-                        else dA = cur;
-                        my_pred = cur_pred == 0xffffffffu ? cur_pred : lo + cur_pred;
-                    }
-                    if (near.x == 0) dj = cur;
+                }
+                if (lane == a) {
+                    if (high) dB = cur;
+                    else dA = cur;
+                    my_pred = cur_pred == 0xffffffffu ? cur_pred : lo + cur_pred;
+                }
+                if (near.x == 0) dj = cur;
+                if constexpr (decltype(recheck)::value) {
                     if (cur > best_score) {
                         best_score = cur;
                         best_index = i;
@@ -1867,10 +1866,27 @@ __global__ void __launch_bounds__(128) k_chain_big(const uint64_t* __restrict__ 
                         best_key = s_key[i & 127];
                     }
                 }
+            }
+            return my_pred;
+        };
+        for (uint32_t q = 0; q < chunks; q++) {
+            const uint32_t i0 = q * BIG_CHUNK, m = n - i0 < BIG_CHUNK ? n - i0 : BIG_CHUNK;
+            if (w >= BIG_SCORING) {
+                // the keys of chunk q + 2 take the slots of chunk q - 2
+                const uint32_t j = (q + 2) * BIG_CHUNK + lane;
+                uint64_t kn = 0;
+                if (w == BIG_SCORING && j < n) kn = dedup[b + j];
+                if (q + 1 < chunks) prepare(q + 1, BIG_SCORING);
+                if (w == BIG_SCORING && j < n) s_key[j & 127] = kn;
+            } else if (w == 0) {
+                const uint32_t my_pred = score(std::true_type{}, q, m);
                 if (lane < m) {
-                    dp[b + i0 + lane] = high ? dB : dA;
+                    dp[b + i0 + lane] = q & 1 ? dB : dA;
                     pred[b + i0 + lane] = my_pred;
                 }
+            } else {
+                const uint32_t my_pred = score(std::false_type{}, q, m);
+                if (lane < m) plain[b + i0 + lane] = make_uint2(__float_as_uint(q & 1 ? dB : dA), my_pred);
             }
             __syncthreads();
         }
@@ -1913,15 +1929,15 @@ __global__ void __launch_bounds__(128) k_chain_big_far(const uint64_t* __restric
 }
 
 // A long orientation per warp, its clusters scored by k_chain_long_prep (without the
-// re-check) and k_chain_big: in order, the clusters whose maximum beats the running best,
-// then the chains.  A kernel apart from k_chain4: the rings there take the shared memory
+// re-check) and k_chain_big: in order, the clusters whose maximum beats the running best
+// and those whose own re-check changed a score, then the chains.  A kernel apart from k_chain4: the rings there take the shared memory
 // that the L1 needs here (the walks are chains of dependent loads; 300-500 cycles an
 // anchor from L2).
 template <bool RING>
 __global__ void __launch_bounds__(128) k_chain_long(const uint64_t* __restrict__ off, const uint64_t* seg_off,
                                                     uint64_t* dedup, float* dp, uint32_t* pred, uint32_t* aux,
-                                                    uint64_t total_anchors, unsigned long long* scratch, AnchorPack ap,
-                                                    ChainCtx cc, NamRec* nam_out, uint32_t* nam_seg_count, uint64_t* anc_out,
+                                                    uint64_t total_anchors, unsigned long long* scratch,
+                                                    const uint2* plain, AnchorPack ap, ChainCtx cc, NamRec* nam_out, uint32_t* nam_seg_count, uint64_t* anc_out,
                                                     uint64_t* anc_start, const uint32_t* long_list, uint32_t n_long,
                                                     const uint32_t* long_n, const uint32_t* long_c,
                                                     uint32_t lane_max) {
@@ -1949,11 +1965,8 @@ __global__ void __launch_bounds__(128) k_chain_long(const uint64_t* __restrict__
             const uint32_t my_fire = my_big ? info[my_lo + 1] : NONE;
             uint32_t from = 0;
             for (;;) {
-                // a cluster that its own re-check changed counts up to the score
-                // that a chain's end needs: below it, its anchors are in no chain
-                const bool rec = c < C && lane >= from &&
-                                 (best_index == NONE || m > best_score ||
-                                  (my_fire != NONE && !(m < __fmul_rn(best_score, cc.cp.valid_score_threshold))));
+                const bool rec =
+                    c < C && lane >= from && (best_index == NONE || m > best_score || my_fire != NONE);
                 const uint32_t bal = __ballot_sync(FULL, rec);
                 if (!bal) break;
                 const uint32_t l = __ffs(bal) - 1;
@@ -1972,12 +1985,20 @@ __global__ void __launch_bounds__(128) k_chain_long(const uint64_t* __restrict__
                         }
                         continue;
                     }
+                    // an earlier cluster held the running best when the re-check fired: from
+                    // there on the scores are those without it
+                    for (uint32_t i = i0 + lane; i < hi; i += 32) {
+                        const uint2 s = plain[b + i];
+                        dp[b + i] = __uint_as_float(s.x);
+                        pred[b + i] = s.y;
+                    }
+                    __syncwarp();
                 } else {
-                    // the values scored without the re-check stand up to the first
-                    // anchor where it would fire; only the rest is scored again
-                    i0 = recheck_first_fire(dedup, dp, b, lo, hi, max_ref_gap, cc, ap, best_score, best_index,
-                                            best_key);
+                    i0 = lo;
                 }
+                // the values scored without the re-check stand up to the first anchor
+                // where it would fire; only the rest is scored again
+                i0 = recheck_first_fire(dedup, dp, b, i0, hi, max_ref_gap, cc, ap, best_score, best_index, best_key);
                 if (i0 < hi) {
                     if (RING)
                         warp_chain_regs(dedup, dp, pred, b, i0, hi, lo, max_ref_gap, cc, ap, best_score, best_index,
@@ -2519,13 +2540,21 @@ uint32_t run_nam_pipeline(const DevIndex& ix, const DevRefs& refs, const NamConf
                                                  ws.pred.p, ws.aux.p, total_anchors, ap, cc, long_sorted, n_list[2],
                                                  long_n, long_c, ws.chain_big.p + 2, ws.chain_big.p, lane_max);
         const unsigned bgrid = (unsigned)(sm_count() * 8);
-        (ring ? k_chain_big : k_chain_big_far)<<<bgrid, 128, 0, sl>>>(
-            ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p, total_anchors, ap, cc, long_sorted,
-            long_n, long_c, ws.chain_big.p + 2, ws.chain_big.p);
+        // the sorted anchors have been copied out: their room for the scores without the
+        // re-check, then for the extraction
+        uint2* const plain = reinterpret_cast<uint2*>(ws.anchors_sorted.p);
+        if (ring)
+            k_chain_big<<<bgrid, 32 * BIG_WARPS, 0, sl>>>(ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p,
+                                                          plain, ws.aux.p, total_anchors, ap, cc, long_sorted, long_n,
+                                                          long_c, ws.chain_big.p + 2, ws.chain_big.p);
+        else
+            k_chain_big_far<<<bgrid, 128, 0, sl>>>(ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p,
+                                                   total_anchors, ap, cc, long_sorted, long_n, long_c,
+                                                   ws.chain_big.p + 2, ws.chain_big.p);
         (ring ? k_chain_long<true> : k_chain_long<false>)<<<pgrid, 128, 0, sl>>>(
             ws.off.p, ws.seg_off.p, ws.anchors.p, ws.dp.p, ws.pred.p, ws.aux.p, total_anchors,
-            reinterpret_cast<unsigned long long*>(ws.anchors_sorted.p), ap, cc, ws.nam_scratch.p, ws.nam_seg_count.p,
-            anc_out, anc_start, long_sorted, n_list[2], long_n, long_c, lane_max);
+            reinterpret_cast<unsigned long long*>(ws.anchors_sorted.p), plain, ap, cc, ws.nam_scratch.p,
+            ws.nam_seg_count.p, anc_out, anc_start, long_sorted, n_list[2], long_n, long_c, lane_max);
         launches += 3;
     }
     if (n_list[0]) {

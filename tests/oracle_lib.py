@@ -57,6 +57,8 @@ def oracle() -> C.CDLL:
                                     C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]
     lib.ora_index_from_fasta.restype = C.c_void_p
     lib.ora_index_from_fasta.argtypes = [C.c_char_p, C.c_size_t, C.c_int32, C.c_double]
+    lib.ora_index_from_table.restype = C.c_void_p
+    lib.ora_index_from_table.argtypes = [C.c_size_t, C.c_uint32, C.c_size_t, C.c_void_p, C.c_size_t, C.c_void_p]
     lib.ora_index_free.argtypes = [C.c_void_p]
     lib.ora_index_info.argtypes = [C.c_void_p, C.POINTER(C.c_uint64)]
     lib.ora_index_arrays.argtypes = [C.c_void_p, C.c_void_p, C.POINTER(C.c_uint64)]
@@ -153,6 +155,16 @@ class OracleIndex:
         self.lib = oracle()
         self.h = self.lib.ora_index_from_fasta(str(fasta).encode(), read_length, bits, filter_fraction)
         assert self.h
+
+    @classmethod
+    def from_table(cls, read_length: int, bits: int, filter_cutoff: int, table: np.ndarray, buckets: np.ndarray):
+        """An index over a given sorted table (16-byte entries) and its bucket directory."""
+        o = cls.__new__(cls)
+        o.lib = oracle()
+        table, buckets = np.ascontiguousarray(table), np.ascontiguousarray(buckets, np.uint64)
+        o.h = o.lib.ora_index_from_table(read_length, bits, filter_cutoff, table.ctypes.data, len(table),
+                                         buckets.ctypes.data)
+        return o
 
     def info(self):
         o = (C.c_uint64 * 3)()
