@@ -7,7 +7,9 @@ uint32_t ssw16_max_qlen(const AlignScores& sc) {
     if (sc.match == 0 || sc.match > 16 || sc.mismatch > 64 || sc.gap_open <= sc.gap_extend || sc.gap_extend > 31 ||
         sc.gap_extend > 8 * sc.match)
         return 0;
-    return std::min<uint32_t>(SSW16_MAX_QLEN, 1022u / sc.match);
+    // a lane of ceil(L / 8) rows
+    const uint32_t by_raise = sc.gap_extend ? 8 * (1024u / sc.gap_extend) : SSW16_MAX_QLEN;
+    return std::min({SSW16_MAX_QLEN, 1022u / sc.match, by_raise});
 }
 
 void launch_ssw16(const Ssw16Args& a, uint32_t longest) {

@@ -25,11 +25,13 @@ struct Ssw16Args {
 };
 
 // The longest read whose scores fit (0: these scores do not).  Scores are scaled by 32 in
-// 16 bits: match * L <= 1022 keeps every H with its row key below 2^15.  The other limits
-// keep the raise's row offsets (gap_extend <= 31, and no more than a lane's rows add
-// to the score) and a word pass's first lane of two rows or more (a byte pass overflows at
-// 255 - mismatch, which takes 12 rows or more) within what the kernel assumes; the
-// lazy-F raise is exact for gap_open > gap_extend.
+// 16 bits: match * L <= 1022 keeps every H with its row key below 2^15, and
+// gap_extend * ceil(L / 8) <= 1024 the raise above -2^15, which a word pass takes through a
+// lane's two pieces from 0 on (match 3, extension 24: reads up to 336 of the 340 nt that the
+// scores allow).  The other limits keep the raise's row offsets (gap_extend <= 31, and no
+// more than a lane's rows add to the score) and a word pass's first lane of two rows or more
+// (a byte pass overflows at 255 - mismatch, which takes 12 rows or more) within what the
+// kernel assumes; the lazy-F raise is exact for gap_open > gap_extend.
 uint32_t ssw16_max_qlen(const AlignScores& sc);
 
 // The end searches of every task of a read up to a.qmax nt; longest: the longest such read.
