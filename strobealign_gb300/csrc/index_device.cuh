@@ -120,10 +120,12 @@ __device__ __forceinline__ uint32_t idx_count_full(const DevIndex& ix, uint64_t 
 // rounds and fewer sectors: a bucket of up to 8 entries is read with independent loads
 // instead of a binary search (the lower bound is the number of smaller keys), larger ones
 // narrow 8-ary; a hash's repeat test looks first at the entry after it, which those
-// loads hold (the table is sorted: no equal neighbour, no run of `cutoff`), and the reverse
-// complement is looked up only for hashes that are there.  Random 32-byte sectors bound
-// the lookups: 1.4 M reads of 150 nt on a 310 Mbp human-shaped index took 5.1 ms with both
-// orientations and the entries a cutoff further read for every hash, 3.8 ms now.
+// loads hold (the table is sorted: no equal neighbour, no run of `cutoff`; a bucket's last
+// entry has its neighbour in the next bucket, where only a partial lookup's run can go on, and
+// only under a mask shorter than the bucket number), and the reverse complement is looked
+// up only for hashes that are there.  Random 32-byte sectors bound the lookups: 1.4 M reads
+// of 150 nt on a 310 Mbp human-shaped index took 5.1 ms with both orientations and the
+// entries a cutoff further read for every hash, 3.8 ms now.
 // bucket range [ps, pe) of a full hash (same directory reads as idx_get_masked_from)
 __device__ __forceinline__ void idx_bucket(const DevIndex& ix, uint64_t hash, uint64_t& ps, uint64_t& pe) {
     const uint64_t top = hash >> (64 - ix.bits);
@@ -231,6 +233,9 @@ __device__ __forceinline__ void idx_full_probe(const DevIndex& ix, uint64_t h, u
             const uint32_t at = idx_find8(e, len, h & mask, mask, next_eq);
             if (at == len) return;
             pos = start + at;
+            // a mask that leaves out leading bits of the bucket number: the run goes on in
+            // the next bucket
+            if (at + 1 == len && (~mask >> (64 - ix.bits)) != 0) next_eq = true;
         } else {
             pos = idx_get_masked_from(ix, h, mask, false, 0);
             if (pos == UINT64_MAX) return;
