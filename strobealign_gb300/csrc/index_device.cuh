@@ -224,6 +224,7 @@ __device__ __forceinline__ void idx_full_probe(const DevIndex& ix, uint64_t h, u
     uint32_t len;
     bool many, whole;
     filtered = found_partial = false;
+    const bool always = cutoff == 0;  // an entry is then too frequent by itself
     pos = idx_lookup8(ix, h, many, e, start, len, whole);
     if (pos == UINT64_MAX) {
         if (!partial) return;
@@ -241,18 +242,18 @@ __device__ __forceinline__ void idx_full_probe(const DevIndex& ix, uint64_t h, u
             if (pos == UINT64_MAX) return;
         }
         found_partial = true;
-        filtered = next_eq && idx_too_frequent_partial(ix, pos, cutoff);
+        filtered = (next_eq || always) && idx_too_frequent_partial(ix, pos, cutoff);
         return;
     }
     // is_too_frequent: either orientation's run reaches the cutoff, or both together pass it
-    if (many && idx_too_frequent_forward(ix, pos, cutoff)) {
+    if ((many || always) && idx_too_frequent_forward(ix, pos, cutoff)) {
         filtered = true;
         return;
     }
     bool many_rc;
     const uint64_t rc = idx_lookup8(ix, hrc, many_rc, e, start, len, whole);
     if (rc == UINT64_MAX) return;
-    if (many_rc && idx_too_frequent_forward(ix, rc, cutoff)) {
+    if ((many_rc || always) && idx_too_frequent_forward(ix, rc, cutoff)) {
         filtered = true;
         return;
     }

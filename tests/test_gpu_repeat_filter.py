@@ -1,8 +1,8 @@
 """The repeat filter of full and partial lookups (src/index.rs:298-337) at the edges that
 a look at the neighbouring entry does not settle: a main hash mask with fewer leading bits
 than the bucket directory (a run of equal masked hashes then goes on in the next bucket),
-and a filter cutoff of 1 (as an index file may have it).  Counts per read equal a
-restatement over the table."""
+and filter cutoffs of 0 and 1 (as an index file may have them; 0 filters every hash that
+is not one of the table's last).  Counts per read equal a restatement over the table."""
 import numpy as np
 import pytest
 
@@ -57,7 +57,7 @@ def _counts(hashes, mask, bits, cutoff, rs):
 
 @pytest.mark.parametrize("mask_bits,bits,cutoff", [
     (8, 8, None), (8, 9, None), (8, 12, None), (8, 16, None), (12, 14, 1), (0, 12, None),
-    (0, 12, 1), (8, 12, 1)])
+    (0, 12, 1), (8, 12, 1), (0, 12, 0), (8, 12, 0)])
 def test_filtered_counts(mask_bits, bits, cutoff, tmp_path):
     import strobealign_gb300 as sa
     from strobealign_gb300 import synthetic as syn
@@ -85,6 +85,7 @@ def test_filtered_counts(mask_bits, bits, cutoff, tmp_path):
                        for o in (fwd, rc)], axis=0)
         assert [int(det[n][i]) for n in names] == want.tolist(), i
         total += want
-    assert total[0] and total[2] and total[5], total
+    found = 1 if cutoff == 0 else 2
+    assert total[0] and total[found] and total[found + 3], total
     if mask_bits:
         assert total[4], total
