@@ -252,8 +252,9 @@ void Mapper::prepare(const sa_read_batch* r1, const sa_read_batch* r2) {
     bv_ = BatchView();
     bv_.paired = paired;
     rec_read_.clear();
-    const uint64_t n = r1->n, o1 = r1->seq_offsets[0], o2 = paired ? r2->seq_offsets[0] : 0;
-    const uint64_t total = r1->seq_offsets[n] - o1 + (paired ? r2->seq_offsets[n] - o2 : 0);
+    // a batch of no reads may come without arrays
+    const uint64_t n = r1->n, o1 = n ? r1->seq_offsets[0] : 0, o2 = n && paired ? r2->seq_offsets[0] : 0;
+    const uint64_t total = n ? r1->seq_offsets[n] - o1 + (paired ? r2->seq_offsets[n] - o2 : 0) : 0;
     prepare_reads(n, paired ? 2 : 1, total, [&](uint64_t i) {
         const uint64_t l1 = r1->seq_offsets[i + 1] - r1->seq_offsets[i];
         if (!paired) {
@@ -276,8 +277,8 @@ void Mapper::prepare_interleaved(const sa_read_batch* reads) {
     bv_ = BatchView();
     pair_records_by_name(*reads, true, rec_read_);
     bv_.rec_read = rec_read_.data();
-    const uint64_t o = reads->seq_offsets[0];
-    prepare_reads(n, 1, reads->seq_offsets[n] - o, [&](uint64_t i) {
+    const uint64_t o = n ? reads->seq_offsets[0] : 0;
+    prepare_reads(n, 1, n ? reads->seq_offsets[n] - o : 0, [&](uint64_t i) {
         reads_[i] = read_view(reads, i);
         h_off_.p[i] = reads->seq_offsets[i] - o;
         return (uint64_t)(reads->seq_offsets[i + 1] - reads->seq_offsets[i]);
