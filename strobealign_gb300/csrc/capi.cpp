@@ -294,8 +294,8 @@ int32_t sa_index_read_sti(const char* path, const sa_seeding_params* p, int32_t 
     idx->bits = sbits;
     idx->filter_cutoff = cutoff;
     idx->n = n;
-    idx->rs.reserve(n);
-    idx->buckets.reserve(nb);
+    idx->rs.reserve(n, true);
+    idx->buckets.reserve(nb, true);
     if (n) SA_CUDA(cudaMemcpy(idx->rs.p, rs.data(), n * 16, cudaMemcpyHostToDevice));
     SA_CUDA(cudaMemcpy(idx->buckets.p, bs.data(), nb * 8, cudaMemcpyHostToDevice));
     finish_index(idx.get());

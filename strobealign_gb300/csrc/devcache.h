@@ -34,16 +34,21 @@ public:
     DevCache(const DevCache&) = delete;
     DevCache& operator=(const DevCache&) = delete;
 
-    void* alloc(size_t bytes) {
+    // exact: for a buffer that stays (an index, a read arena): a block of its own size.
+    // Others may get a quarter more (or 64 KB), so that calls of nearly one size share blocks.
+    void* alloc(size_t bytes, bool exact = false) {
         DevPlace at;
         if (!be_.place(at)) return be_.alloc(bytes);
-        const size_t size = round_size(bytes);
+        size_t size = round_to_512(bytes);
         {
             std::lock_guard<std::mutex> g(mu_);
             Pool& pool = pool_of(at);
+            // a block that is too large to be kept is not rounded up either
+            if (!exact && round_size(bytes) <= pool.bound) size = round_size(bytes);
+            const size_t most = exact ? size : size + (size / 4 > SLACK_MIN ? size / 4 : SLACK_MIN);
             size_t best = pool.free.size();
             for (size_t i = 0; i < pool.free.size(); i++)
-                if (pool.free[i].size >= size && pool.free[i].size <= 2 * size &&
+                if (pool.free[i].size >= size && pool.free[i].size <= most &&
                     (best == pool.free.size() || pool.free[i].size < pool.free[best].size))
                     best = i;
             if (best < pool.free.size()) {
@@ -81,10 +86,6 @@ public:
         }
         std::lock_guard<std::mutex> g(mu_);
         Pool& pool = pool_of(at);
-        if (!pool.bound_known) {
-            pool.bound = be_.keep_bound();
-            pool.bound_known = true;
-        }
         if (l.size > pool.bound) {
             be_.free(p);
             return;
@@ -106,17 +107,20 @@ public:
     // bytes kept at a place; blocks handed out that may be kept, of all places
     size_t kept(const DevPlace& at) {
         std::lock_guard<std::mutex> g(mu_);
-        return pool_of(at).kept;
+        for (const Pool& p : pools_)
+            if (p.at == at) return p.kept;
+        return 0;
     }
     size_t live() {
         std::lock_guard<std::mutex> g(mu_);
         return live_.size();
     }
 
-    // Sizes in steps of an eighth of a power of two, so that calls of nearly one size share
-    // blocks.
+    static constexpr size_t SLACK_MIN = 64 << 10;
+    static size_t round_to_512(size_t n) { return (n + 511) / 512 * 512; }
+    // sizes in steps of an eighth of a power of two
     static size_t round_size(size_t n) {
-        if (n <= 4096) return (n + 511) / 512 * 512;
+        if (n <= 4096) return round_to_512(n);
         size_t step = 512;
         while (step * 16 < n) step *= 2;
         return (n + step - 1) / step * step;
@@ -133,7 +137,6 @@ private:
     };
     struct Pool {
         DevPlace at;
-        bool bound_known = false;
         size_t bound = 0, kept = 0;
         std::vector<Block> free;  // oldest first
         Block take(size_t i) {
@@ -143,11 +146,12 @@ private:
             return b;
         }
     };
-    Pool& pool_of(const DevPlace& at) {
+    Pool& pool_of(const DevPlace& at) {  // of the current place
         for (Pool& p : pools_)
             if (p.at == at) return p;
         pools_.emplace_back();
         pools_.back().at = at;
+        pools_.back().bound = be_.keep_bound();
         return pools_.back();
     }
 

@@ -67,7 +67,7 @@ DevCache& cache() {
 
 }  // namespace
 
-void* dev_alloc(size_t bytes) { return cache().alloc(bytes); }
+void* dev_alloc(size_t bytes, bool exact) { return cache().alloc(bytes, exact); }
 void dev_free(void* p) { cache().free(p); }
 void dev_trim() { cache().trim(); }
 

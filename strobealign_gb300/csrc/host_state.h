@@ -60,8 +60,9 @@ inline uint64_t sm_count() {
 }
 
 // Device memory from a bounded cache of freed blocks (devmem.cpp); null when there is none.
-// dev_free waits for the device, as cudaFree does; dev_trim gives the cache back.
-void* dev_alloc(size_t bytes);
+// exact: no larger block than that.  dev_free waits for the device, as cudaFree does;
+// dev_trim gives the cache back.
+void* dev_alloc(size_t bytes, bool exact = false);
 void dev_free(void* p);
 void dev_trim();
 
@@ -79,12 +80,13 @@ struct DevBuf {
         p = nullptr;
         n = 0;
     }
-    // grow-only reallocation; contents are not preserved
-    void reserve(size_t count) {
+    // grow-only reallocation; contents are not preserved.  exact: for buffers that stay for
+    // the life of an index, a mapper or a session
+    void reserve(size_t count, bool exact = false) {
         if (count <= n && p) return;
         release();
         size_t c = std::max<size_t>(count, 1);
-        p = static_cast<T*>(dev_alloc(c * sizeof(T)));
+        p = static_cast<T*>(dev_alloc(c * sizeof(T), exact));
         if (!p) throw Error(SA_ERR_OOM, "cudaMalloc of " + std::to_string(c * sizeof(T)) + " bytes failed");
         n = c;
     }

@@ -309,7 +309,7 @@ void build_index_gpu(const std::vector<Contig>& contigs, const SeedParams& sp, u
     if (nsy) k_syncmer_info<<<grid_for(nsy, 256), 256, 0, st>>>(d_words.p, d_woff.p, d_cstart.p, nc, d_gpos.p, d_count.p, sp, d_sy.p);
     d_gpos.release();
     DevBuf<RefRandstrobe> d_unsorted;
-    d_unsorted.reserve(nsy);
+    d_unsorted.reserve(nsy, true);
     if (nsy) k_ref_randstrobes<<<grid_for(nsy, 256), 256, 0, st>>>(d_sy.p, d_count.p, sp, d_unsorted.p);
     SA_CUDA(cudaStreamSynchronize(st));
     SA_CUDA(cudaGetLastError());
@@ -320,7 +320,7 @@ void build_index_gpu(const std::vector<Contig>& contigs, const SeedParams& sp, u
     // bits that the longest contig has: 11 passes of 8 bits for contigs below 2^24 nt
     // and 8 for one contig, of the 16 that the whole 128-bit key takes (240 us each for
     // 20 M entries: 2.66 ms of passes for 24 contigs, 3.68 ms before).
-    idx.rs.reserve(nsy);
+    idx.rs.reserve(nsy, true);
     if (nsy) {
         uint32_t max_len = 0;
         for (uint32_t c = 0; c < nc; c++) max_len = std::max(max_len, clen[c]);
@@ -345,7 +345,7 @@ void build_index_gpu(const std::vector<Contig>& contigs, const SeedParams& sp, u
     d_unsorted.release();
     // (5) bucket directory and filter cutoff
     uint64_t nb = (1ULL << bits) + 1;
-    idx.buckets.reserve(nb);
+    idx.buckets.reserve(nb, true);
     DevBuf<unsigned long long> d_hist;  // the histogram, then the two extents
     d_hist.reserve(104);
     SA_CUDA(cudaMemsetAsync(d_hist.p, 0, 104 * 8, st));

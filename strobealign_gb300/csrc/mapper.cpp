@@ -56,9 +56,9 @@ Mapper::Mapper(const sa_index* idx, const sa_refs* refs, const sa_chaining_param
     }
     std::vector<uint64_t> hw(nw, 0);
     for (uint32_t c = 0; c < nc; c++) std::copy(cs[c].words.begin(), cs[c].words.end(), hw.begin() + woff[c]);
-    d_words_.reserve(nw);
-    d_woff_.reserve(nc);
-    d_clen_.reserve(nc);
+    d_words_.reserve(nw, true);
+    d_woff_.reserve(nc, true);
+    d_clen_.reserve(nc, true);
     SA_CUDA(cudaMemcpy(d_words_.p, hw.data(), nw * 8, cudaMemcpyHostToDevice));
     SA_CUDA(cudaMemcpy(d_woff_.p, woff.data(), nc * 8, cudaMemcpyHostToDevice));
     SA_CUDA(cudaMemcpy(d_clen_.p, clen.data(), nc * 4, cudaMemcpyHostToDevice));

@@ -96,9 +96,9 @@ Session::Session(const sa_index* idx, const sa_refs* refs, const sa_chaining_par
     }
     std::vector<uint64_t> hw(nw, 0);
     for (uint32_t c = 0; c < nc; c++) std::copy(cs[c].words.begin(), cs[c].words.end(), hw.begin() + woff[c]);
-    d_words_.reserve(std::max<uint64_t>(nw, 1));
-    d_woff_.reserve(std::max<uint32_t>(nc, 1));
-    d_clen_.reserve(std::max<uint32_t>(nc, 1));
+    d_words_.reserve(std::max<uint64_t>(nw, 1), true);
+    d_woff_.reserve(std::max<uint32_t>(nc, 1), true);
+    d_clen_.reserve(std::max<uint32_t>(nc, 1), true);
     if (nw) SA_CUDA(cudaMemcpy(d_words_.p, hw.data(), nw * 8, cudaMemcpyHostToDevice));
     if (nc) {
         SA_CUDA(cudaMemcpy(d_woff_.p, woff.data(), nc * 8, cudaMemcpyHostToDevice));
@@ -122,8 +122,8 @@ Session::Session(const sa_index* idx, const sa_refs* refs, const sa_chaining_par
         cfg_.max_inflight_bases = std::min<uint64_t>(1ull << 33, std::max<uint64_t>(1ull << 24, usable / 8));
     }
     const uint64_t slots = cfg_.max_inflight_bases / 32 + 65536;
-    arena_seq_.reserve(cfg_.max_inflight_bases + 16);
-    arena_off_.reserve(slots);
+    arena_seq_.reserve(cfg_.max_inflight_bases + 16, true);
+    arena_off_.reserve(slots, true);
     seq_alloc_.reset(cfg_.max_inflight_bases);
     off_alloc_.reset(slots);
     unsigned nt = cfg_.policy_threads ? cfg_.policy_threads : std::max(1u, std::thread::hardware_concurrency());

@@ -22,7 +22,7 @@ struct Fake : DevBackend {
     };
     DevPlace now;
     bool known = true;
-    size_t bound[2] = {40000, 100000}, capacity = 1 << 20;
+    size_t bound[2] = {40000, 900000}, capacity = 4 << 20;
     std::map<void*, Owned> owned;
     std::map<int, size_t> used;
     uintptr_t next = 0x1000;
@@ -67,14 +67,20 @@ int main() {
         f.known = !untold;
         if (rng() % 2 && held.size() < 60) {
             // up to beyond either bound
-            const size_t bytes = 1 + rng() % (rng() % 20 ? 9000 : 120000);
+            const size_t bytes = 1 + rng() % (rng() % 20 ? 9000 : 500000);
             const uintptr_t before = f.next;
-            void* p = c.alloc(bytes);
+            const bool exact = rng() % 3 == 0;
+            void* p = c.alloc(bytes, exact);
             if (p) {
                 reused += f.next == before;
                 check(f.owned.count(p) == 1, "a block that is handed out is allocated");
                 check(f.owned[p].at == places[x], "a block serves its own place");
-                check(f.owned[p].bytes >= bytes, "a block is large enough");
+                const size_t size = f.owned[p].bytes;
+                check(size >= bytes, "a block is large enough");
+                if (exact) check(size < bytes + 512, "a block that stays is no larger than asked for");
+                else check(size <= DevCache::round_size(bytes) * 5 / 4 ||
+                               size <= DevCache::round_size(bytes) + DevCache::SLACK_MIN,
+                           "a block is not much larger than asked for");
                 for (const Held& h : held) check(h.p != p, "a block is handed out once");
                 held.push_back(Held{p, bytes, x});
             }
