@@ -42,6 +42,16 @@ const char* sa_last_error(void);
 /* Library version string. */
 const char* sa_version(void);
 
+/* ---------------------------------------------------------------- device memory
+ * The library keeps device blocks that it has freed for its next calls on the same device
+ * and context: at most 8 GiB and a 32nd of the device's memory (8 GiB of a GB300's), also
+ * once every handle is freed.  It gives them back itself when one of its own allocations
+ * fails and when a session looks for free memory; other allocators of the process do not
+ * see them as free.  sa_device_trim gives back what is kept for the current device and
+ * context; *released (may be NULL) is its size in bytes.  It may be called at any time, from
+ * any thread; buffers in use stay. */
+int32_t sa_device_trim(uint64_t* released);
+
 /* ---------------------------------------------------------------- parameters */
 /* SeedingParameters (src/seeding/parameters.rs:164-171; presets :102-159). */
 typedef struct {

@@ -719,6 +719,14 @@ class Session:
         self.close()
 
 
+def device_trim() -> int:
+    """sa_device_trim: gives back the freed device blocks that the library keeps for its next
+    calls on the current device; their bytes."""
+    n = C.c_uint64()
+    L.check(lib().sa_device_trim(C.byref(n)))
+    return n.value
+
+
 def measure_int_alu() -> dict:
     """sa_measure_int_alu: the device's integer instruction rates (per second)."""
     out = (C.c_double * 2)()

@@ -138,6 +138,7 @@ SIGNATURES = {
     "sa_session_get_info": (i32, [vp, P(SessionInfo)]),
     "sa_last_error": (cp, []),
     "sa_version": (cp, []),
+    "sa_device_trim": (i32, [P(u64)]),
     "sa_seeding_params_from_read_length": (i32, [sz, P(SeedingParams)]),
     "sa_chaining_params_default": (None, [P(ChainingParams)]),
     "sa_mapping_params_default": (None, [P(MappingParams)]),

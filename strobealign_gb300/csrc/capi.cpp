@@ -98,6 +98,14 @@ void finish_index(sa_index* idx) {
 extern "C" {
 
 const char* sa_last_error(void) { return g_last_error.c_str(); }
+int32_t sa_device_trim(uint64_t* released) {
+    SA_TRY
+    const size_t bytes = dev_trim();
+    if (released) *released = bytes;
+    return SA_OK;
+    SA_CATCH
+}
+
 const char* sa_version(void) { return "strobealign_gb300 0.1.0 (reference strobealign 0.18.0-alpha)"; }
 
 int32_t sa_seeding_params_from_read_length(size_t read_length, sa_seeding_params* out) {

@@ -95,13 +95,15 @@ public:
         pool.kept += l.size;
     }
 
-    // Gives back what is kept at the current place.
-    void trim() {
+    // Gives back what is kept at the current place; its bytes.
+    size_t trim() {
         DevPlace at;
-        if (!be_.place(at)) return;
+        if (!be_.place(at)) return 0;
         std::lock_guard<std::mutex> g(mu_);
         Pool& pool = pool_of(at);
+        const size_t bytes = pool.kept;
         while (!pool.free.empty()) be_.free(pool.take(pool.free.size() - 1).p);
+        return bytes;
     }
 
     // bytes kept at a place; blocks handed out that may be kept, of all places

@@ -2,7 +2,7 @@
 // dozen buffers and gives them back at its end; allocating and freeing them took 2-3 ms of
 // a 5 ms call (100k reads to NAMs) and of an 11 ms build (100 Mbp).  Freed blocks are kept for the
 // next allocation instead (devcache.h), up to a bound.  They are given back when an
-// allocation fails and before the free device memory is asked for.
+// allocation fails, before the free device memory is asked for and by sa_device_trim.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -69,6 +69,6 @@ DevCache& cache() {
 
 void* dev_alloc(size_t bytes, bool exact) { return cache().alloc(bytes, exact); }
 void dev_free(void* p) { cache().free(p); }
-void dev_trim() { cache().trim(); }
+size_t dev_trim() { return cache().trim(); }
 
 }  // namespace sa

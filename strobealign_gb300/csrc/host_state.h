@@ -61,10 +61,10 @@ inline uint64_t sm_count() {
 
 // Device memory from a bounded cache of freed blocks (devmem.cpp); null when there is none.
 // exact: no larger block than that.  dev_free waits for the device, as cudaFree does;
-// dev_trim gives the cache back.
+// dev_trim gives the cache back and returns its bytes.
 void* dev_alloc(size_t bytes, bool exact = false);
 void dev_free(void* p);
-void dev_trim();
+size_t dev_trim();
 
 // Device buffer with RAII release.
 template <class T>
