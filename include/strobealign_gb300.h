@@ -522,8 +522,8 @@ int32_t sa_mapper_set_schedule(sa_mapper* m, const sa_schedule_params* p);
  *                           largest value, stands for all reads that the 16-bit kernel
  *                           takes (511 nt with the default scores)
  *   chain_lane_cluster_max  clusters of a long read orientation's anchors up to this
- *                           size (at least 2) are chained by one thread, larger ones by a
- *                           block
+ *                           size are chained by one thread, larger ones by a block; 1 is
+ *                           taken as 2, the smallest value
  *   l2_fetch_bytes          the context's L2 fetch granularity for DRAM reads
  *                           (cudaLimitMaxL2FetchGranularity: 32, 64 or 128; 0 keeps the
  *                           value the context had when the mapper was created).  It is a

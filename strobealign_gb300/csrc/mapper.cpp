@@ -779,7 +779,7 @@ void Mapper::set_tuning(const Tuning& t) {
     set_wave_min_jobs(std::max<uint64_t>(1, t.wave_min_jobs));
     set_max_wave_jobs(t.max_wave_jobs);
     ews_.wave_qmax = std::max<uint32_t>(1, t.wave_qmax);
-    chain_lane_max_ = std::max<uint32_t>(1, t.chain_lane_max);
+    chain_lane_max_ = std::max<uint32_t>(2, t.chain_lane_max);
     if (t.l2_fetch != l2_fetch_) {
         const size_t v = t.l2_fetch ? t.l2_fetch : l2_fetch_default_;
         if (v) SA_CUDA(cudaDeviceSetLimit(cudaLimitMaxL2FetchGranularity, v));
