@@ -352,8 +352,8 @@ uint32_t Mapper::schedule(std::vector<ChunkState>& chunks, uint32_t& launches, u
     bool nam_done = false;  // every part's NAMs are in (the plain form waits for it)
 
     // NAM pipelines, a part at a time on each lane; a part's chunks become ready once its
-    // NAMs are in.  The plain form and profiled maps (their events time one stream) use one.
-    const unsigned n_lanes = overlap_ && !kt_nam_.enabled && n_parts_ > 1 ? NAM_LANES : 1;
+    // NAMs are in.
+    const unsigned n_lanes = n_parts_ > 1 ? lanes_used() : 1;
     size_t next_part = 0, parts_done = 0;
     std::vector<std::thread> nam_threads;
     auto nam_lane = [&](unsigned l) {
@@ -616,9 +616,10 @@ void Mapper::map_uploaded(sa_output* out) {
     // output order are those of the whole batch; read and record indices inside a part
     // are local to it
     const size_t nchunks = chunks.size();
-    // at least parts_target_ parts, and enough that a part holds at most
-    // MAX_PART_BASES bases (the NAM workspace takes about 100 bytes per base)
-    const size_t by_bases = (size_t)((total_bases_ + MAX_PART_BASES - 1) / MAX_PART_BASES);
+    // at least parts_target_ parts, and enough that the parts in work at once (one a lane)
+    // hold at most MAX_PART_BASES bases together
+    const uint64_t part_max = lanes_used() > 1 ? MAX_PART_BASES / NAM_LANES : MAX_PART_BASES;
+    const size_t by_bases = (size_t)((total_bases_ + part_max - 1) / part_max);
     n_parts_ = std::max<size_t>(1, std::min<size_t>(std::max<size_t>(parts_target_, by_bases), nchunks / 4));
     while (parts_.size() < n_parts_) parts_.push_back(std::make_unique<Part>());
     // the first part is half the size of the others, so that the policy threads and the

@@ -11,6 +11,7 @@ namespace sa {
 
 class Mapper {
   public:
+    // bases in the NAM workspaces at once: these take about 150 bytes a base, 20 GB at most
     static constexpr uint64_t MAX_PART_BASES = 1ULL << 27;
     Mapper(const sa_index* idx, const sa_refs* refs, const sa_chaining_params& cp, const sa_mapping_params& mp);
     ~Mapper();
@@ -102,6 +103,8 @@ class Mapper {
         PinnedBuf<uint64_t> off;  // the part's local read offsets
     };
     static constexpr unsigned NAM_LANES = 2;
+    // the plain form and profiled maps (their events time one stream) use one
+    unsigned lanes_used() const { return overlap_ && !kt_nam_.enabled ? NAM_LANES : 1; }
     void part_nams(Part& p, NamLane& lane, uint32_t& launches);
     void prepare(const sa_read_batch* r1, const sa_read_batch* r2);
     void prepare_interleaved(const sa_read_batch* reads);
