@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(256, 5) k_probe(DevIndex ix, const uint64_t* _
 // orientation heuristic (src/chainer.rs:205-216, src/hit.rs:76-81).  The first pass
 // reads k_probe's per-slot answers.  Counts come from ballots, and the walk over filtered
 // stretches, hit after hit on one lane, is entered only when some stretch is long enough
-// (0.7 M reads: 2.0 ms with six warp sums per orientation and the walk for every read, 1.1 ms).
+// (1.4 M reads: 4.0 ms with six warp sums per orientation and the walk for every read, 2.2 ms).
 __global__ void __launch_bounds__(256) k_hits(DevIndex ix, const uint64_t* __restrict__ off, uint32_t n,
                                               uint64_t total, uint32_t mcs, uint32_t rescue_distance,
                                               const uint64_t* qr_hash, const uint64_t* qr_hash_rc,
@@ -641,7 +641,7 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t& total) 
 // The anchors of each read orientation (src/chainer.rs:304-384): counted, then written to the
 // next free range of the anchor array while the table entries are still in the L1 (a launch
 // each for counts and anchors read the table's random sectors twice: 11.2 KB of DRAM per read
-// on a human-sized index; 3.0 ms for 0.7 M reads, 2.3 ms now).  The ranges' order does not
+// on a human-sized index; 6.0 ms for 1.4 M reads, 4.6 ms now).  The ranges' order does not
 // matter to the stages after.  Past the array's capacity nothing is written; *cursor then
 // tells what it takes. Five blocks an SM in 48 registers: the NAM stage of 100,000 reads takes
 // 1.60 ms, with four in 64 registers 1.62 ms; six gain nothing more.
@@ -1229,7 +1229,8 @@ __device__ __forceinline__ void chain_candidates(uint32_t j, bool in, const uint
 
 // The lookback DP of collinear_chaining (src/chainer.rs:85-180) over anchors [c0, c1)
 // of one read orientation (its anchors at dedup[b ..]) by the whole warp, for a
-// max_lookback of 64 or more (warp_chain_regs otherwise): 32 predecessors per step, the early-break rules as a prefix max over the lanes.
+// max_lookback of 64 or more (warp_chain_regs otherwise): 32 predecessors per step, the
+// early-break rules as a prefix max over the lanes.
 // Predecessors never go below c0 (earlier anchors lie max_ref_gap or more behind, or
 // on another reference, and end the reference's scan without contributing).  With
 // recheck, (best_score, best_index, best_key) is the running best over all anchors
@@ -1738,9 +1739,11 @@ struct BigCluster {
 // the same diagonal.  A scoring warp holds those anchors' scores two per lane.
 //
 // The longest clusters of 53k-read parts on a 310 Mbp human-shaped genome (up to 3,100
-// anchors): 0.34 ms a launch on average, 0.56 at most; with the whole DP in one warp 1.06
-// and 1.69 ms, and 1.1 and 1.9 ms with the predecessors in shared memory.  The second scoring
-// costs nothing that shows (200k pairs to PAF 19.0 ms, 19.3 with the first alone).
+// anchors): 0.34 ms a launch on average, 0.56 at most, with the first scoring alone; with the
+// whole DP in one warp 1.06 and 1.69 ms, and 1.1 and 1.9 ms with the predecessors in shared
+// memory.  The second scoring makes a launch a tenth longer (parts of 185k reads: 0.56 ->
+// 0.62 ms on average, with cold caches) and spares k_chain_long serial work (0.43 -> 0.41,
+// at most 0.73 -> 0.52); 200k pairs to PAF take 19.0 ms, 19.3 with the first alone.
 constexpr uint32_t BIG_CHUNK = 32, BIG_SCORING = 2, BIG_WARPS = 5;
 
 __global__ void __launch_bounds__(32 * BIG_WARPS) k_chain_big(const uint64_t* __restrict__ off, const uint64_t* seg_off,
@@ -1930,14 +1933,15 @@ __global__ void __launch_bounds__(128) k_chain_big_far(const uint64_t* __restric
 
 // A long orientation per warp, its clusters scored by k_chain_long_prep (without the
 // re-check) and k_chain_big: in order, the clusters whose maximum beats the running best
-// and those whose own re-check changed a score, then the chains.  A kernel apart from k_chain4: the rings there take the shared memory
-// that the L1 needs here (the walks are chains of dependent loads; 300-500 cycles an
-// anchor from L2).
+// and those whose own re-check changed a score, then the chains.  A kernel apart from
+// k_chain4: the rings there take the shared memory that the L1 needs here (the walks are
+// chains of dependent loads; 300-500 cycles an anchor from L2).
 template <bool RING>
 __global__ void __launch_bounds__(128) k_chain_long(const uint64_t* __restrict__ off, const uint64_t* seg_off,
                                                     uint64_t* dedup, float* dp, uint32_t* pred, uint32_t* aux,
                                                     uint64_t total_anchors, unsigned long long* scratch,
-                                                    const uint2* plain, AnchorPack ap, ChainCtx cc, NamRec* nam_out, uint32_t* nam_seg_count, uint64_t* anc_out,
+                                                    const uint2* plain, AnchorPack ap, ChainCtx cc, NamRec* nam_out,
+                                                    uint32_t* nam_seg_count, uint64_t* anc_out,
                                                     uint64_t* anc_start, const uint32_t* long_list, uint32_t n_long,
                                                     const uint32_t* long_n, const uint32_t* long_c,
                                                     uint32_t lane_max) {

@@ -5,7 +5,14 @@
 namespace sa {
 
 constexpr uint32_t SSW16_MAX_QLEN = 511;
-// below this many tasks a block's two warps share a task's byte and word passes
+// Below this many tasks a block's two warps share a task's byte and word passes.  Both passes
+// then always run, so it pays while a launch lasts as long as one task: 2000 pairs to SAM
+// (waves of 30 to 500 tasks) 3.46 ms, 4.01 never shared; a session of 24 requests 11.0 and
+// 12.0 ms.  Alignment calls, whose tasks have no diagonal, gain up to about 10,000 tasks (4,000
+// of 100-300 nt 2.0 and 2.2 ms, 8,000 2.4 and 2.9) and lose beyond (16,000 of 250 nt 2.6 and
+// 2.4 ms; 60,000 of 100-300 nt 6.8 and 6.1 ms).  Mapping's larger waves, whose tasks mostly
+// have a diagonal that spares them the byte pass, take the same either way (100k pairs to SAM
+// within 1 %).  4096 is on the safe side: below it both kinds gain.
 constexpr uint32_t SSW16_PAIR_TASKS = 4096;
 
 struct Ssw16Args {
