@@ -112,7 +112,7 @@ void Mapper::prepare_reads(uint64_t n_rec, unsigned per_rec, uint64_t total, Vie
     total_bases_ = total;
     n_reads_ = (uint32_t)n;
     h2d_bytes_ = (n + 1) * 8;
-    have_batch_ = true;
+    have_batch_ = pending_ = true;
 }
 
 // The prepared batch's bases onto the device.
@@ -124,6 +124,7 @@ void Mapper::upload_all() {
     SA_CUDA(cudaMemcpyAsync(nws_.seq.p, h_seq_.p, total_bases_, cudaMemcpyHostToDevice, st_));
     h2d_bytes_ += total_bases_;
     SA_CUDA(cudaStreamSynchronize(st_));
+    pending_ = false;
 }
 
 // The NAM pipeline for one part, on its lane: the part's bases are uploaded if the batch's
@@ -303,16 +304,7 @@ void Mapper::upload_interleaved(const sa_read_batch* reads) {
 void Mapper::map_prepared(std::chrono::steady_clock::time_point t0, sa_output* out) {
     const uint64_t h2d = h2d_bytes_;
     const double tu = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-    pending_ = true;
-    try {
-        map_uploaded(out);
-    } catch (...) {
-        // some parts may not be on the device
-        pending_ = false;
-        have_batch_ = false;
-        throw;
-    }
-    pending_ = false;
+    map_uploaded(out);
     stats_.seconds_upload = tu;
     stats_.h2d_bytes += h2d;
     stats_.seconds_total = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -673,6 +665,7 @@ void Mapper::map_uploaded(sa_output* out) {
         throw;
     }
     const auto t_sched_end = std::chrono::steady_clock::now();
+    pending_ = false;  // every part is on the device
     launches += nam_launches;
     double t_nams = 0;
     for (size_t pi = 0; pi < n_parts_; pi++) t_nams += parts_[pi]->seconds;

@@ -123,7 +123,9 @@ class Mapper {
     // empty for uniform batches
     std::vector<uint32_t> rec_read_;
     bool have_batch_ = false;
-    bool pending_ = false;  // the batch's bases are uploaded part by part, by the NAM pipelines
+    // the batch's bases are not (all) on the device: the NAM pipelines upload them, part by
+    // part; after a map that failed, again by the next one
+    bool pending_ = false;
     uint32_t max_qlen_ = 1;
     sa_mapper_stats stats_{};
     double t_ext_ = 0;
